@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "gd_coarse.cuh"
+#include "gd_krylov.cuh"
 #include "gd_stream.cuh"
 #include "gd_tile.cuh"
 
@@ -34,10 +35,12 @@ struct gd_plan_s {
   int sms = 148;  // SMs of the plan's device (tile launches below one CTA per SM run wider CTAs)
   gd_params prm{};
   bool fp64 = false;
+  bool any_masked = false;
   std::vector<InstInfo> inst;
   std::vector<LevelInfo> lv;
   std::vector<Tile> tiles;
   int fine_base = 0, fine_count = 0, depth = 0;
+  int kr_base = 0, kr_count = 0;  // tiles of the Krylov kernels
   std::vector<int> down_base, down_count, up_base, up_count;     // strip maps per level
   std::vector<int> tdown_base, tdown_count, tup_base, tup_count;  // tile maps per level
   std::vector<char> tsmall;  // per level: tiles of the small shape (fewer large tiles than SMs)
@@ -253,10 +256,12 @@ struct Runner {
                          (int)SmallDown<S>::smem);
     cudaFuncSetAttribute(small_up<S>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)SmallUp<S>::smem);
-    cudaFuncSetAttribute(st::k_pupdate_s<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)st::pupdate_smem<T>());
-    cudaFuncSetAttribute(st::k_cgupdate_s<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)st::cgupdate_smem<T>());
+    cudaFuncSetAttribute(kr::k_pupdate<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)kr::pupdate_smem<T>());
+    cudaFuncSetAttribute(kr::k_cgupdate<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)kr::cgupdate_smem<T>(true));
+    cudaFuncSetAttribute(kr::k_cgupdate<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)kr::cgupdate_smem<T>(false));
     cudaFuncSetAttribute(st::k_refresh_s<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)st::refresh_smem<T>());
     cudaFuncSetAttribute(st::k_refresh_s<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -430,15 +435,18 @@ struct Runner {
   template <int S>
   static void iteration(gd_plan p, const Args<T> &a, cudaStream_t st, bool refresh) {
     vcycle<S>(p, a, st);
-    const Args<T> f = at_tiles(a, p->fine_base);
+    const Args<T> f = at_tiles(a, p->kr_base);
     const double c = p->fine_cells;
     prof_begin(p, GD_K_PUPDATE, c, st);
-    chain_launch(p, st::k_pupdate_s<T>, p->fine_count, st::kThreads, st::pupdate_smem<T>(), st,
-                 f);
+    chain_launch(p, kr::k_pupdate<T>, p->kr_count, kr::kThreads, kr::pupdate_smem<T>(), st, f);
     prof_end(p, st);
     prof_begin(p, GD_K_CGUPDATE, c, st);
-    chain_launch(p, st::k_cgupdate_s<T>, p->fine_count, st::kThreads, st::cgupdate_smem<T>(),
-                 st, f);
+    if (p->any_masked)
+      chain_launch(p, kr::k_cgupdate<T, true>, p->kr_count, kr::kThreads,
+                   kr::cgupdate_smem<T>(true), st, f);
+    else
+      chain_launch(p, kr::k_cgupdate<T, false>, p->kr_count, kr::kThreads,
+                   kr::cgupdate_smem<T>(false), st, f);
     prof_end(p, st);
     if (refresh) launch_refresh(p, a, st);
   }
@@ -746,10 +754,9 @@ int build_plan(gd_plan p, const gd_grid_desc *grids) {
   const int target_warps = std::max(p->prm.strip_target_warps, 0);
   long long cap[3] = {0, 0, 0};
   {
-    bool any_masked = false;
-    for (int i = 0; i < p->n; ++i) any_masked = any_masked || p->inst[i].bc == BC_MASK;
+    for (int i = 0; i < p->n; ++i) p->any_masked = p->any_masked || p->inst[i].bc == BC_MASK;
     if (p->fp64) Runner<double>::dispatch_capacity(p, false, cap);
-    else Runner<float>::dispatch_capacity(p, !any_masked, cap);
+    else Runner<float>::dispatch_capacity(p, !p->any_masked, cap);
   }
   for (int i = 0; i < p->n; ++i) p->inst[i].rz_rows = st::kRzRows;
   for (int l = 0; l < p->depth; ++l) {
@@ -777,6 +784,17 @@ int build_plan(gd_plan p, const gd_grid_desc *grids) {
     I.fine_end = (int)p->tiles.size() - p->fine_base;
   }
   p->fine_count = (int)p->tiles.size() - p->fine_base;
+  p->kr_base = (int)p->tiles.size();
+  for (int i = 0; i < p->n; ++i) {
+    InstInfo &I = p->inst[i];
+    const int cols = ceil_div(I.nx, kFTX);
+    I.kr_rows = kr::tile_rows(I.ny, I.nx);
+    I.kr_begin = (int)p->tiles.size() - p->kr_base;
+    for (int ty = 0; ty < ceil_div(I.ny, I.kr_rows); ++ty)
+      for (int tx = 0; tx < cols; ++tx) p->tiles.push_back(Tile{I.level0, i, ty, tx});
+    I.kr_end = (int)p->tiles.size() - p->kr_base;
+  }
+  p->kr_count = (int)p->tiles.size() - p->kr_base;
   p->down_base.assign(p->depth, 0);
   p->down_count.assign(p->depth, 0);
   p->up_base.assign(p->depth, 0);
@@ -854,10 +872,11 @@ int build_plan(gd_plan p, const gd_grid_desc *grids) {
       for (int ty = 0; ty < ceil_div(F.ny, rows); ++ty)
         for (int tx = 0; tx < ceil_div(F.nx, up_ow); ++tx)
           p->tiles.push_back(Tile{I.level0 + l, i, ty, tx});
+      if (l == 0) I.up0_ctas = ceil_div(F.ny, rows) * ceil_div(F.nx, up_ow);
     }
     p->up_count[l] = (int)p->tiles.size() - p->up_base[l];
   }
-  p->max_partials = std::max(1, std::max(p->fine_count, rz_parts));
+  p->max_partials = std::max({1, p->fine_count, p->kr_count, rz_parts});
   p->launch_cells.assign(2 * std::max(p->depth, 1), 0.0);
   p->fine_cells = 0;
   for (int i = 0; i < p->n; ++i) {

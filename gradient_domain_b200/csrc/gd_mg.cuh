@@ -25,7 +25,6 @@ constexpr int kTileCells = 1 << 18;
 constexpr int kFTY = 64, kFTX = 128, kFThreads = 128;
 constexpr int kVThreads = 128;     // down / up kernels
 constexpr int kBThreads = 1024;    // bottom kernel
-constexpr int kLastWarps = kFThreads / 32;
 
 enum : int { BC_DIR = 0, BC_NEU = 1, BC_MASK = 2 };
 // FLAG_RU: an FP64 refresh is due (set by cgupdate, cleared by the residual).
@@ -77,7 +76,10 @@ struct InstInfo {
   long long r_off, p_off, d_off, z_off, q_off;  // p is double-buffered: p_off / q_off
   long long xs_off;  // the plan's own FP64 copy of the solution (element offset, row pitch `pitch`)
   int fine_begin, fine_end;  // tile range in the fine map
+  int kr_begin, kr_end;      // tile range in the Krylov map
+  int kr_rows;               // rows of its Krylov tiles (depends on the instance alone)
   int up0_begin, up0_end;    // range of its r.z group partials (empty if bottom is level 0)
+  int up0_ctas;              // CTAs of the level-0 up kernel
   int zero_mean;
   int rz_rows;  // rows per r.z group partial: level 0's strip height for the instance alone
   // set per solve
@@ -96,7 +98,7 @@ struct InstState {
   int refreshes;  // FP64 refreshes after the initial residual
   int xzero;      // the solution is known to be zero (zero-start solve, nothing folded yet)
   int mean_known; // mean holds the solution's mean (set by a refresh that folds)
-  int pad;
+  unsigned ticket; // CTAs of the instance that have finished their part of a reduction
 };
 
 struct Tile {

@@ -29,27 +29,48 @@ __device__ __forceinline__ bool in_grid(const LevelInfo &L, int y, int x) {
   return y >= 0 && y < L.ny && x >= 0 && x < L.nx;
 }
 
-// Last-CTA handshake: every CTA calls it once; returns true in the last one.
-__device__ __forceinline__ bool last_block(unsigned *counter) {
+// Last-CTA handshake over the `ctas` CTAs of one instance: each calls it once;
+// returns true in the last one.  The instance's ticket is zero again after it
+// (the CTAs of the next kernel run after this one's), and since every instance
+// has its own, its reductions finish side by side instead of one after another
+// in the launch's last CTA.
+__device__ __forceinline__ bool last_of_instance(unsigned *ticket, int ctas) {
   __shared__ bool am_last;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    const unsigned prev = atomicAdd(counter, 1u);
-    am_last = (prev == gridDim.x - 1);
-    if (am_last) *counter = 0u;
+    const unsigned prev = atomicAdd(ticket, 1u);
+    am_last = (prev == (unsigned)ctas - 1u);
+    if (am_last) *ticket = 0u;
   }
   __syncthreads();
   if (am_last) __threadfence();
   return am_last;
 }
 
-// Deterministic per-instance sum of partials [b, e) by one warp (L2 reads).
-__device__ __forceinline__ double warp_range_sum(const double *p, int b, int e) {
+// Sum of `count` partials from `p` by the whole CTA in a fixed pattern; valid
+// in thread 0.
+template <int NT>
+__device__ __forceinline__ double block_range_sum(const double *p, int count) {
   double s = 0.0;
 #pragma unroll 8
-  for (int k = b + (threadIdx.x & 31); k < e; k += 32) s += __ldcg(p + k);
-  return warp_sum(s);
+  for (int k = threadIdx.x; k < count; k += NT) s += __ldcg(p + k);
+  return block_sum<NT>(s);
+}
+
+// Per-instance reduction: this CTA's per-thread values become its partial
+// (blockIdx.x, the instance's CTAs being `ctas` consecutive ones from `first`);
+// the instance's last CTA returns true, with the sum of all of them in its
+// thread 0.  The pattern depends on the instance alone, so a batch gives every
+// instance the sums it gets alone.
+template <int NT>
+__device__ __forceinline__ bool instance_sum(double *part, int first, int ctas, double v,
+                                             unsigned *ticket, double *sum) {
+  v = block_sum<NT>(v);
+  if (threadIdx.x == 0) part[blockIdx.x] = v;
+  if (!last_of_instance(ticket, ctas)) return false;
+  *sum = block_range_sum<NT>(part + first, ctas);
+  return true;
 }
 
 // The search direction lives in two buffers: k_pupdate reads the current one
@@ -387,22 +408,22 @@ template <typename T>
 __global__ void __launch_bounds__(kFThreads) k_fmean(Args<T> a) {
   const Tile tl = a.tiles[blockIdx.x];
   dep_enter();
-  if (blockIdx.x == 0 && threadIdx.x == 0) a.counter[kErrWord] = 0u;  // a solve starts
+  if (blockIdx.x == 0 && threadIdx.x == 0) {  // a solve starts
+    a.counter[kErrWord] = 0u;
+    *a.n_active = 0;
+  }
   const InstInfo &I = a.inst[tl.inst];
-  double part = 0.0;
-  if (I.zero_mean) {
-    const int Y0 = tl.ty * kFTY, gx = tl.tx * kFTX + threadIdx.x;
-    if (gx < I.nx) part = column_sum(I.f, I.upitch, Y0, min(Y0 + kFTY, I.ny), gx);
+  if (!I.zero_mean) {
+    if (blockIdx.x == I.fine_begin && threadIdx.x == 0) a.st[tl.inst].fmean = 0.0;
+    return;
   }
-  part = block_sum<kFThreads>(part);
-  if (threadIdx.x == 0) a.part0[blockIdx.x] = part;
-  if (!last_block(a.counter + 5)) return;
-  const int warp = threadIdx.x >> 5;
-  for (int i = warp; i < a.ninst; i += kLastWarps) {
-    const InstInfo &J = a.inst[i];
-    const double s = J.zero_mean ? warp_range_sum(a.part0, J.fine_begin, J.fine_end) : 0.0;
-    if ((threadIdx.x & 31) == 0) a.st[i].fmean = s / ((double)J.ny * (double)J.nx);
-  }
+  const int Y0 = tl.ty * kFTY, gx = tl.tx * kFTX + threadIdx.x;
+  const double part = gx < I.nx ? column_sum(I.f, I.upitch, Y0, min(Y0 + kFTY, I.ny), gx) : 0.0;
+  double sum;
+  if (instance_sum<kFThreads>(a.part0, I.fine_begin, I.fine_end - I.fine_begin, part,
+                              &a.st[tl.inst].ticket, &sum) &&
+      threadIdx.x == 0)
+    a.st[tl.inst].fmean = sum / ((double)I.ny * (double)I.nx);
 }
 
 // Mean removal for zero-mean (Neumann) instances: partial sums, then subtract.
@@ -411,25 +432,18 @@ __global__ void __launch_bounds__(kFThreads) k_mean(Args<T> a) {
   const Tile tl = a.tiles[blockIdx.x];
   dep_enter();
   const InstInfo &I = a.inst[tl.inst];
-  double part = 0.0;
   // only solutions no refresh has summed: a caller's x that met the tolerance at once
-  if (I.zero_mean && !a.st[tl.inst].mean_known) {
-    const bool own = a.st[tl.inst].xcur != 0;
-    const double *X = own ? a.xs + I.xs_off : I.x;
-    const long long pitch = own ? (long long)I.pitch : I.upitch;
-    const int Y0 = tl.ty * kFTY, gx = tl.tx * kFTX + threadIdx.x;
-    if (gx < I.nx) part = column_sum(X, pitch, Y0, min(Y0 + kFTY, I.ny), gx);
-  }
-  part = block_sum<kFThreads>(part);
-  if (threadIdx.x == 0) a.part0[blockIdx.x] = part;
-  if (!last_block(a.counter + 4)) return;
-  const int warp = threadIdx.x >> 5;
-  for (int i = warp; i < a.ninst; i += kLastWarps) {
-    const InstInfo &J = a.inst[i];
-    if (!J.zero_mean || a.st[i].mean_known) continue;
-    const double s = warp_range_sum(a.part0, J.fine_begin, J.fine_end);
-    if ((threadIdx.x & 31) == 0) a.st[i].mean = s / ((double)J.ny * (double)J.nx);
-  }
+  if (!I.zero_mean || a.st[tl.inst].mean_known) return;
+  const bool own = a.st[tl.inst].xcur != 0;
+  const double *X = own ? a.xs + I.xs_off : I.x;
+  const long long pitch = own ? (long long)I.pitch : I.upitch;
+  const int Y0 = tl.ty * kFTY, gx = tl.tx * kFTX + threadIdx.x;
+  const double part = gx < I.nx ? column_sum(X, pitch, Y0, min(Y0 + kFTY, I.ny), gx) : 0.0;
+  double sum;
+  if (instance_sum<kFThreads>(a.part0, I.fine_begin, I.fine_end - I.fine_begin, part,
+                              &a.st[tl.inst].ticket, &sum) &&
+      threadIdx.x == 0)
+    a.st[tl.inst].mean = sum / ((double)I.ny * (double)I.nx);
 }
 
 // The solution into the caller's buffer: x - mean for zero-mean instances, a

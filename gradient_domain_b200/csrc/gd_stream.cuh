@@ -25,7 +25,7 @@ namespace gd {
 namespace st {
 
 constexpr int kLanes = 32;
-constexpr int kWarps = 4;          // warps per CTA of the Krylov and refresh kernels
+constexpr int kWarps = 4;          // warps per CTA of the refresh kernel
 constexpr int kThreads = kWarps * kLanes;
 // The down / up kernels run one warp (one strip) per CTA: the block scheduler
 // then spreads a launch's strips evenly over the SMs (a launch of four-warp
@@ -40,8 +40,7 @@ struct UpCta {
   static constexpr int W = LEVEL0 ? 4 : 1;
   static constexpr int NT = W * kLanes;
 };
-constexpr int kKrylovRows = 16;    // rows per warp in the Krylov kernels
-constexpr int kKrylovCols = 128;   // columns per warp (and per CTA)
+constexpr int kRefRows = 16;       // rows per warp of the refresh
 
 template <typename T>
 struct V4 {
@@ -152,21 +151,6 @@ struct CodeRing {
   __device__ __forceinline__ unsigned read(int s) const { return *slot(s); }
 };
 
-// Per-lane ring of one element per row: the column just outside the warp
-// (left of lane 0, right of lane 31), so edge values arrive with their row.
-template <typename T>
-struct EdgeRing {
-  T *base;
-  __device__ __forceinline__ explicit EdgeRing(T *smem) : base(smem + threadIdx.x) {}
-  __device__ __forceinline__ T *slot(int s) const { return base + (s & (kRing - 1)) * kThreads; }
-  __device__ __forceinline__ void issue(int s, const T *A, const LevelInfo &L, int y, int x) const {
-    const bool ok = y >= 0 && y < L.ny && x >= 0 && x < L.nx;
-    __pipeline_memcpy_async(slot(s), ok ? A + (long long)y * L.pitch + x : A, sizeof(T),
-                            ok ? 0 : sizeof(T));
-  }
-  __device__ __forceinline__ T read(int s) const { return *slot(s); }
-};
-
 // Dynamic shared memory of the streaming kernels (rings).
 template <typename T, int NT = kThreads>
 constexpr size_t ring_bytes() { return (size_t)kRing * NT * 4 * sizeof(T); }
@@ -174,14 +158,6 @@ template <typename T, int NT = kSThreads>
 constexpr size_t level_smem() {
   return 2 * ring_bytes<T, NT>() + (size_t)kRing * NT * 4;
 }
-template <typename T>
-constexpr size_t edge_bytes() { return (size_t)kRing * kThreads * sizeof(T); }
-
-template <typename T>
-constexpr size_t pupdate_smem() { return 2 * ring_bytes<T>() + 2 * edge_bytes<T>(); }
-template <typename T>
-constexpr size_t cgupdate_smem() { return 3 * ring_bytes<T>() + edge_bytes<T>(); }
-
 // Lanes whose output is exact for a dependency radius of R columns.
 template <int R>
 struct Halo {
@@ -943,8 +919,8 @@ struct UpGeom {
 // height is a power-of-two multiple of it, so a group never spans two warps and
 // the grouping does not depend on the batch: a warp adds its lanes' products
 // over the group's rows and writes the group's warp sum when the group ends.
-// The last CTA of the launch sums an instance's partials in a fixed pattern, so
-// an instance gives the same r.z whatever strip heights its batch chose.
+// The instance's last CTA sums its partials in a fixed pattern, so an instance
+// gives the same r.z whatever strip heights its batch chose.
 constexpr int kRzRows = 8;  // the smallest group (and strip) height
 struct RzGroups {
   double *base;  // partial of group 0 of this column strip
@@ -1405,300 +1381,19 @@ __global__ void __launch_bounds__(UpCta<LEVEL0>::NT,
       }
     }
   }
-  if (!LEVEL0) return;
+  if (!LEVEL0 || !active) return;
   // the lane that wrote a warp's group partials makes them visible before the
   // CTA takes its ticket (one fence per warp)
   if ((threadIdx.x & 31) == 0) __threadfence();
-  if (!last_block(a.counter + 3)) return;
-  // one warp per instance (instances in parallel): each lane sums every 32nd of
-  // the instance's groups, then a fixed shuffle tree, so an instance gets the
-  // same r.z in any batch
-  const int warp = threadIdx.x >> 5, nw = UpCta<LEVEL0>::NT >> 5;
-  for (int i = warp; i < a.ninst; i += nw) {
-    const InstInfo &I = a.inst[i];
-    if (I.up0_end <= I.up0_begin) continue;
-    InstState &S = a.st[i];
-    if (S.status != GD_ACTIVE) continue;
-    const double rz = warp_range_sum(a.part0, I.up0_begin, I.up0_end);
-    if ((threadIdx.x & 31) == 0) finish_rz(S, rz);
-  }
+  InstState &S = a.st[tl.inst];
+  const InstInfo &I = a.inst[tl.inst];
+  if (!last_of_instance(&S.ticket, I.up0_ctas)) return;
+  const double rz = block_range_sum<UpCta<LEVEL0>::NT>(a.part0 + I.up0_begin,
+                                                       I.up0_end - I.up0_begin);
+  if (threadIdx.x == 0) finish_rz(S, rz);
 }
 
 // ---------------------------------------------------------------------------
-// Krylov kernels on level 0: a warp covers 128 columns x kKrylovRows rows and
-// the CTA four such row bands.  The one column outside the warp on each side
-// comes from a scalar load by lanes 0 and 31.
-
-template <typename T>
-__device__ __forceinline__ T edge_value(const T *A, const LevelInfo &L, int y, int x) {
-  return (y >= 0 && y < L.ny && x >= 0 && x < L.nx) ? A[(long long)y * L.pitch + x] : T(0);
-}
-
-template <typename T, bool INT>
-__device__ __forceinline__ double pupdate_rows(const Args<T> &a, const InstInfo &I,
-                                               const LevelInfo &L, const ClassTable<T> &tab,
-                                               int lane, int x0, int y0, int y1, T beta,
-                                               const T *z, const T *p, T *pn,
-                                               unsigned char *smem) {
-  const Coef<T, INT> C{tab, tab.d[1], tab.inv[1]};
-  const Ring<T> rz(reinterpret_cast<T *>(smem));
-  const Ring<T> rp(reinterpret_cast<T *>(smem) + kRing * kThreads * 4);
-  const EdgeRing<T> ez(reinterpret_cast<T *>(smem) + 2 * kRing * kThreads * 4);
-  const EdgeRing<T> ep(reinterpret_cast<T *>(smem) + 2 * kRing * kThreads * 4 + kRing * kThreads);
-  const int xe = lane == 0 ? x0 - 1 : x0 + 4;  // edge column of lanes 0 and 31
-  const bool edge_lane = lane == 0 || lane == 31;
-  const bool read_p = beta != T(0);
-  const int nsteps = y1 - y0 + 2;  // rows y0 - 1 .. y1; nothing past them is copied
-  auto issue = [&](int q) {
-    if (q < nsteps) {
-      const int y = y0 - 1 + q;
-      rz.issue(q, z, L, y, x0);
-      if (read_p) rp.issue(q, p, L, y, x0);
-      if (edge_lane) {
-        ez.issue(q, z, L, y, xe);
-        if (read_p) ep.issue(q, p, L, y, xe);
-      }
-    }
-    __pipeline_commit();
-  };
-  for (int q = 0; q < kRing - 1; ++q) issue(q);
-  int step = 0;
-  T edge_next = T(0);
-  // The first direction is p = z: with beta == 0 the old buffer is not read
-  // (it need not be initialised), so the rings for p are left idle.
-  const bool use_p = beta != T(0);
-  auto newp = [&]() {
-    __pipeline_wait_prior(kRing - 2);
-    V4<T> zz = rz.read(step);
-    T e = edge_lane ? ez.read(step) : T(0);
-    if (use_p) {
-      const V4<T> pp = rp.read(step);
-      if (edge_lane) e += beta * ep.read(step);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) zz.v[j] += beta * pp.v[j];
-    }
-    edge_next = e;
-    issue(step + kRing - 1);
-    ++step;
-    return zz;
-  };
-  double part = 0.0;
-  V4<T> up = newp(), cu = newp(), dn;
-  T edge_cu = edge_next;
-  const bool full = x0 + 3 < L.nx;
-  for (int y = y0; y < y1; ++y) {
-    dn = newp();
-    T left = shfl_up1(cu.v[3]), right = shfl_dn1(cu.v[0]);
-    if (lane == 0) left = edge_cu;
-    if (lane == 31) right = edge_cu;
-    edge_cu = edge_next;
-    const unsigned c = INT ? 0u : row_classes(L, a.codes, y, x0);
-    const V4<T> ap = arow(cu, up, dn, left, right, c, C);
-    T acc = T(0);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc += cu.v[j] * ap.v[j];
-    part += (double)acc;
-    if (x0 < L.nx) {
-      T *dst = pn + (long long)y * L.pitch + x0;
-      if (full) st4(dst, cu);
-      else
-        for (int j = 0; j < 4 && x0 + j < L.nx; ++j) dst[j] = cu.v[j];
-    }
-    up = cu;
-    cu = dn;
-  }
-  __pipeline_wait_prior(0);
-  return part;
-}
-
-// p_new = z + beta p_old (read from one buffer, written to the other) and p.Ap.
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_pupdate_s(Args<T> a) {
-  __shared__ ClassTable<T> tab;
-  const Tile tl = a.tiles[blockIdx.x];
-  dep_enter();
-  const bool active = a.st[tl.inst].status == GD_ACTIVE;
-  double part = 0.0;
-  if (active) {
-    const InstInfo &I = a.inst[tl.inst];
-    const LevelInfo L = a.lv[I.level0];
-    fill_table(tab, L.wall);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int y0 = (tl.ty * kWarps + warp) * kKrylovRows;
-    const int xl = tl.tx * kKrylovCols;
-    const int x0 = xl + 4 * lane;
-    if (y0 < L.ny) {
-      const int y1 = min(y0 + kKrylovRows, L.ny);
-      const T beta = (T)a.st[tl.inst].beta;
-      const int cur = a.st[tl.inst].pcur;
-      const T *z = a.arena + I.z_off;
-      const T *p = a.arena + p_offset(I, cur);
-      T *pn = a.arena + p_offset(I, cur ^ 1);
-      extern __shared__ __align__(16) unsigned char smem[];
-      if (strip_interior(L, y0, y1 - 1, xl, xl + 127))
-        part = pupdate_rows<T, true>(a, I, L, tab, lane, x0, y0, y1, beta, z, p, pn, smem);
-      else
-        part = pupdate_rows<T, false>(a, I, L, tab, lane, x0, y0, y1, beta, z, p, pn, smem);
-    }
-  }
-  part = block_sum<kThreads>(part);
-  if (threadIdx.x == 0) a.part0[blockIdx.x] = part;
-  if (!last_block(a.counter + 0)) return;
-  const int warp = threadIdx.x >> 5;
-  for (int i = warp; i < a.ninst; i += kWarps) {
-    InstState &S = a.st[i];
-    if (S.status != GD_ACTIVE) continue;
-    const InstInfo &I = a.inst[i];
-    const double pAp = warp_range_sum(a.part0, I.fine_begin, I.fine_end);
-    if ((threadIdx.x & 31) == 0) {
-      const double alpha = S.rz / pAp;
-      S.pAp = pAp;
-      S.pcur ^= 1;
-      if (!(pAp > 0.0) || !isfinite(alpha)) {
-        S.status = GD_BREAKDOWN;
-        S.flags |= FLAG_RU;
-      } else {
-        S.alpha = alpha;
-      }
-    }
-  }
-}
-
-template <typename T, bool INT>
-__device__ __forceinline__ double cgupdate_rows(const Args<T> &a, const LevelInfo &L,
-                                                const ClassTable<T> &tab, int lane, int x0,
-                                                int y0, int y1, T alpha, const T *p, T *d, T *r,
-                                                bool dzero, unsigned char *smem) {
-  const Coef<T, INT> C{tab, tab.d[1], tab.inv[1]};
-  const Ring<T> rp(reinterpret_cast<T *>(smem));
-  const Ring<T> rd(reinterpret_cast<T *>(smem) + kRing * kThreads * 4);
-  const Ring<T> rr(reinterpret_cast<T *>(smem) + 2 * kRing * kThreads * 4);
-  const EdgeRing<T> ep(reinterpret_cast<T *>(smem) + 3 * kRing * kThreads * 4);
-  const int xe = lane == 0 ? x0 - 1 : x0 + 4;  // edge column of lanes 0 and 31
-  const bool edge_lane = lane == 0 || lane == 31;
-  // p streams rows y0 - 1 .. y1; d and r the band's own rows y0 .. y1 - 1, used
-  // one step later (the slots of the two halo rows are never read); nothing past
-  // row y1 is copied
-  const int nsteps = y1 - y0 + 2;
-  auto issue = [&](int q) {
-    if (q < nsteps) {
-      const int y = y0 - 1 + q;
-      const bool own = y >= y0 && y < y1;
-      rp.issue(q, p, L, y, x0);
-      if (own && !dzero) rd.issue(q, d, L, y, x0);
-      if (own) rr.issue(q, r, L, y, x0);
-      if (edge_lane) ep.issue(q, p, L, y, xe);
-    }
-    __pipeline_commit();
-  };
-  for (int q = 0; q < kRing - 1; ++q) issue(q);
-  int step = 0;
-  V4<T> dcur, rcur, dnext = zero4<T>(), rnext = zero4<T>();
-  T edge_next = T(0);
-  auto next = [&]() {
-    __pipeline_wait_prior(kRing - 2);
-    const V4<T> pp = rp.read(step);
-    dcur = dnext;
-    rcur = rnext;
-    dnext = dzero ? zero4<T>() : rd.read(step);
-    rnext = rr.read(step);
-    edge_next = edge_lane ? ep.read(step) : T(0);
-    issue(step + kRing - 1);
-    ++step;
-    return pp;
-  };
-  double part = 0.0;
-  V4<T> up = next(), cu = next(), dn;
-  T edge_cu = edge_next;
-  const bool full = x0 + 3 < L.nx;
-  for (int y = y0; y < y1; ++y) {
-    dn = next();
-    T left = shfl_up1(cu.v[3]), right = shfl_dn1(cu.v[0]);
-    if (lane == 0) left = edge_cu;
-    if (lane == 31) right = edge_cu;
-    edge_cu = edge_next;
-    const unsigned c = INT ? 0u : row_classes(L, a.codes, y, x0);
-    const V4<T> ap = arow(cu, up, dn, left, right, c, C);
-    if (x0 < L.nx) {
-      const long long g = (long long)y * L.pitch + x0;
-      if (full) {
-        V4<T> dd = dcur, rv = rcur;
-        T acc = T(0);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          dd.v[j] += alpha * cu.v[j];
-          rv.v[j] -= alpha * ap.v[j];
-          acc += rv.v[j] * rv.v[j];
-        }
-        part += (double)acc;
-        st4(d + g, dd);
-        st4(r + g, rv);
-      } else {
-        for (int j = 0; j < 4 && x0 + j < L.nx; ++j) {
-          d[g + j] = (dzero ? T(0) : d[g + j]) + alpha * cu.v[j];
-          const T rn = r[g + j] - alpha * ap.v[j];
-          r[g + j] = rn;
-          part += (double)rn * (double)rn;
-        }
-      }
-    }
-    up = cu;
-    cu = dn;
-  }
-  __pipeline_wait_prior(0);
-  return part;
-}
-
-// d += alpha p, r -= alpha A p and r.r; schedules FP64 refreshes.
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_cgupdate_s(Args<T> a) {
-  __shared__ ClassTable<T> tab;
-  const Tile tl = a.tiles[blockIdx.x];
-  dep_enter();
-  const bool active = a.st[tl.inst].status == GD_ACTIVE;
-  double part = 0.0;
-  if (active) {
-    const InstInfo &I = a.inst[tl.inst];
-    const LevelInfo L = a.lv[I.level0];
-    fill_table(tab, L.wall);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int y0 = (tl.ty * kWarps + warp) * kKrylovRows;
-    const int xl = tl.tx * kKrylovCols;
-    const int x0 = xl + 4 * lane;
-    if (y0 < L.ny) {
-      const int y1 = min(y0 + kKrylovRows, L.ny);
-      const T alpha = (T)a.st[tl.inst].alpha;
-      const T *p = a.arena + p_offset(I, a.st[tl.inst].pcur);
-      T *d = a.arena + I.d_off;
-      T *r = a.arena + I.r_off;
-      const bool dzero = a.st[tl.inst].flags & FLAG_DZERO;
-      extern __shared__ __align__(16) unsigned char smem[];
-      if (strip_interior(L, y0, y1 - 1, xl, xl + 127))
-        part = cgupdate_rows<T, true>(a, L, tab, lane, x0, y0, y1, alpha, p, d, r, dzero, smem);
-      else
-        part = cgupdate_rows<T, false>(a, L, tab, lane, x0, y0, y1, alpha, p, d, r, dzero, smem);
-    }
-  }
-  part = block_sum<kThreads>(part);
-  if (threadIdx.x == 0) a.part0[blockIdx.x] = part;
-  if (!last_block(a.counter + 1)) return;
-  const int warp = threadIdx.x >> 5;
-  for (int i = warp; i < a.ninst; i += kWarps) {
-    InstState &S = a.st[i];
-    if (S.status != GD_ACTIVE) continue;
-    const InstInfo &I = a.inst[i];
-    const double rr = warp_range_sum(a.part0, I.fine_begin, I.fine_end);
-    if ((threadIdx.x & 31) == 0) {
-      S.rr = rr;
-      S.iters += 1;
-      S.flags &= ~FLAG_DZERO;  // every CTA of this launch has read it
-      if (rr <= a.delta2 * S.rr_ref || rr <= a.tol2 * S.ff || S.iters >= a.max_iter ||
-          !isfinite(rr))
-        S.flags |= FLAG_RU;
-    }
-  }
-}
-
 // FP64 refresh: x' = x + d (the FP32 correction folded into the FP64
 // solution), r = scale (f - fmean) - A x', the residual norm and the
 // convergence decision per instance, in one pass.  With INIT: the residual of
@@ -1711,7 +1406,7 @@ __global__ void __launch_bounds__(kThreads) k_cgupdate_s(Args<T> a) {
 // When d restarted since the last refresh (FLAG_DZERO) there is nothing to
 // fold and the current copy stays where it is.
 //
-// A warp covers 128 columns (four per lane) and kKrylovRows rows of the
+// A warp covers 128 columns (four per lane) and kRefRows rows of the
 // 64 x 128 fine tile, plus one halo row above and below; horizontal
 // neighbours come from shuffles and lanes 0 and 31 take the column just
 // outside the warp.  Rows arrive through a ring of kRefRing slots in shared
@@ -1747,8 +1442,8 @@ struct RefSmem {
 template <typename T>
 constexpr size_t refresh_smem() { return RefSmem<T>::bytes; }
 
-static_assert(kFTX == 4 * kLanes && kFTY == kWarps * kKrylovRows,
-              "the refresh maps one warp to 128 columns and kKrylovRows rows of a fine tile");
+static_assert(kFTX == 4 * kLanes && kFTY == kWarps * kRefRows,
+              "the refresh maps one warp to 128 columns and kRefRows rows of a fine tile");
 
 // x[x0 .. x0 + 3] of one FP64 row into two 16-byte chunks; `nv` (0..4) of the
 // four columns are inside the grid, the others are zero-filled.  `row` is any
@@ -2110,8 +1805,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_refresh_s(Args<T> a) {
     const int col0 = tl.tx * kFTX;
     w.x0 = col0 + 4 * lane;
     w.nv = max(0, min(4, w.nx - w.x0));
-    w.y0 = tl.ty * kFTY + warp * kKrylovRows;
-    w.y1 = min(w.y0 + kKrylovRows, w.ny);
+    w.y0 = tl.ty * kFTY + warp * kRefRows;
+    w.y1 = min(w.y0 + kRefRows, w.ny);
     w.ecol = lane == 0 ? w.x0 - 1 : w.x0 + 4;
     w.ecol_in = w.ecol >= 0 && w.ecol < w.nx;
     unsigned *const err = a.counter + kErrWord;
@@ -2136,73 +1831,64 @@ __global__ void __launch_bounds__(kThreads, 4) k_refresh_s(Args<T> a) {
     __syncthreads();
     part_f = block_sum<kThreads>(part_f);
   }
+  if (!work) return;
   if (threadIdx.x == 0) {
     a.part0[blockIdx.x] = part;
     a.part1[blockIdx.x] = part_f;  // INIT: ||f||^2; a refresh that folds: the sum of x + d
   }
-  if (!last_block(a.counter + 2)) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int active = 0;
-  for (int i = warp; i < a.ninst; i += kWarps) {
-    InstState &S = a.st[i];
-    const InstInfo &I = a.inst[i];
-    const bool part_of = INIT || (S.flags & FLAG_RU);
-    if (part_of) {
-      const double rr = warp_range_sum(a.part0, I.fine_begin, I.fine_end);
-      const double p1 = warp_range_sum(a.part1, I.fine_begin, I.fine_end);
-      if (lane == 0) {
-        if (INIT) {
-          S.ff = p1;
-          S.mean = 0.0;
-          S.mean_known = a.zero_start;  // a zero start has mean zero
-          S.iters = 0;
-          S.first = 1;
-          S.rz = 0.0;
-          S.beta = 0.0;
-          S.pcur = 0;
-          S.xcur = 0;
-          S.xzero = a.zero_start;
-          S.refreshes = 0;
-          S.status = GD_ACTIVE;
-        } else {
-          S.refreshes += 1;
-          if (!(S.flags & FLAG_DZERO)) {
-            S.xcur ^= 1;  // x + d went to the other copy
-            S.xzero = 0;
-            S.mean = p1 / ((double)I.ny * (double)I.nx);  // of the new solution
-            S.mean_known = 1;
-          }
-        }
-        // A refresh that barely lowers the true residual (less than 3x), once
-        // it is already below 1e-6 of ||f||, means the FP64 rounding floor is
-        // reached: stop with the current iterate instead of iterating on noise.
-        const bool stalled = !INIT && rr > 0.1 * S.rr_prev && rr <= 1e-12 * S.ff;
-        if (INIT || rr < S.rr_prev) S.rr_prev = rr;
-        S.rr_true = rr;
-        S.rr_ref = rr;
-        S.rr = rr;
-        if (rr <= a.tol2 * S.ff) {
-          S.status = GD_CONVERGED;
-        } else if (!isfinite(rr)) {
-          S.status = GD_BREAKDOWN;
-        } else if (S.status == GD_ACTIVE && stalled) {
-          S.status = GD_STAGNATED;
-        } else if (S.status == GD_ACTIVE && S.iters >= a.max_iter) {
-          S.status = GD_MAX_ITERATIONS;
-        }
-        S.flags = FLAG_DZERO;  // the correction restarts after every refresh
-      }
-    }
-    if (lane == 0 && S.status == GD_ACTIVE) ++active;
-  }
-  __shared__ int cnt[kWarps];
-  if (lane == 0) cnt[warp] = active;
+  InstState &S = a.st[tl.inst];
+  const InstInfo &I = a.inst[tl.inst];
+  const int ctas = I.fine_end - I.fine_begin;
+  if (!last_of_instance(&S.ticket, ctas)) return;
+  const double rr = block_range_sum<kThreads>(a.part0 + I.fine_begin, ctas);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int w = 0; w < kWarps; ++w) t += cnt[w];
-    *a.n_active = t;
+  const double p1 = block_range_sum<kThreads>(a.part1 + I.fine_begin, ctas);
+  if (threadIdx.x != 0) return;
+  if (INIT) {
+    S.ff = p1;
+    S.mean = 0.0;
+    S.mean_known = a.zero_start;  // a zero start has mean zero
+    S.iters = 0;
+    S.first = 1;
+    S.rz = 0.0;
+    S.beta = 0.0;
+    S.pcur = 0;
+    S.xcur = 0;
+    S.xzero = a.zero_start;
+    S.refreshes = 0;
+    S.status = GD_ACTIVE;
+  } else {
+    S.refreshes += 1;
+    if (!(S.flags & FLAG_DZERO)) {
+      S.xcur ^= 1;  // x + d went to the other copy
+      S.xzero = 0;
+      S.mean = p1 / ((double)I.ny * (double)I.nx);  // of the new solution
+      S.mean_known = 1;
+    }
   }
+  // A refresh that barely lowers the true residual (less than 3x), once
+  // it is already below 1e-6 of ||f||, means the FP64 rounding floor is
+  // reached: stop with the current iterate instead of iterating on noise.
+  const bool stalled = !INIT && rr > 0.1 * S.rr_prev && rr <= 1e-12 * S.ff;
+  if (INIT || rr < S.rr_prev) S.rr_prev = rr;
+  S.rr_true = rr;
+  S.rr_ref = rr;
+  S.rr = rr;
+  if (rr <= a.tol2 * S.ff) {
+    S.status = GD_CONVERGED;
+  } else if (!isfinite(rr)) {
+    S.status = GD_BREAKDOWN;
+  } else if (S.status == GD_ACTIVE && stalled) {
+    S.status = GD_STAGNATED;
+  } else if (S.status == GD_ACTIVE && S.iters >= a.max_iter) {
+    S.status = GD_MAX_ITERATIONS;
+  }
+  S.flags = FLAG_DZERO;  // the correction restarts after every refresh
+  // the instances still iterating: counted up by the initial residual (k_fmean
+  // starts from zero) and down by the refresh that stops one.  Every instance a
+  // refresh works on was counted: only counted instances ask for one.
+  if (INIT && S.status == GD_ACTIVE) atomicAdd(a.n_active, 1);
+  if (!INIT && S.status != GD_ACTIVE) atomicSub(a.n_active, 1);
 }
 
 }  // namespace st
