@@ -473,15 +473,14 @@ def ours(args) -> None:
         if tpc:
             traffic = tpc * per_launch_cells
     total_ms = sum(v["ms"] for v in kinds.values())
-    # launches in the headline pass: per solve the two init kernels, the loop gate, and per
-    # executed iteration the iteration's kernels without the refresh plus the refresh gate
-    # and the loop gate, one refresh kernel per refresh that ran, then the solution kernel
-    # (the zero-start plan's refreshes leave the mean, so no mean kernel; the device loop
-    # runs exactly max(iterations) iterations)
+    # launches in the headline pass: per solve the two init kernels, per executed iteration
+    # the iteration's kernels without the refresh, one refresh kernel per refresh that ran,
+    # then the solution kernel (the zero-start plan's refreshes leave the mean, so no mean
+    # kernel; the device loop runs exactly max(iterations) iterations)
     iter_kinds = [k for k in kinds if k not in ("init", "mean", "resid")]
     per_iter = sum(kinds[k]["launches"] for k in iter_kinds) / max(kinds["pupdate"]["launches"], 1)
     refreshes = max(r.refreshes for r in results)
-    launches = args.steps * (2 + 1 + max(its) * (per_iter + 2) + refreshes + 1)
+    launches = args.steps * (2 + max(its) * per_iter + refreshes + 1)
 
     smoother = smoother_gate(size, hbm, kinds, params.sweeps) if rank == 0 else None
 

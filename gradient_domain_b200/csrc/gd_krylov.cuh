@@ -192,6 +192,11 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) k_pupdate(Args<T> a) {
   const Tile tl = a.tiles[blockIdx.x];
   dep_enter();
+  if (blockIdx.x == 0 && threadIdx.x == 0 && a.loop) {
+    const int t = *a.trips + 1;
+    *a.trips = t;
+    if (t >= a.trip_cap) set_condition(a.loop, 0u);
+  }
   const InstInfo &I = a.inst[tl.inst];
   InstState &S = a.st[tl.inst];
   // every descriptor field is requested before the first is used
@@ -216,6 +221,7 @@ __global__ void __launch_bounds__(kThreads) k_pupdate(Args<T> a) {
     if (!(pAp > 0.0) || !isfinite(alpha)) {
       S.status = GD_BREAKDOWN;
       S.flags |= FLAG_RU;
+      set_condition(a.refresh, 1u);
     } else {
       S.alpha = alpha;
     }
@@ -328,8 +334,10 @@ __global__ void __launch_bounds__(kThreads) k_cgupdate(Args<T> a) {
     S.rr = rr;
     S.iters = iters;
     int f = flags & ~FLAG_DZERO;  // every CTA of this instance has read it
-    if (rr <= a.delta2 * rr_ref || rr <= a.tol2 * ff || iters >= a.max_iter || !isfinite(rr))
+    if (rr <= a.delta2 * rr_ref || rr <= a.tol2 * ff || iters >= a.max_iter || !isfinite(rr)) {
       f |= FLAG_RU;
+      set_condition(a.refresh, 1u);
+    }
     S.flags = f;
   }
 }

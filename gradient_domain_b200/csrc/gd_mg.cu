@@ -221,6 +221,11 @@ void chain_launch(gd_plan p, void (*kernel)(KP...), int grid, int block, size_t 
   cudaLaunchKernelEx(&cfg, kernel, std::forward<AT>(args)...);
 }
 
+// Most iterations of a solve's loop, whatever the instances' states say.
+int loop_cap(gd_plan p) {
+  return (int)std::min<long long>((long long)p->prm.max_iterations + 8, 1ll << 30);
+}
+
 // Strip geometry of the down / up kernels for a plan's precision and sweeps.
 template <typename T, int S>
 struct StripCfg {
@@ -338,6 +343,9 @@ struct Runner {
     a.delta2 = p->fp64 ? 0.0 : p->prm.reliable_delta * p->prm.reliable_delta;
     a.max_iter = p->prm.max_iterations;
     a.zero_start = p->prm.zero_start != 0;
+    a.loop = a.refresh = 0;
+    a.trips = reinterpret_cast<int *>(p->ws + p->o_trip);
+    a.trip_cap = loop_cap(p);
     return a;
   }
 
@@ -1102,26 +1110,6 @@ extern "C" int gd_plan_prepare(gd_plan p, cudaStream_t st) {
 
 namespace {
 
-// Condition of the solve graph's while loop: iterate while any instance is
-// active, at most `cap` times.  `start` resets the trip counter.
-__global__ void k_loop_gate(cudaGraphConditionalHandle h, const int *n_active, int *trips,
-                            int start, int cap) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int t = start ? 0 : *trips + 1;
-  *trips = t;
-  cudaGraphSetConditional(h, (*n_active > 0 && t < cap) ? 1u : 0u);
-}
-
-// Condition of the refresh node in the loop body: some instance asked for an
-// FP64 refresh (FLAG_RU).  Iterations without one launch no refresh kernel.
-__global__ void k_refresh_gate(cudaGraphConditionalHandle h, const InstState *st, int n) {
-  if (blockIdx.x != 0) return;
-  bool any = false;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) any = any || (st[i].flags & FLAG_RU);
-  any = __any_sync(0xffffffffu, any);
-  if (threadIdx.x == 0) cudaGraphSetConditional(h, any ? 1u : 0u);
-}
-
 template <typename T>
 void launch_init(gd_plan p, const Args<T> &fine, cudaStream_t st) {
   prof_begin(p, GD_K_INIT, p->fine_cells, st);
@@ -1152,97 +1140,74 @@ void launch_finish(gd_plan p, const Args<T> &fine, cudaStream_t st) {
   prof_end(p, st);
 }
 
-int loop_cap(gd_plan p) {
-  return (int)std::min<long long>((long long)p->prm.max_iterations + 8, 1ll << 30);
-}
-
 // One graph per plan for a whole solve: the initial residual, a conditional
 // while node whose body is one Krylov iteration (V-cycle, p update, d / r
 // update, then the FP64 refresh behind an if node, launched only when some
-// instance asked for one) followed by k_loop_gate, and the zero-mean
-// projection.  The device decides when to stop, so a solve is a single graph
-// launch with no host round trip and no iteration past the last active
-// instance.
+// instance asked for one), and the zero-mean projection.  The kernels that
+// decide - the initial residual, the reductions, the refresh - set the two
+// conditions themselves (Args::loop, Args::refresh), so a solve is a single
+// graph launch with no host round trip, no kernel that only decides, and no
+// iteration past the last active instance.
 template <typename T>
-int build_solve_graph(gd_plan p, const Args<T> &a, const Args<T> &fine) {
+int build_solve_graph(gd_plan p, const Args<T> &direct) {
   if (!p->cap) {
     GD_CHECK_CUDA(cudaGetDevice(&p->cap_device));
     GD_CHECK_CUDA(capture_stream_get(p->cap_device, &p->cap));
   }
   cudaStream_t cs = p->cap;
-  int *trips = reinterpret_cast<int *>(p->ws + p->o_trip);
-  const int cap = loop_cap(p);
-  GD_CHECK_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-  cudaError_t e = cudaSuccess;
-  cudaGraphConditionalHandle h{};
-  cudaGraph_t body = nullptr;
-  do {
-    launch_init(p, fine, cs);
+  Args<T> a = direct;
+  // the graph and dependencies that capture on cs has reached; adds a conditional
+  // node of `type` there and returns its body
+  auto add_conditional = [&](cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type,
+                             cudaGraph_t *body) -> cudaError_t {
     cudaStreamCaptureStatus status;
     cudaGraph_t cg = nullptr;
     const cudaGraphNode_t *deps = nullptr;
     size_t nd = 0;
-    if ((e = cudaStreamGetCaptureInfo(cs, &status, nullptr, &cg, &deps, &nd)) != cudaSuccess) break;
-    if ((e = cudaGraphConditionalHandleCreate(&h, cg, 0, cudaGraphCondAssignDefault)) !=
-        cudaSuccess)
-      break;
-    k_loop_gate<<<1, 32, 0, cs>>>(h, a.n_active, trips, 1, cap);
-    if ((e = cudaGetLastError()) != cudaSuccess) break;
-    if ((e = cudaStreamGetCaptureInfo(cs, &status, nullptr, &cg, &deps, &nd)) != cudaSuccess) break;
+    cudaError_t e = cudaStreamGetCaptureInfo(cs, &status, nullptr, &cg, &deps, &nd);
+    if (e != cudaSuccess) return e;
     cudaGraphNodeParams cp = {};
     cp.type = cudaGraphNodeTypeConditional;
     cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.type = type;
     cp.conditional.size = 1;
-    cudaGraphNode_t wn;
-    if ((e = cudaGraphAddNode(&wn, cg, deps, nd, &cp)) != cudaSuccess) break;
-    body = cp.conditional.phGraph_out[0];
-    if ((e = cudaStreamUpdateCaptureDependencies(cs, &wn, 1, cudaStreamSetCaptureDependencies)) !=
-        cudaSuccess)
-      break;
-    launch_finish(p, fine, cs);
+    cudaGraphNode_t node;
+    if ((e = cudaGraphAddNode(&node, cg, deps, nd, &cp)) != cudaSuccess) return e;
+    *body = cp.conditional.phGraph_out[0];
+    return cudaStreamUpdateCaptureDependencies(cs, &node, 1, cudaStreamSetCaptureDependencies);
+  };
+  // a handle (initially 0 in every launch of the graph) on the graph being captured
+  auto new_handle = [&](cudaGraphConditionalHandle *h) -> cudaError_t {
+    cudaStreamCaptureStatus status;
+    cudaGraph_t cg = nullptr;
+    const cudaError_t e = cudaStreamGetCaptureInfo(cs, &status, nullptr, &cg, nullptr, nullptr);
+    if (e != cudaSuccess) return e;
+    return cudaGraphConditionalHandleCreate(h, cg, 0, cudaGraphCondAssignDefault);
+  };
+  GD_CHECK_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
+  cudaError_t e = cudaSuccess;
+  cudaGraph_t body = nullptr, refresh_body = nullptr;
+  do {
+    if ((e = new_handle(&a.loop)) != cudaSuccess) break;
+    launch_init(p, Runner<T>::at_tiles(a, p->fine_base), cs);
+    if ((e = cudaGetLastError()) != cudaSuccess) break;
+    if ((e = add_conditional(a.loop, cudaGraphCondTypeWhile, &body)) != cudaSuccess) break;
+    launch_finish(p, Runner<T>::at_tiles(a, p->fine_base), cs);
     e = cudaGetLastError();
   } while (0);
   cudaGraph_t g = nullptr;
   const cudaError_t ee = cudaStreamEndCapture(cs, &g);
   if (e == cudaSuccess) e = ee;
-  // loop body: an iteration without the refresh, the refresh behind an if
-  // node that k_refresh_gate sets, then the loop gate
-  cudaGraph_t refresh_body = nullptr;
+  // loop body: an iteration without the refresh, then the refresh behind its if node
   if (e == cudaSuccess) {
     e = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0,
                                       cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
       do {
+        if ((e = new_handle(&a.refresh)) != cudaSuccess) break;
         Runner<T>::dispatch_iteration(p, a, cs, false);
-        cudaStreamCaptureStatus status;
-        cudaGraph_t cg = nullptr;
-        const cudaGraphNode_t *deps = nullptr;
-        size_t nd = 0;
-        cudaGraphConditionalHandle hr{};
-        if ((e = cudaStreamGetCaptureInfo(cs, &status, nullptr, &cg, &deps, &nd)) != cudaSuccess)
-          break;
-        if ((e = cudaGraphConditionalHandleCreate(&hr, cg, 0, cudaGraphCondAssignDefault)) !=
-            cudaSuccess)
-          break;
-        k_refresh_gate<<<1, 32, 0, cs>>>(hr, a.st, p->n);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
-        if ((e = cudaStreamGetCaptureInfo(cs, &status, nullptr, &cg, &deps, &nd)) != cudaSuccess)
-          break;
-        cudaGraphNodeParams ip = {};
-        ip.type = cudaGraphNodeTypeConditional;
-        ip.conditional.handle = hr;
-        ip.conditional.type = cudaGraphCondTypeIf;
-        ip.conditional.size = 1;
-        cudaGraphNode_t in;
-        if ((e = cudaGraphAddNode(&in, cg, deps, nd, &ip)) != cudaSuccess) break;
-        refresh_body = ip.conditional.phGraph_out[0];
-        if ((e = cudaStreamUpdateCaptureDependencies(cs, &in, 1,
-                                                     cudaStreamSetCaptureDependencies)) !=
-            cudaSuccess)
-          break;
-        k_loop_gate<<<1, 32, 0, cs>>>(h, a.n_active, trips, 0, cap);
-        e = cudaGetLastError();
+        e = add_conditional(a.refresh, cudaGraphCondTypeIf, &refresh_body);
       } while (0);
       cudaGraph_t bg = nullptr;
       const cudaError_t eb = cudaStreamEndCapture(cs, &bg);
@@ -1285,12 +1250,12 @@ int enqueue_solve(gd_plan p, cudaStream_t st) {
   const bool graph = p->prm.use_graph && !p->profiling && p->solves >= 1;
   if (graph) {
     if (!p->gexec) {
-      int rc = build_solve_graph<T>(p, a, fine);
+      int rc = build_solve_graph<T>(p, a);
       if (rc != GD_OK && p->persistent) {
         // a graph that cannot hold the cooperative launch: levels one by one
         cudaGetLastError();
         p->persistent = false;
-        rc = build_solve_graph<T>(p, a, fine);
+        rc = build_solve_graph<T>(p, a);
       }
       if (rc != GD_OK) return rc;
     }

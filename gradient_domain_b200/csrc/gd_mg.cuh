@@ -125,7 +125,21 @@ struct Args {
   double tol2, delta2;
   int max_iter;
   int zero_start;  // solves start from x = 0 without reading the caller's x
+  // Conditional handles of the solve graph (0 in direct launches): the loop over
+  // iterations, set by the initial residual while an instance is active and
+  // cleared by the refresh that stops the last one; and the FP64 refresh of an
+  // iteration, set by whoever asks for one (FLAG_RU) and cleared by the refresh.
+  // trips counts the loop's iterations and ends it at trip_cap, whatever the
+  // states say.
+  cudaGraphConditionalHandle loop, refresh;
+  int *trips;
+  int trip_cap;
 };
+
+// Sets a condition of the solve graph (nothing in direct launches).
+__device__ __forceinline__ void set_condition(cudaGraphConditionalHandle h, unsigned value) {
+  if (h) cudaGraphSetConditional(h, value);
+}
 
 // Cell class: 0 = no unknown, else 1 + number of walls (missing neighbours).
 __host__ __device__ __forceinline__ int rect_class(int y, int x, int ny, int nx) {

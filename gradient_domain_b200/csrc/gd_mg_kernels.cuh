@@ -80,10 +80,12 @@ __device__ __forceinline__ long long p_offset(const InstInfo &I, int which) {
   return which ? I.q_off : I.p_off;
 }
 
-__device__ __forceinline__ void finish_rz(InstState &S, double rz) {
+__device__ __forceinline__ void finish_rz(InstState &S, double rz,
+                                          cudaGraphConditionalHandle refresh) {
   if (!(rz > 0.0) || !isfinite(rz)) {
     S.status = GD_BREAKDOWN;
     S.flags |= FLAG_RU;
+    set_condition(refresh, 1u);
     return;
   }
   S.beta = S.first ? 0.0 : rz / S.rz;
@@ -363,7 +365,7 @@ __device__ __forceinline__ void bottom_instance(const Args<T> &a, const int inst
   }
   if (top_is_fine) {
     part = block_sum<kBThreads>(part);
-    if (threadIdx.x == 0) finish_rz(S, part);
+    if (threadIdx.x == 0) finish_rz(S, part, a.refresh);
   }
 }
 
@@ -411,6 +413,7 @@ __global__ void __launch_bounds__(kFThreads) k_fmean(Args<T> a) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {  // a solve starts
     a.counter[kErrWord] = 0u;
     *a.n_active = 0;
+    *a.trips = 0;
   }
   const InstInfo &I = a.inst[tl.inst];
   if (!I.zero_mean) {

@@ -1390,7 +1390,7 @@ __global__ void __launch_bounds__(UpCta<LEVEL0>::NT,
   if (!last_of_instance(&S.ticket, I.up0_ctas)) return;
   const double rz = block_range_sum<UpCta<LEVEL0>::NT>(a.part0 + I.up0_begin,
                                                        I.up0_end - I.up0_begin);
-  if (threadIdx.x == 0) finish_rz(S, rz);
+  if (threadIdx.x == 0) finish_rz(S, rz, a.refresh);
 }
 
 // ---------------------------------------------------------------------------
@@ -1772,6 +1772,7 @@ template <typename T, bool INIT>
 __global__ void __launch_bounds__(kThreads, 4) k_refresh_s(Args<T> a) {
   const Tile tl = a.tiles[blockIdx.x];
   dep_enter();
+  if (!INIT && blockIdx.x == 0 && threadIdx.x == 0) set_condition(a.refresh, 0u);
   const int flags = a.st[tl.inst].flags;
   const bool work = INIT || (flags & FLAG_RU);
   double part = 0.0, part_f = 0.0;
@@ -1887,8 +1888,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_refresh_s(Args<T> a) {
   // the instances still iterating: counted up by the initial residual (k_fmean
   // starts from zero) and down by the refresh that stops one.  Every instance a
   // refresh works on was counted: only counted instances ask for one.
-  if (INIT && S.status == GD_ACTIVE) atomicAdd(a.n_active, 1);
-  if (!INIT && S.status != GD_ACTIVE) atomicSub(a.n_active, 1);
+  if (INIT && S.status == GD_ACTIVE) {
+    atomicAdd(a.n_active, 1);
+    set_condition(a.loop, 1u);
+  }
+  if (!INIT && S.status != GD_ACTIVE && atomicSub(a.n_active, 1) == 1) set_condition(a.loop, 0u);
 }
 
 }  // namespace st
