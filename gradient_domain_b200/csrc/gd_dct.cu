@@ -4,13 +4,11 @@
 // on the device with this library's own FFT kernels.
 //
 // Three passes over HBM, each CTA working on two lines (rows or columns) at
-// once, held in shared memory as one complex sequence z = a + i b:
+// once as one complex sequence z = a + i b:
 //   rows:    load two rows of b, DCT-II along x, write the coefficients to T;
 //   columns: load two columns of T, DCT-II along y, divide by the
 //            eigenvalues, inverse transform (DCT-III) along y, write back;
 //   rows:    load two rows of T, DCT-III along x, write u.
-// so b is read once, u written once and T read and written twice: 48 bytes
-// per cell against 16 for b and u alone.
 //
 // One DCT-II of length N is one complex FFT of length N (Makhoul's
 // reordering v = (x0, x2, x4, ..., x5, x3, x1), X_k = Re(e^{-i pi k/2N} V_k));
@@ -22,13 +20,26 @@
 // forward / inverse pair is exact either way and the solve only divides by
 // the eigenvalues in between.
 //
-// The FFT is a mixed-radix transform in place in shared memory: forward
-// passes decimate in frequency (natural order in, digit-reversed order out),
-// inverse passes decimate in time (digit-reversed in, natural out), so no
-// reordering pass is needed between them.  Radices 8, 4 and 2 have dedicated
-// butterflies, 3, 5 and 7 a small direct DFT per butterfly, and any larger
-// prime factor a direct DFT computed one output per thread.  Twiddles come
-// from per-plan tables of e^{-2 pi i m / N} computed with sincospi at bind.
+// Layout of T.  T[c][p] is the pair of columns 2c, 2c + 1 of the row at place p
+// of the reordering along y, 16 bytes, p fastest.  The column pass then reads
+// and writes contiguous memory in exactly the order its FFT wants, and since a
+// row CTA takes the rows at places 2p and 2p + 1, what it reads or writes for a
+// column pair is one whole 32-byte sector.  (With T stored row by row the column
+// pass used half of every sector: 284 us a channel at 4096 x 4096.)
+//
+// The FFTs are mixed-radix, forward passes decimating in frequency (natural
+// order in, digit-reversed out), inverse passes in time (digit-reversed in,
+// natural out).  What bounds them is FP64 arithmetic and shared-memory
+// bandwidth, so passes are few and large (radices up to 16), the first forward
+// pass takes its operands straight from global memory, and the last inverse one
+// writes its results there.  Lengths 512 .. 8192 that are powers of two run
+// kernels whose every index is known at compile time, one radix-16 butterfly per
+// thread and pass, with the values in registers from the loads to the
+// coefficients: 3 passes and 2 exchanges for 4096 where radix 8 with staging
+// took 4 passes and 6.  Other lengths take the radices of the cheapest
+// factorisation (choose_passes) at run time.  Measured per channel, rows + columns
+// + rows: 4096 x 4096 72 + 117 + 84 us (88 + 284 + 111 before), 1080 x 1920
+// 26 + 41 + 23 us (54 + 82 + 44).
 
 #include <algorithm>
 #include <cstdint>
@@ -40,42 +51,117 @@ namespace gd {
 namespace dct {
 
 constexpr int kMaxLen = 8192;   // longest line (128 KB of complex values in shared memory)
-constexpr int kMaxStages = 16;  // 8192 = 8^4 * 2
-constexpr int kThreads = 256;
-constexpr int kMaxPerThread = kMaxLen / kThreads;  // outputs per thread of a large-prime stage
+constexpr int kMaxPasses = 14;
+constexpr int kThreads = 256;   // most threads of the run-time kernels; the large-prime ones' size
+constexpr int kMaxPerThread = kMaxLen / kThreads;  // outputs per thread of a large-prime pass
 
-// Radix sequence of one transform length, largest radices first.
-struct Radices {
-  int n = 0, count = 0;
-  int r[kMaxStages] = {0};
+// One pass of a run-time transform: radix r on sub-transforms of length r m;
+// step = N / (r m); div = ceil(2^32 / m) divides butterfly numbers by m.
+struct Pass {
+  int r, m, step;
+  unsigned div;
 };
 
-inline Radices factor(int n) {
+struct Radices {
+  int n = 0, count = 0;
+  Pass p[kMaxPasses] = {};
+};
+
+// FP64 instructions per point of one pass of radix r (butterfly and twiddles,
+// counted from the code below), plus what a pass costs besides: its exchange
+// through shared memory and its barrier, worth about eight instructions a point.
+inline double pass_cost(int r) {
+  switch (r) {
+    case 2: return 8 + 4.0;
+    case 3: return 8 + 9.0;
+    case 4: return 8 + 9.0;
+    case 5: return 8 + 13.0;
+    case 6: return 8 + 11.0;
+    case 7: return 8 + 17.0;
+    case 8: return 8 + 13.0;
+    case 9: return 8 + 16.0;
+    case 10: return 8 + 15.0;
+    case 11: return 8 + 24.0;
+    case 12: return 8 + 14.0;
+    case 13: return 8 + 28.0;
+    case 14: return 8 + 19.0;
+    case 15: return 8 + 18.0;
+    case 16: return 8 + 17.0;
+    default: return 8 + 10.0 * r;  // a prime above 13: direct
+  }
+}
+
+// Radices of the cheapest factorisation of n, primes above 13 on their own.
+inline double cheapest(int n, int *first) {
+  double best = -1.0;
+  *first = n;
+  if (n == 1) return 0.0;
+  auto consider = [&](int r) {
+    int rest;
+    const double c = pass_cost(r) + cheapest(n / r, &rest);
+    if (best < 0.0 || c < best) {
+      best = c;
+      *first = r;
+    }
+  };
+  for (int r = 16; r >= 2; --r)
+    if (n % r == 0) consider(r);
+  if (best >= 0.0) return best;
+  int q = 17;
+  while (q * q <= n && n % q) q += 2;
+  consider(n % q ? n : q);
+  return best;
+}
+
+inline Radices choose_passes(int n) {
   Radices f;
   f.n = n;
-  int m = n;
-  auto push = [&](int r) { f.r[f.count++] = r; m /= r; };
-  while (m % 8 == 0) push(8);
-  if (m % 4 == 0) push(4);
-  if (m % 2 == 0) push(2);
-  for (int p = 3; m > 1; p += 2)
-    while (m % p == 0) push(p);
+  int r[kMaxPasses], count = 0;
+  for (int m = n; m > 1;) {
+    int first;
+    cheapest(m, &first);
+    r[count++] = first;
+    m /= first;
+  }
+  std::sort(r, r + count, [](int a, int b) { return a > b; });
+  int L = n;
+  for (int s = 0; s < count; ++s) {
+    const int m = L / r[s];
+    f.p[s] = Pass{r[s], m, n / L, m > 1 ? (unsigned)((0x100000000ull + m - 1) / m) : 0u};
+    L = m;
+  }
+  f.count = count;
   return f;
 }
 
-// Per-axis tables: FFT twiddles e^{-2 pi i m / N} (N entries), the DCT
-// twiddles e^{-i pi k / 2N} (N entries) and the eigenvalue terms
-// 2 cos(pi k / N) (N entries).  The eigenvalue of mode (i, j) is formed as
-// (2 cos(pi i / m) + 2 cos(pi j / n)) - 4 with cos(pi k / N) evaluated from the
-// rounded product pi k, as solvers.py:253-258 does: the smallest eigenvalues
-// cancel most of their digits in that sum, and the solution's smoothest modes
-// carry that rounding, so the same expression keeps the result within
-// rounding of the reference's.
+inline bool has_large_prime(const Radices &r) {
+  for (int s = 0; s < r.count; ++s)
+    if (r.p[s].r > 16) return true;
+  return false;
+}
+
+// Threads of a run-time kernel: one butterfly each in the pass that has most.
+inline int gen_threads(const Radices &r) {
+  if (has_large_prime(r)) return kThreads;
+  int most = 1;
+  for (int s = 0; s < r.count; ++s) most = std::max(most, r.n / r.p[s].r);
+  return std::min(kThreads, (most + 31) / 32 * 32);
+}
+
+// Per-axis tables: FFT twiddles e^{-2 pi i m / N}, the DCT twiddles
+// e^{-i pi k / 2N}, the eigenvalue terms 2 cos(pi k / N) and the place of
+// frequency k in the digit-reversed output (N entries each).  The eigenvalue of
+// mode (i, j) is formed as (2 cos(pi i / m) + 2 cos(pi j / n)) - 4 with
+// cos(pi k / N) evaluated from the rounded product pi k, as solvers.py:253-258
+// does: the smallest eigenvalues cancel most of their digits in that sum, and
+// the solution's smoothest modes carry that rounding, so the same expression
+// keeps the result within rounding of the reference's.
 struct Axis {
   Radices rad;
   const double2 *tw;
   const double2 *post;
   const double *eig;
+  const unsigned short *rev;
 };
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
@@ -95,6 +181,11 @@ template <int SIGN>
 __device__ __forceinline__ double2 rot90(double2 a) {
   return SIGN < 0 ? make_double2(a.y, -a.x) : make_double2(-a.y, a.x);
 }
+// multiply by c + SIGN i s
+template <int SIGN>
+__device__ __forceinline__ double2 rot(double2 a, double c, double s) {
+  return make_double2(c * a.x - SIGN * s * a.y, c * a.y + SIGN * s * a.x);
+}
 
 // In-register DFTs y_q = sum_j x_j e^{SIGN 2 pi i j q / R}, natural order.
 template <int SIGN>
@@ -105,24 +196,23 @@ __device__ __forceinline__ void dft2(double2 &a, double2 &b) {
 }
 
 template <int SIGN>
-__device__ __forceinline__ void dft4(double2 (&x)[4]) {
-  double2 a0 = cadd(x[0], x[2]), a1 = csub(x[0], x[2]);
-  double2 b0 = cadd(x[1], x[3]), b1 = rot90<SIGN>(csub(x[1], x[3]));
-  x[0] = cadd(a0, b0);
-  x[2] = csub(a0, b0);
-  x[1] = cadd(a1, b1);
-  x[3] = csub(a1, b1);
+__device__ __forceinline__ void dft4(double2 &x0, double2 &x1, double2 &x2, double2 &x3) {
+  const double2 a0 = cadd(x0, x2), a1 = csub(x0, x2);
+  const double2 b0 = cadd(x1, x3), b1 = rot90<SIGN>(csub(x1, x3));
+  x0 = cadd(a0, b0);
+  x2 = csub(a0, b0);
+  x1 = cadd(a1, b1);
+  x3 = csub(a1, b1);
 }
 
 template <int SIGN>
 __device__ __forceinline__ void dft8(double2 (&x)[8]) {
   constexpr double h = 0.70710678118654752440;  // sqrt(1/2)
   // two DFT-4 of the even and odd samples, then the radix-2 combination
-  double2 e[4] = {x[0], x[2], x[4], x[6]};
+  dft4<SIGN>(x[0], x[2], x[4], x[6]);
+  dft4<SIGN>(x[1], x[3], x[5], x[7]);
+  const double2 e[4] = {x[0], x[2], x[4], x[6]};
   double2 o[4] = {x[1], x[3], x[5], x[7]};
-  dft4<SIGN>(e);
-  dft4<SIGN>(o);
-  // o_q *= e^{SIGN 2 pi i q / 8}
   o[1] = make_double2(h * (o[1].x - SIGN * o[1].y), h * (o[1].y + SIGN * o[1].x));
   o[2] = rot90<SIGN>(o[2]);
   o[3] = make_double2(h * (-o[3].x - SIGN * o[3].y), h * (-o[3].y + SIGN * o[3].x));
@@ -133,76 +223,629 @@ __device__ __forceinline__ void dft8(double2 (&x)[8]) {
   }
 }
 
-// Direct DFT of a small odd radix, roots of unity from the length-N table.
-template <int R, int SIGN>
-__device__ __forceinline__ void dft_odd(double2 (&x)[R], const double2 *tw, int n) {
-  double2 y[R];
-  const int s = n / R;
-#pragma unroll
-  for (int q = 0; q < R; ++q) {
-    double2 acc = x[0];
-#pragma unroll
-    for (int j = 1; j < R; ++j) {
-      const double2 w = tw[((j * q) % R) * s];
-      acc = cadd(acc, SIGN < 0 ? cmul(x[j], w) : cmulc(x[j], w));
-    }
-    y[q] = acc;
-  }
-#pragma unroll
-  for (int q = 0; q < R; ++q) x[q] = y[q];
-}
-
-template <int R, int SIGN>
-__device__ __forceinline__ void dft_small(double2 (&x)[R], const double2 *tw, int n) {
-  if constexpr (R == 2) dft2<SIGN>(x[0], x[1]);
-  else if constexpr (R == 4) dft4<SIGN>(x);
-  else if constexpr (R == 8) dft8<SIGN>(x);
-  else dft_odd<R, SIGN>(x, tw, n);
-}
-
-// One decimation-in-frequency pass of radix R on sub-transforms of length L:
-// each butterfly reads R values spaced L/R apart, transforms them and
-// multiplies output q by e^{-2 pi i q k / L}.  A thread owns whole butterflies,
-// so the pass is in place.
-template <int R>
-__device__ void dif_pass(double2 *z, int n, int L, const double2 *tw) {
-  const int m = L / R, step = n / L;
-  for (int t = threadIdx.x; t < n / R; t += blockDim.x) {
-    const int blk = t / m, k = t - blk * m;
-    double2 *p = z + blk * L + k;
-    double2 x[R];
-#pragma unroll
-    for (int j = 0; j < R; ++j) x[j] = p[j * m];
-    dft_small<R, -1>(x, tw, n);
-    p[0] = x[0];
-#pragma unroll
-    for (int q = 1; q < R; ++q) p[q * m] = cmul(x[q], tw[q * k * step]);
-  }
-}
-
-// The inverse: decimation in time on sub-transforms of length L = R m; input
-// q is multiplied by e^{+2 pi i q k / L} before the DFT.
-template <int R>
-__device__ void dit_pass(double2 *z, int n, int L, const double2 *tw) {
-  const int m = L / R, step = n / L;
-  for (int t = threadIdx.x; t < n / R; t += blockDim.x) {
-    const int blk = t / m, k = t - blk * m;
-    double2 *p = z + blk * L + k;
-    double2 x[R];
-    x[0] = p[0];
-#pragma unroll
-    for (int q = 1; q < R; ++q) x[q] = cmulc(p[q * m], tw[q * k * step]);
-    dft_small<R, 1>(x, tw, n);
-#pragma unroll
-    for (int j = 0; j < R; ++j) p[j * m] = x[j];
-  }
-}
-
-// A pass of a prime radix above 7: one output per thread and step, computed
-// into registers from the whole butterfly, then written back after a barrier.
+// 4 x 4: DFT-4 over samples a, a + 4, a + 8, a + 12, twiddles e^{SIGN 2 pi i a b / 16},
+// DFT-4 over a; output b + 4 c.
 template <int SIGN>
-__device__ void prime_pass(double2 *z, int n, int L, int r, const double2 *tw) {
-  const int m = L / r, step = n / L, s = n / r;
+__device__ __forceinline__ void dft16(double2 (&x)[16]) {
+  constexpr double c1 = 0.9238795325112867, s1 = 0.3826834323650898, h = 0.70710678118654752440;
+#pragma unroll
+  for (int a = 0; a < 4; ++a) dft4<SIGN>(x[a], x[a + 4], x[a + 8], x[a + 12]);
+  // x[a + 4 b] now holds G[a][b]
+  x[5] = rot<SIGN>(x[5], c1, s1);
+  x[9] = make_double2(h * (x[9].x - SIGN * x[9].y), h * (x[9].y + SIGN * x[9].x));
+  x[13] = rot<SIGN>(x[13], s1, c1);
+  x[6] = make_double2(h * (x[6].x - SIGN * x[6].y), h * (x[6].y + SIGN * x[6].x));
+  x[10] = rot90<SIGN>(x[10]);
+  x[14] = make_double2(h * (-x[14].x - SIGN * x[14].y), h * (-x[14].y + SIGN * x[14].x));
+  x[7] = rot<SIGN>(x[7], s1, c1);
+  x[11] = make_double2(h * (-x[11].x - SIGN * x[11].y), h * (-x[11].y + SIGN * x[11].x));
+  x[15] = rot<SIGN>(x[15], -c1, -s1);
+#pragma unroll
+  for (int b = 0; b < 4; ++b) dft4<SIGN>(x[4 * b], x[4 * b + 1], x[4 * b + 2], x[4 * b + 3]);
+  // x[4 b + c] holds output b + 4 c: transpose in registers
+#pragma unroll
+  for (int b = 0; b < 4; ++b)
+#pragma unroll
+    for (int c = b + 1; c < 4; ++c) {
+      const double2 t = x[4 * b + c];
+      x[4 * b + c] = x[4 * c + b];
+      x[4 * c + b] = t;
+    }
+}
+
+// Odd primes by the symmetric sums and differences of the samples j and P - j.
+template <int P>
+struct Roots;  // cos and sin of 2 pi j / P, j = 1 .. (P - 1) / 2
+template <>
+struct Roots<3> {
+  static __device__ __forceinline__ double c(int) { return -0.5; }
+  static __device__ __forceinline__ double s(int) { return 0.8660254037844386; }
+};
+template <>
+struct Roots<5> {
+  static __device__ __forceinline__ double c(int j) {
+    return j == 1 ? 0.30901699437494745 : -0.8090169943749475;
+  }
+  static __device__ __forceinline__ double s(int j) {
+    return j == 1 ? 0.9510565162951535 : 0.5877852522924731;
+  }
+};
+template <>
+struct Roots<7> {
+  static __device__ __forceinline__ double c(int j) {
+    return j == 1 ? 0.6234898018587335 : j == 2 ? -0.2225209339563144 : -0.9009688679024191;
+  }
+  static __device__ __forceinline__ double s(int j) {
+    return j == 1 ? 0.7818314824680298 : j == 2 ? 0.9749279121818236 : 0.4338837391175581;
+  }
+};
+template <>
+struct Roots<11> {
+  static __device__ __forceinline__ double c(int j) {
+    return j == 1   ? 0.8412535328311812
+           : j == 2 ? 0.41541501300188644
+           : j == 3 ? -0.14231483827328514
+           : j == 4 ? -0.6548607339452851
+                    : -0.9594929736144974;
+  }
+  static __device__ __forceinline__ double s(int j) {
+    return j == 1   ? 0.5406408174555976
+           : j == 2 ? 0.9096319953545183
+           : j == 3 ? 0.9898214418809327
+           : j == 4 ? 0.7557495743542583
+                    : 0.28173255684142967;
+  }
+};
+template <>
+struct Roots<13> {
+  static __device__ __forceinline__ double c(int j) {
+    return j == 1   ? 0.8854560256532099
+           : j == 2 ? 0.5680647467311558
+           : j == 3 ? 0.12053668025532305
+           : j == 4 ? -0.3546048870425356
+           : j == 5 ? -0.7485107481711011
+                    : -0.970941817426052;
+  }
+  static __device__ __forceinline__ double s(int j) {
+    return j == 1   ? 0.46472317204376856
+           : j == 2 ? 0.8229838658936564
+           : j == 3 ? 0.992708874098054
+           : j == 4 ? 0.9350162426854148
+           : j == 5 ? 0.6631226582407952
+                    : 0.23931566428755777;
+  }
+};
+
+template <int P, int SIGN>
+__device__ __forceinline__ void dft_prime(double2 (&x)[P]) {
+  constexpr int H = (P - 1) / 2;
+  double2 t[H], d[H];
+  double2 sum = x[0];
+#pragma unroll
+  for (int j = 0; j < H; ++j) {
+    t[j] = cadd(x[j + 1], x[P - 1 - j]);
+    d[j] = csub(x[j + 1], x[P - 1 - j]);
+    sum = cadd(sum, t[j]);
+  }
+  const double2 x0 = x[0];
+#pragma unroll
+  for (int k = 1; k <= H; ++k) {
+    double2 a = x0, b = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int j = 1; j <= H; ++j) {
+      const int e = (j * k) % P;                  // e^{2 pi i e / P}
+      const int f = e <= H ? e : P - e;           // table index
+      const double c = Roots<P>::c(f), s = e <= H ? Roots<P>::s(f) : -Roots<P>::s(f);
+      a.x += c * t[j - 1].x;
+      a.y += c * t[j - 1].y;
+      b.x += s * d[j - 1].x;
+      b.y += s * d[j - 1].y;
+    }
+    // X_k = a + SIGN i b, X_{P-k} = a - SIGN i b
+    x[k] = make_double2(a.x - SIGN * b.y, a.y + SIGN * b.x);
+    x[P - k] = make_double2(a.x + SIGN * b.y, a.y - SIGN * b.x);
+  }
+  x[0] = sum;
+}
+
+template <int R, int SIGN>
+__device__ __forceinline__ void dft(double2 (&x)[R]);
+
+// A B with coprime factors (Good-Thomas): no twiddles between the two sets of DFTs.
+template <int A, int B, int SIGN>
+__device__ __forceinline__ void dft_coprime(double2 (&x)[A * B]) {
+  constexpr int R = A * B;
+  double2 g[A][B];
+#pragma unroll
+  for (int n1 = 0; n1 < A; ++n1) {
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) g[n1][n2] = x[(B * n1 + A * n2) % R];
+    dft<B, SIGN>(g[n1]);
+  }
+  constexpr auto inverse = [](int a, int m) {  // a^-1 mod m
+    for (int i = 1; i < m; ++i)
+      if ((a * i) % m == 1) return i;
+    return 1;
+  };
+  constexpr int ea = B * inverse(B % A, A), eb = A * inverse(A % B, B);
+#pragma unroll
+  for (int k2 = 0; k2 < B; ++k2) {
+    double2 y[A];
+#pragma unroll
+    for (int n1 = 0; n1 < A; ++n1) y[n1] = g[n1][k2];
+    dft<A, SIGN>(y);
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) x[(k1 * ea + k2 * eb) % R] = y[k1];
+  }
+}
+
+template <int SIGN>
+__device__ __forceinline__ void dft9(double2 (&x)[9]) {
+  double2 g[3][3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+#pragma unroll
+    for (int b = 0; b < 3; ++b) g[a][b] = x[a + 3 * b];
+    dft_prime<3, SIGN>(g[a]);
+  }
+  g[1][1] = rot<SIGN>(g[1][1], 0.766044443118978, 0.6427876096865394);
+  g[1][2] = rot<SIGN>(g[1][2], 0.17364817766693036, 0.984807753012208);
+  g[2][1] = rot<SIGN>(g[2][1], 0.17364817766693036, 0.984807753012208);
+  g[2][2] = rot<SIGN>(g[2][2], -0.9396926207859084, 0.3420201433256687);
+#pragma unroll
+  for (int b = 0; b < 3; ++b) {
+    double2 y[3] = {g[0][b], g[1][b], g[2][b]};
+    dft_prime<3, SIGN>(y);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) x[b + 3 * c] = y[c];
+  }
+}
+
+template <int R, int SIGN>
+__device__ __forceinline__ void dft(double2 (&x)[R]) {
+  if constexpr (R == 2) dft2<SIGN>(x[0], x[1]);
+  else if constexpr (R == 4) dft4<SIGN>(x[0], x[1], x[2], x[3]);
+  else if constexpr (R == 8) dft8<SIGN>(x);
+  else if constexpr (R == 16) dft16<SIGN>(x);
+  else if constexpr (R == 9) dft9<SIGN>(x);
+  else if constexpr (R == 6) dft_coprime<2, 3, SIGN>(x);
+  else if constexpr (R == 10) dft_coprime<2, 5, SIGN>(x);
+  else if constexpr (R == 12) dft_coprime<4, 3, SIGN>(x);
+  else if constexpr (R == 14) dft_coprime<2, 7, SIGN>(x);
+  else if constexpr (R == 15) dft_coprime<3, 5, SIGN>(x);
+  else if constexpr (R > 1) dft_prime<R, SIGN>(x);
+}
+
+// x[q] *= w^q (forward) or conj(w)^q (inverse), q < R, the powers from w by
+// products: four at a time from the last multiple of w^4, so that few are live.
+template <int R, int SIGN>
+__device__ __forceinline__ void twiddle(double2 (&x)[R], double2 w1) {
+  auto mul = [](double2 a, double2 t) { return SIGN < 0 ? cmul(a, t) : cmulc(a, t); };
+  if constexpr (R > 1) x[1] = mul(x[1], w1);
+  if constexpr (R > 2) {
+    const double2 w2 = cmul(w1, w1);
+    x[2] = mul(x[2], w2);
+    if constexpr (R > 3) {
+      const double2 w3 = cmul(w2, w1);
+      x[3] = mul(x[3], w3);
+      if constexpr (R > 4) {
+        const double2 w4 = cmul(w2, w2);
+        double2 base = w4;
+#pragma unroll
+        for (int b = 4; b < R; b += 4) {
+          x[b] = mul(x[b], base);
+          if (b + 1 < R) x[b + 1] = mul(x[b + 1], cmul(base, w1));
+          if (b + 2 < R) x[b + 2] = mul(x[b + 2], cmul(base, w2));
+          if (b + 3 < R) x[b + 3] = mul(x[b + 3], cmul(base, w3));
+          if (b + 4 < R) base = cmul(base, w4);
+        }
+      }
+    }
+  }
+}
+
+// Shared-memory slot of element idx.  A warp's 16-byte accesses are served eight
+// lanes at a time, without conflict when the eight hit different slots modulo
+// eight; storing element idx at idx ^ (XOR of the octal digits above the lowest)
+// gives that to any eight elements that differ in three consecutive index bits,
+// so to every butterfly stride of a power-of-two length.  at(i ^ j) = at(i) ^ at(j).
+__device__ __forceinline__ int fold(int idx) {
+  const int x = idx >> 3;
+  return (x ^ (x >> 3) ^ (x >> 6) ^ (x >> 9)) & 7;
+}
+__device__ __forceinline__ int at(int idx) { return idx ^ fold(idx); }
+
+// Where sample j of a line sits in Makhoul's even/odd reordering, and the sample
+// at place p.
+__device__ __forceinline__ int mak_sample(int p, int n) {
+  return p < (n + 1) / 2 ? 2 * p : 2 * (n - 1 - p) + 1;
+}
+
+// Forward DCT coefficients of the two lines packed in Z, at frequency k and
+// its partner n - k (k in 1 .. n-1): X_a[k], X_b[k], X_a[n-k], X_b[n-k].
+struct Coef4 {
+  double ak, bk, an, bn;
+};
+
+// tk = e^{-i pi k / 2n}; its partner e^{-i pi (n-k) / 2n} is (-tk.y, -tk.x)
+__device__ __forceinline__ Coef4 split(double2 zk, double2 zn, double2 tk) {
+  // A_k = (Z_k + conj Z_{n-k}) / 2, B_k = (Z_k - conj Z_{n-k}) / 2i; A_{n-k} = conj A_k
+  const double2 A = make_double2(0.5 * (zk.x + zn.x), 0.5 * (zk.y - zn.y));
+  const double2 B = make_double2(0.5 * (zk.y + zn.y), 0.5 * (zn.x - zk.x));
+  Coef4 c;
+  c.ak = tk.x * A.x - tk.y * A.y;   // Re(t_k A_k)
+  c.bk = tk.x * B.x - tk.y * B.y;
+  c.an = -tk.y * A.x - tk.x * A.y;  // Re(t_{n-k} conj A_k)
+  c.bn = -tk.y * B.x - tk.x * B.y;
+  return c;
+}
+
+// W_k = conj(t_k) (X_k - i X_{n-k}) for both lines, packed as W_a + i W_b.
+__device__ __forceinline__ double2 pack_inverse(double xa, double xan, double xb, double xbn,
+                                                double2 tk) {
+  // conj(t) (x - i y) = (c + i s)(x - i y) with t = c - i s
+  const double c = tk.x, s = -tk.y;
+  const double2 wa = make_double2(c * xa + s * xan, s * xa - c * xan);
+  const double2 wb = make_double2(c * xb + s * xbn, s * xb - c * xbn);
+  return make_double2(wa.x - wb.y, wa.y + wb.x);
+}
+
+// The two rows of a row CTA: places 2p and 2p + 1 of the reordering along y.
+struct RowPair {
+  int p0, ra, rb;
+  bool two;
+  __device__ __forceinline__ explicit RowPair(int h) {
+    p0 = 2 * blockIdx.x;
+    two = p0 + 1 < h;
+    ra = mak_sample(p0, h);
+    rb = two ? mak_sample(p0 + 1, h) : ra;
+  }
+};
+
+// ---------------------------------------------------------------------------
+// Powers of two, 512 .. 8192: N / 16 threads, sixteen values each.
+// Passes: radix 16 while the sub-transform allows, the last of radix 2^(LOG mod 4)
+// (or 16).  After the forward passes thread t holds the frequencies t + TP i.
+template <int LOG>
+struct P2 {
+  static constexpr int N = 1 << LOG, TP = N / 16;
+  static constexpr int REM = LOG % 4 ? LOG % 4 : 4;
+  static constexpr int LR = 1 << REM;               // radix of the last pass
+  static constexpr int G = 16 / LR;                 // its butterflies per thread
+  static constexpr int MID = (LOG - REM) / 4 - 1;   // radix-16 passes after the first
+  static constexpr size_t smem = (size_t)N * sizeof(double2);
+
+  // e^{-2 pi i k / L} of this thread's butterfly in the first pass and the middle ones
+  struct Twiddles {
+    double2 w[MID + 1];
+    __device__ __forceinline__ explicit Twiddles(const double2 *tw) {
+      const int t = threadIdx.x;
+      w[0] = tw[t];
+#pragma unroll
+      for (int s = 1; s <= MID; ++s) w[s] = tw[(t & ((TP >> (4 * s)) - 1)) << (4 * s)];
+    }
+  };
+  // first element of this thread's butterfly in middle pass s (stride TP >> 4 s)
+  template <int S>
+  static __device__ __forceinline__ int mid_base() {
+    constexpr int M = TP >> (4 * S);
+    const int t = threadIdx.x;
+    return ((t & ~(M - 1)) << 4) | (t & (M - 1));
+  }
+  // place of frequency f (< N / LR) in the digit-reversed order
+  static __device__ __forceinline__ int last_base(int f) {
+    int pos = 0;
+#pragma unroll
+    for (int s = 0; s <= MID; ++s) pos |= ((f >> (4 * s)) & 15) << (LOG - 4 * s - 4);
+    return pos;
+  }
+  template <int SIGN, int S>
+  static __device__ __forceinline__ void mid_pass(double2 *z, const Twiddles &tw) {
+    constexpr int M = TP >> (4 * S);
+    const int b = at(mid_base<S>());
+    double2 x[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = z[b ^ at(j * M)];
+    if constexpr (SIGN > 0) twiddle<16, 1>(x, tw.w[S]);
+    dft16<SIGN>(x);
+    if constexpr (SIGN < 0) twiddle<16, -1>(x, tw.w[S]);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) z[b ^ at(j * M)] = x[j];
+    __syncthreads();
+  }
+  // x[j] = v[t + TP j] -> x[i] = V[t + TP i]; the shared memory may be in use by
+  // this thread's own columns (places = t mod TP) on entry
+  static __device__ __forceinline__ void forward(double2 (&x)[16], double2 *z,
+                                                 const Twiddles &tw) {
+    const int b = at(threadIdx.x);
+    dft16<-1>(x);
+    twiddle<16, -1>(x, tw.w[0]);
+#pragma unroll
+    for (int q = 0; q < 16; ++q) z[b ^ at(q * TP)] = x[q];
+    __syncthreads();
+    if constexpr (MID >= 1) mid_pass<-1, 1>(z, tw);
+    if constexpr (MID >= 2) mid_pass<-1, 2>(z, tw);
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const int p = last_base(threadIdx.x + TP * g);
+      double2 y[LR];
+#pragma unroll
+      for (int j = 0; j < LR; ++j) y[j] = z[at(p + j)];
+      dft<LR, -1>(y);
+#pragma unroll
+      for (int q = 0; q < LR; ++q) x[g + G * q] = y[q];
+    }
+    __syncthreads();
+  }
+  // the inverse (unscaled); the shared memory is free on entry
+  static __device__ __forceinline__ void inverse(double2 (&x)[16], double2 *z,
+                                                 const Twiddles &tw) {
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const int p = last_base(threadIdx.x + TP * g);
+      double2 y[LR];
+#pragma unroll
+      for (int q = 0; q < LR; ++q) y[q] = x[g + G * q];
+      dft<LR, 1>(y);
+#pragma unroll
+      for (int j = 0; j < LR; ++j) z[at(p + j)] = y[j];
+    }
+    __syncthreads();
+    if constexpr (MID >= 2) mid_pass<1, 2>(z, tw);
+    if constexpr (MID >= 1) mid_pass<1, 1>(z, tw);
+    const int b = at(threadIdx.x);
+#pragma unroll
+    for (int q = 0; q < 16; ++q) x[q] = z[b ^ at(q * TP)];
+    twiddle<16, 1>(x, tw.w[0]);
+    dft16<1>(x);
+  }
+};
+
+// e^{-i pi i / 32}, i = 0 .. 15: the DCT twiddle of frequency t + TP i is that of t times it.
+__device__ __forceinline__ double2 c32(int i) {
+  constexpr double c[17] = {1.0, 0.9951847266721969, 0.9807852804032304, 0.9569403357322088,
+                            0.9238795325112867, 0.881921264348355, 0.8314696123025452,
+                            0.773010453362737, 0.7071067811865476, 0.6343932841636455,
+                            0.5555702330196022, 0.47139673682599764, 0.3826834323650898,
+                            0.2902846772544624, 0.19509032201612828, 0.0980171403295606, 0.0};
+  return make_double2(c[i], -c[16 - i]);
+}
+
+// CTAs per SM for 128 registers a thread.
+template <int LOG>
+constexpr int kP2Ctas = P2<LOG>::TP >= 512 ? 1 : 512 / P2<LOG>::TP;
+
+template <int LOG>
+__global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
+    k_rows_p2(double2 *__restrict__ T, int hp, const double *__restrict__ bsrc, long long bpitch,
+              int h, const double2 *__restrict__ twt, const double2 *__restrict__ post) {
+  using F = P2<LOG>;
+  constexpr int N = F::N, TP = F::TP;
+  extern __shared__ double2 z[];
+  const int t = threadIdx.x;
+  const RowPair rp(h);
+  const double *ra = bsrc + rp.ra * bpitch, *rb = bsrc + rp.rb * bpitch;
+  double2 x[16];
+  double2 va[8], vb[8];
+  if (((reinterpret_cast<uintptr_t>(ra) | reinterpret_cast<uintptr_t>(rb)) & 15) == 0) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      va[j] = reinterpret_cast<const double2 *>(ra)[t + TP * j];
+      vb[j] = reinterpret_cast<const double2 *>(rb)[t + TP * j];
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int m = 2 * (t + TP * j);
+      va[j] = make_double2(ra[m], ra[m + 1]);
+      vb[j] = make_double2(rb[m], rb[m + 1]);
+    }
+  }
+  const typename F::Twiddles tw(twt);
+  double2 pt = post[t];
+  pt = make_double2(0.5 * pt.x, 0.5 * pt.y);
+  // the even samples are this thread's, the odd ones belong to place N - 1 - m
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    x[j] = make_double2(va[j].x, rp.two ? vb[j].x : 0.0);
+    z[at(N - 1 - (t + TP * j))] = make_double2(va[j].y, rp.two ? vb[j].y : 0.0);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 8; j < 16; ++j) x[j] = z[at(t + TP * j)];
+  F::forward(x, z, tw);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) z[at(t + TP * i)] = x[i];
+  __syncthreads();
+  // lanes 2l and 2l + 1 hold one column pair: the even one takes row a, the odd one row b
+  const int odd = t & 1;
+  double2 *dst = T + (long long)(t >> 1) * hp + rp.p0 + odd;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const double2 zk = x[i], zn = z[at((N - (t + TP * i)) & (N - 1))];
+    const double2 tk = cmul(pt, c32(i));  // half the DCT twiddle
+    const double2 A = make_double2(zk.x + zn.x, zk.y - zn.y);
+    const double2 B = make_double2(zk.y + zn.y, zn.x - zk.x);
+    const double xa = tk.x * A.x - tk.y * A.y, xb = tk.x * B.x - tk.y * B.y;
+    const double got = __shfl_xor_sync(0xffffffffu, odd ? xa : xb, 1);
+    const double2 v = odd ? make_double2(got, xb) : make_double2(xa, got);
+    if (!odd || rp.two) dst[(long long)(TP / 2 * i) * hp] = v;
+  }
+}
+
+template <int LOG>
+__global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
+    k_cols_p2(double2 *__restrict__ T, int hp, int w, const double2 *__restrict__ twt,
+              const double2 *__restrict__ post, const double *__restrict__ eig,
+              const double *__restrict__ eig_w) {
+  using F = P2<LOG>;
+  constexpr int N = F::N, TP = F::TP;
+  extern __shared__ double2 z[];
+  const int t = threadIdx.x, c0 = 2 * blockIdx.x;
+  double2 *col = T + (long long)blockIdx.x * hp;
+  double2 x[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) x[j] = col[t + TP * j];
+  const typename F::Twiddles tw(twt);
+  const double2 pt = post[t];
+  const double ew_a = eig_w[c0], ew_b = c0 + 1 < w ? eig_w[c0 + 1] : 0.0;
+  F::forward(x, z, tw);
+  // pairs (k, N - k) with k = t + TP i, i < 8: the upper halves change hands
+#pragma unroll
+  for (int i = 8; i < 16; ++i) z[at(t + TP * i)] = x[i];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int k = t + TP * i;
+    const double ek = eig[k];
+    if (k == 0) {
+      // X_a[0] = Re Z_0, X_b[0] = Im Z_0, W_0 = X_0; mode (0, 0) is the constant: zero
+      const double la = (ek + ew_a) - 4.0, lb = (ek + ew_b) - 4.0;
+      x[0] = make_double2(c0 == 0 ? 0.0 : x[0].x / la, x[0].y / lb);
+    } else {
+      const int pn = at(N - k);
+      const double en = eig[N - k];
+      const double2 tk = cmul(pt, c32(i));
+      Coef4 c = split(x[i], z[pn], tk);
+      c.ak /= (ek + ew_a) - 4.0;
+      c.bk /= (ek + ew_b) - 4.0;
+      c.an /= (en + ew_a) - 4.0;
+      c.bn /= (en + ew_b) - 4.0;
+      x[i] = pack_inverse(c.ak, c.an, c.bk, c.bn, tk);
+      z[pn] = pack_inverse(c.an, c.ak, c.bn, c.bk, make_double2(-tk.y, -tk.x));
+    }
+  }
+  if (t == 0) {  // k = N / 2 is its own partner
+    const double ek = eig[N / 2];
+    const double2 tk = c32(8);
+    Coef4 c = split(x[8], x[8], tk);
+    c.ak /= (ek + ew_a) - 4.0;
+    c.bk /= (ek + ew_b) - 4.0;
+    z[at(N / 2)] = pack_inverse(c.ak, c.ak, c.bk, c.bk, tk);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 8; i < 16; ++i) x[i] = z[at(t + TP * i)];
+  __syncthreads();
+  F::inverse(x, z, tw);
+  constexpr double inv_n = 1.0 / (double)N;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) col[t + TP * j] = make_double2(x[j].x * inv_n, x[j].y * inv_n);
+}
+
+template <int LOG>
+__global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
+    k_irows_p2(double *__restrict__ u, long long upitch, const double2 *__restrict__ T, int hp,
+               int h, const double2 *__restrict__ twt, const double2 *__restrict__ post) {
+  using F = P2<LOG>;
+  constexpr int N = F::N, TP = F::TP;
+  extern __shared__ double2 z[];
+  const int t = threadIdx.x, odd = t & 1;
+  const RowPair rp(h);
+  // the even lane of a column pair loads row a, the odd one row b
+  const double2 *src = T + (long long)(t >> 1) * hp + rp.p0 + (rp.two ? odd : 0);
+  double2 x[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) x[i] = src[(long long)(TP / 2 * i) * hp];
+  const typename F::Twiddles tw(twt);
+  const double2 pt = post[t];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const double got = __shfl_xor_sync(0xffffffffu, odd ? x[i].x : x[i].y, 1);
+    x[i] = odd ? make_double2(got, x[i].y) : make_double2(x[i].x, got);  // (X_a[k], X_b[k])
+    if (!rp.two) x[i].y = 0.0;
+    z[at(t + TP * i)] = x[i];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int k = t + TP * i;
+    double2 xn = z[at((N - k) & (N - 1))];
+    if (k == 0) xn = make_double2(0.0, 0.0);  // X_N = 0
+    x[i] = pack_inverse(x[i].x, xn.x, x[i].y, xn.y, cmul(pt, c32(i)));
+  }
+  __syncthreads();
+  F::inverse(x, z, tw);
+  constexpr double inv_n = 1.0 / (double)N;
+  // place N - 1 - m holds the odd sample of pair m
+#pragma unroll
+  for (int j = 8; j < 16; ++j) z[at(t + TP * j)] = x[j];
+  __syncthreads();
+  double *ua = u + rp.ra * upitch, *ub = u + rp.rb * upitch;
+  const bool vec = ((reinterpret_cast<uintptr_t>(ua) | reinterpret_cast<uintptr_t>(ub)) & 15) == 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int m = t + TP * j;
+    const double2 o = z[at(N - 1 - m)];
+    const double2 a = make_double2(x[j].x * inv_n, o.x * inv_n);
+    const double2 b = make_double2(x[j].y * inv_n, o.y * inv_n);
+    if (vec) {
+      reinterpret_cast<double2 *>(ua)[m] = a;
+      if (rp.two) reinterpret_cast<double2 *>(ub)[m] = b;
+    } else {
+      ua[2 * m] = a.x;
+      ua[2 * m + 1] = a.y;
+      if (rp.two) {
+        ub[2 * m] = b.x;
+        ub[2 * m + 1] = b.y;
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Any other length: the passes of choose_passes at run time, in place in shared
+// memory.  PRIME: the length has a prime factor above 13 (a separate
+// instantiation, so that the register buffer of prime_pass does not weigh on the
+// common lengths).
+
+// Butterfly t of a pass: its first element and its twiddle index within the sub-transform.
+__device__ __forceinline__ int butterfly(const Pass &p, int t, int *k) {
+  const int blk = p.div ? (int)__umulhi((unsigned)t, p.div) : t;
+  *k = t - blk * p.m;
+  return blk * p.r * p.m + *k;
+}
+
+// Decimation in frequency; src(i) gives element i (shared memory, or the line itself
+// in the first pass).
+template <int R, class Src>
+__device__ __forceinline__ void dif_pass(double2 *z, int n, const Pass &p, const double2 *tw,
+                                         Src src) {
+  for (int t = threadIdx.x; t < n / R; t += blockDim.x) {
+    int k;
+    const int base = butterfly(p, t, &k);
+    double2 x[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) x[j] = src(base + j * p.m);
+    dft<R, -1>(x);
+    if (p.m > 1) twiddle<R, -1>(x, tw[k * p.step]);
+#pragma unroll
+    for (int j = 0; j < R; ++j) z[at(base + j * p.m)] = x[j];
+  }
+}
+
+// Decimation in time; dst(i, v) takes element i.
+template <int R, class Dst>
+__device__ __forceinline__ void dit_pass(double2 *z, int n, const Pass &p, const double2 *tw,
+                                         Dst dst) {
+  for (int t = threadIdx.x; t < n / R; t += blockDim.x) {
+    int k;
+    const int base = butterfly(p, t, &k);
+    double2 x[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) x[j] = z[at(base + j * p.m)];
+    if (p.m > 1) twiddle<R, 1>(x, tw[k * p.step]);
+    dft<R, 1>(x);
+#pragma unroll
+    for (int j = 0; j < R; ++j) dst(base + j * p.m, x[j]);
+  }
+}
+
+// A pass of a prime radix above 13, in shared memory: one output per thread and step,
+// computed into registers from the whole butterfly, then written back after a barrier.
+template <int SIGN>
+__device__ void prime_pass(double2 *z, int n, const Pass &p, const double2 *tw) {
+  const int r = p.r, m = p.m, L = r * m, step = p.step, s = n / r;
   double2 res[kMaxPerThread];
 #pragma unroll
   for (int c = 0; c < kMaxPerThread; ++c) {
@@ -210,11 +853,11 @@ __device__ void prime_pass(double2 *z, int n, int L, int r, const double2 *tw) {
     if (o < n) {
       const int blk = o / L, rem = o - blk * L;
       const int q = rem / m, k = rem - q * m;
-      const double2 *p = z + blk * L + k;
+      const int first = blk * L + k;
       double2 acc = make_double2(0.0, 0.0);
       int e = 0;  // (j q) mod r
       for (int j = 0; j < r; ++j) {
-        double2 v = p[j * m];
+        double2 v = z[at(first + j * m)];
         if (SIGN > 0 && j) v = cmulc(v, tw[j * k * step]);  // DIT: input twiddle
         const double2 w = tw[e * s];
         acc = cadd(acc, SIGN < 0 ? cmul(v, w) : cmulc(v, w));
@@ -229,408 +872,183 @@ __device__ void prime_pass(double2 *z, int n, int L, int r, const double2 *tw) {
 #pragma unroll
   for (int c = 0; c < kMaxPerThread; ++c) {
     const int o = threadIdx.x + c * kThreads;
-    if (o < n) z[o] = res[c];
+    if (o < n) z[at(o)] = res[c];
   }
 }
 
-template <int SIGN, bool PRIME>
-__device__ void run_pass(double2 *z, int n, int L, int r, const double2 *tw) {
-  switch (r) {
-    case 8: SIGN < 0 ? dif_pass<8>(z, n, L, tw) : dit_pass<8>(z, n, L, tw); break;
-    case 4: SIGN < 0 ? dif_pass<4>(z, n, L, tw) : dit_pass<4>(z, n, L, tw); break;
-    case 2: SIGN < 0 ? dif_pass<2>(z, n, L, tw) : dit_pass<2>(z, n, L, tw); break;
-    case 3: SIGN < 0 ? dif_pass<3>(z, n, L, tw) : dit_pass<3>(z, n, L, tw); break;
-    case 5: SIGN < 0 ? dif_pass<5>(z, n, L, tw) : dit_pass<5>(z, n, L, tw); break;
-    case 7: SIGN < 0 ? dif_pass<7>(z, n, L, tw) : dit_pass<7>(z, n, L, tw); break;
+#define GD_DCT_RADICES(X) \
+  X(16) X(15) X(14) X(13) X(12) X(11) X(10) X(9) X(8) X(7) X(6) X(5) X(4) X(3) X(2)
+
+template <bool PRIME, class Src>
+__device__ __forceinline__ void forward_pass(double2 *z, const Axis &a, int s, Src src) {
+  const Pass &p = a.rad.p[s];
+  switch (p.r) {
+#define X(R) case R: dif_pass<R>(z, a.rad.n, p, a.tw, src); break;
+    GD_DCT_RADICES(X)
+#undef X
     default:
-      if constexpr (PRIME) prime_pass<SIGN>(z, n, L, r, tw);
+      if constexpr (PRIME) prime_pass<-1>(z, a.rad.n, p, a.tw);
       break;
   }
 }
 
-// Any length: the radices of the plan, passes dispatched at run time.  PRIME:
-// the length has a prime factor above 7 (a separate instantiation, so that the
-// register buffer of prime_pass does not weigh on the common lengths).
+template <bool PRIME, class Dst>
+__device__ __forceinline__ void inverse_pass(double2 *z, const Axis &a, int s, Dst dst) {
+  const Pass &p = a.rad.p[s];
+  switch (p.r) {
+#define X(R) case R: dit_pass<R>(z, a.rad.n, p, a.tw, dst); break;
+    GD_DCT_RADICES(X)
+#undef X
+    default:
+      if constexpr (PRIME) prime_pass<1>(z, a.rad.n, p, a.tw);
+      break;
+  }
+}
+
+// load(i): sample at place i of the reordered line; natural order in, digit-reversed
+// out in z.  A large prime comes first and then works on staged values.
+template <bool PRIME, class Load>
+__device__ __forceinline__ void forward_fft(double2 *z, const Axis &a, Load load) {
+  int s = 0;
+  bool staged = false;
+  if constexpr (PRIME) staged = a.rad.p[0].r > 16;
+  if (staged) {
+    for (int i = threadIdx.x; i < a.rad.n; i += blockDim.x) z[at(i)] = load(i);
+  } else {
+    forward_pass<false>(z, a, 0, load);
+    s = 1;
+  }
+  __syncthreads();
+  for (; s < a.rad.count; ++s) {
+    forward_pass<PRIME>(z, a, s, [&](int i) { return z[at(i)]; });
+    __syncthreads();
+  }
+}
+
+// digit-reversed in z; store(i, v) takes the (unscaled) value at place i.
+template <bool PRIME, class Store>
+__device__ __forceinline__ void inverse_fft(double2 *z, const Axis &a, Store store) {
+  for (int s = a.rad.count - 1; s >= 1; --s) {
+    inverse_pass<PRIME>(z, a, s, [&](int i, double2 v) { z[at(i)] = v; });
+    __syncthreads();
+  }
+  bool staged = false;
+  if constexpr (PRIME) staged = a.rad.p[0].r > 16;
+  if (staged) {
+    inverse_pass<PRIME>(z, a, 0, [&](int i, double2 v) { z[at(i)] = v; });
+    __syncthreads();
+    for (int i = threadIdx.x; i < a.rad.n; i += blockDim.x) store(i, z[at(i)]);
+  } else {
+    inverse_pass<false>(z, a, 0, store);
+  }
+}
+
+// Pass 1: two rows of b -> their DCT-II coefficients along x in T.
 template <bool PRIME>
-struct GeneralFft {
-  static constexpr int kMinBlocks = PRIME ? 1 : 3;
-  const Axis &a;
-  static constexpr size_t extra_smem(int) { return 0; }
-  __device__ __forceinline__ GeneralFft(const Axis &ax, double2 *) : a(ax) {}
-  __device__ __forceinline__ int n() const { return a.rad.n; }
-  // shared-memory slot of element idx
-  __device__ __forceinline__ int at(int idx) const { return idx; }
-
-  // natural order in, digit-reversed order out
-  __device__ void forward(double2 *z) const {
-    int L = a.rad.n;
-    for (int s = 0; s < a.rad.count; ++s) {
-      __syncthreads();
-      run_pass<-1, PRIME>(z, a.rad.n, L, a.rad.r[s], a.tw);
-      L /= a.rad.r[s];
-    }
-    __syncthreads();
-  }
-  // unscaled inverse: digit-reversed order in, natural order out
-  __device__ void inverse(double2 *z) const {
-    int L = 1;
-    for (int s = a.rad.count - 1; s >= 0; --s) {
-      L *= a.rad.r[s];
-      __syncthreads();
-      run_pass<1, PRIME>(z, a.rad.n, L, a.rad.r[s], a.tw);
-    }
-    __syncthreads();
-  }
-  // position of frequency k in the forward output
-  __device__ __forceinline__ int rev(int k) const {
-    int pos = 0, L = a.rad.n;
-    for (int s = 0; s < a.rad.count; ++s) {
-      const int r = a.rad.r[s];
-      const int q = k % r;
-      k /= r;
-      L /= r;
-      pos += q * L;
-    }
-    return pos;
-  }
-};
-
-// Lengths 2^LOG2N (64 .. 8192): radix-8 passes and one radix-2 or -4 pass,
-// every index a shift or a mask known at compile time.
-//
-// Shared memory: a warp's 16-byte accesses are served eight lanes at a time,
-// without conflict when those eight lanes hit eight different 128-byte bank
-// rows' slots (idx & 7).  Butterflies of stride 4, 2 or 1 and the
-// digit-reversed reads (strides N/8, N/64, ...) would all land on one slot, so
-// element idx is stored at idx ^ fold(idx >> 3), fold = XOR of the octal
-// digits: a permutation inside every aligned group of eight that gives
-// distinct slots to any eight elements spaced by a power of eight, by four
-// (with the pair offset of the radix-8 passes) or by one.
-//
-// Twiddles: one e^{-2 pi i m / N} per butterfly from two small shared tables,
-// hi[m >> 6] * lo[m & 63], and its powers by multiplication (the butterfly of
-// radix R needs w^q, q < R).
-template <int LOG2N>
-struct Pow2Fft {
-  static constexpr int N = 1 << LOG2N;
-  static constexpr int S8 = LOG2N / 3;            // radix-8 passes
-  static constexpr int REM = LOG2N % 3;           // last pass radix 2^REM (none if 0)
-  static constexpr int NST = S8 + (REM ? 1 : 0);
-  static constexpr int HI = N >> 6;
-  static constexpr int kMinBlocks = 3;
-  static constexpr size_t extra_smem(int) { return (size_t)(HI + 64) * sizeof(double2); }
-  const double2 *hi, *lo;
-
-  // fill the tables from the plan's length-N table (every thread calls this)
-  __device__ __forceinline__ Pow2Fft(const Axis &a, double2 *tables) {
-    double2 *h = tables, *l = tables + HI;
-    for (int j = threadIdx.x; j < HI + 64; j += blockDim.x)
-      if (j < HI) h[j] = a.tw[j << 6];
-      else l[j - HI] = a.tw[j - HI];
-    hi = h;
-    lo = l;
-  }
-  __device__ __forceinline__ int n() const { return N; }
-  __device__ __forceinline__ double2 w(int m) const { return cmul(hi[m >> 6], lo[m & 63]); }
-  __device__ __forceinline__ static int at(int idx) {
-    int x = idx >> 3, f = x;
-#pragma unroll
-    for (int d = 3; d < LOG2N - 3; d += 3) f ^= x >> d;
-    return idx ^ (f & 7);
-  }
-
-  __host__ __device__ static constexpr int lr(int s) { return s < S8 ? 3 : REM; }
-
-  // w^q for q < R from w = e^{SIGN 2 pi i m / N}
-  template <int R>
-  __device__ __forceinline__ static void powers(double2 (&t)[R], double2 w1) {
-    t[0] = make_double2(1.0, 0.0);
-    if constexpr (R > 1) t[1] = w1;
-    if constexpr (R > 2) t[2] = cmul(w1, w1);
-    if constexpr (R > 3) t[3] = cmul(t[2], w1);
-    if constexpr (R > 4) {
-      t[4] = cmul(t[2], t[2]);
-      t[5] = cmul(t[4], w1);
-      t[6] = cmul(t[3], t[3]);
-      t[7] = cmul(t[6], w1);
-    }
-  }
-
-  template <int S, int SIGN>
-  __device__ __forceinline__ void pass(double2 *z) const {
-    constexpr int LR = lr(S), R = 1 << LR;
-    constexpr int LL = LOG2N - 3 * S;  // log2 of the sub-transform length
-    constexpr int LM = LL - LR;        // log2 of the butterfly stride
-    for (int t = threadIdx.x; t < (N >> LR); t += blockDim.x) {
-      const int k = t & ((1 << LM) - 1);
-      const int base = ((t >> LM) << LL) + k;
-      double2 x[R], tw[R];
-      powers<R>(tw, w(k << (3 * S)));
-      if constexpr (SIGN < 0) {
-#pragma unroll
-        for (int j = 0; j < R; ++j) x[j] = z[at(base + (j << LM))];
-        dft_small<R, -1>(x, nullptr, N);
-#pragma unroll
-        for (int q = 0; q < R; ++q) z[at(base + (q << LM))] = q ? cmul(x[q], tw[q]) : x[q];
-      } else {
-#pragma unroll
-        for (int q = 0; q < R; ++q) {
-          const double2 v = z[at(base + (q << LM))];
-          x[q] = q ? cmulc(v, tw[q]) : v;
-        }
-        dft_small<R, 1>(x, nullptr, N);
-#pragma unroll
-        for (int j = 0; j < R; ++j) z[at(base + (j << LM))] = x[j];
-      }
-    }
-  }
-
-  template <int S>
-  __device__ __forceinline__ void fwd_from(double2 *z) const {
-    if constexpr (S < NST) {
-      __syncthreads();
-      pass<S, -1>(z);
-      fwd_from<S + 1>(z);
-    }
-  }
-  template <int S>
-  __device__ __forceinline__ void inv_from(double2 *z) const {
-    if constexpr (S >= 0) {
-      __syncthreads();
-      pass<S, 1>(z);
-      inv_from<S - 1>(z);
-    }
-  }
-  __device__ void forward(double2 *z) const {
-    fwd_from<0>(z);
-    __syncthreads();
-  }
-  __device__ void inverse(double2 *z) const {
-    inv_from<NST - 1>(z);
-    __syncthreads();
-  }
-  // digit q_S of k (radix of pass S) lands at stride N / (r_0 ... r_S)
-  __device__ __forceinline__ int rev(int k) const {
-    int pos = 0;
-#pragma unroll
-    for (int S = 0; S < S8; ++S) pos |= ((k >> (3 * S)) & 7) << (LOG2N - 3 * S - 3);
-    if constexpr (REM) pos |= (k >> (3 * S8)) & ((1 << REM) - 1);
-    return pos;
-  }
-};
-
-// Where sample j of a line sits in Makhoul's even/odd reordering.
-__device__ __forceinline__ int mak(int j, int n) { return (j & 1) ? n - 1 - (j >> 1) : (j >> 1); }
-
-// Forward DCT coefficients of the two lines packed in Z, at frequency k and
-// its partner n - k (k in 1 .. n-1): X_a[k], X_b[k], X_a[n-k], X_b[n-k].
-struct Coef4 {
-  double ak, bk, an, bn;
-};
-
-__device__ __forceinline__ Coef4 split(double2 zk, double2 zn, double2 tk, double2 tn) {
-  // A_k = (Z_k + conj Z_{n-k}) / 2, B_k = (Z_k - conj Z_{n-k}) / 2i; A_{n-k} = conj A_k
-  const double2 A = make_double2(0.5 * (zk.x + zn.x), 0.5 * (zk.y - zn.y));
-  const double2 B = make_double2(0.5 * (zk.y + zn.y), 0.5 * (zn.x - zk.x));
-  Coef4 c;
-  c.ak = tk.x * A.x - tk.y * A.y;  // Re(t_k A_k)
-  c.bk = tk.x * B.x - tk.y * B.y;
-  c.an = tn.x * A.x + tn.y * A.y;  // Re(t_{n-k} conj A_k)
-  c.bn = tn.x * B.x + tn.y * B.y;
-  return c;
-}
-
-// W_k = conj(t_k) (X_k - i X_{n-k}) for both lines, packed as W_a + i W_b.
-__device__ __forceinline__ double2 pack_inverse(double xa, double xan, double xb, double xbn,
-                                                double2 tk) {
-  // conj(t) (x - i y) = (c + i s)(x - i y) with t = c - i s
-  const double c = tk.x, s = -tk.y;
-  const double2 wa = make_double2(c * xa + s * xan, s * xa - c * xan);
-  const double2 wb = make_double2(c * xb + s * xbn, s * xb - c * xbn);
-  return make_double2(wa.x - wb.y, wa.y + wb.x);
-}
-
-// The kernels below are bound by memory latency (two lines per CTA, a few
-// CTAs per SM), so every loop that reads global memory first issues the loads
-// of kLoads (kTables for table reads) iterations, then uses them.
-constexpr int kLoads = 8;
-constexpr int kTables = 4;
-
-// Pass 1: rows r0, r0 + 1 of b -> their DCT-II coefficients along x in T.
-template <class F>
-__global__ void __launch_bounds__(kThreads, F::kMinBlocks) k_dct_rows(double *__restrict__ T,
-                                                          long long tpitch,
-                                                          const double *__restrict__ b,
-                                                          long long bpitch, int h, Axis ax) {
+__global__ void __launch_bounds__(kThreads, PRIME ? 1 : 2)
+    k_rows_gen(double2 *__restrict__ T, int hp, const double *__restrict__ b, long long bpitch,
+               int h, Axis ax) {
   extern __shared__ double2 z[];
   const int n = ax.rad.n;
-  const F fft(ax, z + n);
-  const int r0 = 2 * blockIdx.x;
-  const bool two = r0 + 1 < h;
-  const double *ra = b + (long long)r0 * bpitch;
-  const double *rb = ra + bpitch;
-  for (int j0 = threadIdx.x; j0 < n; j0 += kLoads * kThreads) {
-    double va[kLoads], vb[kLoads];
+  const RowPair rp(h);
+  const double *ra = b + rp.ra * bpitch, *rb = b + rp.rb * bpitch;
+  forward_fft<PRIME>(z, ax, [&](int i) {
+    const int j = mak_sample(i, n);
+    return make_double2(ra[j], rp.two ? rb[j] : 0.0);
+  });
+  for (int c = threadIdx.x; 2 * c < n; c += blockDim.x) {
+    double va[2] = {0.0, 0.0}, vb[2] = {0.0, 0.0};
 #pragma unroll
-    for (int u = 0; u < kLoads; ++u) {
-      const int j = j0 + u * kThreads;
-      va[u] = j < n ? ra[j] : 0.0;
-      vb[u] = (two && j < n) ? rb[j] : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < kLoads; ++u) {
-      const int j = j0 + u * kThreads;
-      if (j < n) z[fft.at(mak(j, n))] = make_double2(va[u], vb[u]);
-    }
-  }
-  fft.forward(z);
-  double *ta = T + (long long)r0 * tpitch;
-  double *tb = ta + tpitch;
-  for (int k0 = threadIdx.x; k0 < n; k0 += kTables * kThreads) {
-    double2 tk[kTables], tn[kTables];
-#pragma unroll
-    for (int u = 0; u < kTables; ++u) {
-      const int k = min(k0 + u * kThreads, n - 1);
-      tk[u] = ax.post[k];
-      tn[u] = ax.post[k ? n - k : 0];
-    }
-#pragma unroll
-    for (int u = 0; u < kTables; ++u) {
-      const int k = k0 + u * kThreads;
+    for (int q = 0; q < 2; ++q) {
+      const int k = 2 * c + q;
       if (k >= n) break;
-      const Coef4 c = split(z[fft.at(fft.rev(k))], z[fft.at(fft.rev(k ? n - k : 0))], tk[u],
-                            tn[u]);
-      ta[k] = c.ak;
-      if (two) tb[k] = c.bk;
+      const Coef4 f = split(z[at(ax.rev[k])], z[at(ax.rev[k ? n - k : 0])], ax.post[k]);
+      va[q] = f.ak;
+      vb[q] = f.bk;
     }
+    double2 *dst = T + (long long)c * hp + rp.p0;
+    dst[0] = make_double2(va[0], va[1]);
+    if (rp.two) dst[1] = make_double2(vb[0], vb[1]);
   }
 }
 
 // Pass 2: columns c0, c0 + 1 of T: DCT-II along y, division by the
 // eigenvalues (the constant mode set to zero), DCT-III along y.
-template <class F>
-__global__ void __launch_bounds__(kThreads, F::kMinBlocks) k_dct_cols(double *__restrict__ T,
-                                                          long long tpitch, int w, Axis ay,
-                                                          const double *eig_w) {
+template <bool PRIME>
+__global__ void __launch_bounds__(kThreads, PRIME ? 1 : 2)
+    k_cols_gen(double2 *__restrict__ T, int hp, int w, Axis ay,
+               const double *__restrict__ eig_w) {
   extern __shared__ double2 z[];
-  const int n = ay.rad.n;
-  const F fft(ay, z + n);
-  const int c0 = 2 * blockIdx.x;
-  const bool two = c0 + 1 < w;
-  double *col = T + c0;
-  for (int i0 = threadIdx.x; i0 < n; i0 += kLoads * kThreads) {
-    double2 v[kLoads];
-#pragma unroll
-    for (int u = 0; u < kLoads; ++u) {
-      const int i = i0 + u * kThreads;
-      const double *p = col + (long long)min(i, n - 1) * tpitch;
-      v[u] = two ? *reinterpret_cast<const double2 *>(p) : make_double2(p[0], 0.0);
+  const int n = ay.rad.n, c0 = 2 * blockIdx.x;
+  double2 *col = T + (long long)blockIdx.x * hp;
+  forward_fft<PRIME>(z, ay, [&](int i) { return col[i]; });
+  const double ew_a = eig_w[c0], ew_b = c0 + 1 < w ? eig_w[c0 + 1] : 0.0;
+  for (int k = threadIdx.x; k <= n / 2; k += blockDim.x) {
+    const int pk = at(ay.rev[k]);
+    const double ek = ay.eig[k];
+    if (k == 0) {
+      const double2 z0 = z[pk];  // X_a[0] = Re Z_0, X_b[0] = Im Z_0; W_0 = X_0
+      const double la = (ek + ew_a) - 4.0, lb = (ek + ew_b) - 4.0;
+      // mode (0, 0) is the constant: zero (the zero-mean solution)
+      z[pk] = make_double2(c0 == 0 ? 0.0 : z0.x / la, z0.y / lb);
+      continue;
     }
-#pragma unroll
-    for (int u = 0; u < kLoads; ++u) {
-      const int i = i0 + u * kThreads;
-      if (i < n) z[fft.at(mak(i, n))] = v[u];
-    }
+    const int nk = n - k, pn = at(ay.rev[nk]);
+    const double2 tk = ay.post[k];
+    const double en = ay.eig[nk];
+    Coef4 c = split(z[pk], z[pn], tk);
+    c.ak /= (ek + ew_a) - 4.0;
+    c.bk /= (ek + ew_b) - 4.0;
+    c.an /= (en + ew_a) - 4.0;
+    c.bn /= (en + ew_b) - 4.0;
+    z[pk] = pack_inverse(c.ak, c.an, c.bk, c.bn, tk);
+    if (nk != k) z[pn] = pack_inverse(c.an, c.ak, c.bn, c.bk, make_double2(-tk.y, -tk.x));
   }
-  fft.forward(z);
-  const double ew_a = eig_w[c0], ew_b = two ? eig_w[c0 + 1] : 0.0;
-  for (int k0 = threadIdx.x; k0 <= n / 2; k0 += kTables * kThreads) {
-    double2 tk[kTables], tn[kTables];
-    double ek[kTables], en[kTables];
-#pragma unroll
-    for (int u = 0; u < kTables; ++u) {
-      const int k = min(k0 + u * kThreads, n / 2);
-      tk[u] = ay.post[k];
-      tn[u] = ay.post[(n - k) % n];
-      ek[u] = ay.eig[k];
-      en[u] = ay.eig[(n - k) % n];
-    }
-#pragma unroll
-    for (int u = 0; u < kTables; ++u) {
-      const int k = k0 + u * kThreads;
-      if (k > n / 2) break;
-      const int pk = fft.at(fft.rev(k));
-      if (k == 0) {
-        const double2 z0 = z[pk];  // X_a[0] = Re Z_0, X_b[0] = Im Z_0; W_0 = X_0
-        const double la = (ek[u] + ew_a) - 4.0, lb = (ek[u] + ew_b) - 4.0;
-        // mode (0, 0) is the constant: zero (the zero-mean solution)
-        z[pk] = make_double2(c0 == 0 ? 0.0 : z0.x / la, z0.y / lb);
-        continue;
-      }
-      const int nk = n - k;
-      const int pn = fft.at(fft.rev(nk));
-      Coef4 c = split(z[pk], z[pn], tk[u], tn[u]);
-      c.ak /= (ek[u] + ew_a) - 4.0;
-      c.bk /= (ek[u] + ew_b) - 4.0;
-      c.an /= (en[u] + ew_a) - 4.0;
-      c.bn /= (en[u] + ew_b) - 4.0;
-      z[pk] = pack_inverse(c.ak, c.an, c.bk, c.bn, tk[u]);
-      if (nk != k) z[pn] = pack_inverse(c.an, c.ak, c.bn, c.bk, tn[u]);
-    }
-  }
-  fft.inverse(z);
+  __syncthreads();
   const double inv_n = 1.0 / (double)n;
-  for (int i = threadIdx.x; i < n; i += kThreads) {
-    const double2 v = z[fft.at(mak(i, n))];
-    double *p = col + (long long)i * tpitch;
-    if (two) *reinterpret_cast<double2 *>(p) = make_double2(v.x * inv_n, v.y * inv_n);
-    else p[0] = v.x * inv_n;
-  }
+  inverse_fft<PRIME>(z, ay, [&](int i, double2 v) {
+    col[i] = make_double2(v.x * inv_n, v.y * inv_n);
+  });
 }
 
-// Pass 3: rows r0, r0 + 1 of T (coefficients along x) -> DCT-III -> u.
-template <class F>
-__global__ void __launch_bounds__(kThreads, F::kMinBlocks) k_idct_rows(double *__restrict__ u,
-                                                           long long upitch,
-                                                           const double *__restrict__ T,
-                                                           long long tpitch, int h, Axis ax) {
+// Pass 3: two rows of T (coefficients along x) -> DCT-III -> u.
+template <bool PRIME>
+__global__ void __launch_bounds__(kThreads, PRIME ? 1 : 2)
+    k_irows_gen(double *__restrict__ u, long long upitch, const double2 *__restrict__ T, int hp,
+                int h, Axis ax) {
   extern __shared__ double2 z[];
   const int n = ax.rad.n;
-  const F fft(ax, z + n);
-  const int r0 = 2 * blockIdx.x;
-  const bool two = r0 + 1 < h;
-  const double *ta = T + (long long)r0 * tpitch;
-  const double *tb = two ? ta + tpitch : ta;  // a single row reads its own row twice
-  for (int k0 = threadIdx.x; k0 <= n / 2; k0 += kTables * kThreads) {
-    double xa[kTables], xb[kTables], xan[kTables], xbn[kTables];
-    double2 tk[kTables], tn[kTables];
-#pragma unroll
-    for (int u = 0; u < kTables; ++u) {
-      const int k = min(k0 + u * kThreads, n / 2);
-      const int nk = (n - k) % n;
-      xa[u] = ta[k];
-      xb[u] = tb[k];
-      xan[u] = ta[nk];
-      xbn[u] = tb[nk];
-      tk[u] = ax.post[k];
-      tn[u] = ax.post[nk];
+  const RowPair rp(h);
+  const double *Td = reinterpret_cast<const double *>(T);
+  auto coef = [&](int k) {  // (X_a[k], X_b[k])
+    const double *p = Td + ((long long)(k >> 1) * hp + rp.p0) * 2 + (k & 1);
+    return make_double2(p[0], rp.two ? p[2] : 0.0);
+  };
+  for (int k = threadIdx.x; k <= n / 2; k += blockDim.x) {
+    const double2 xk = coef(k);
+    if (k == 0) {
+      z[at(ax.rev[0])] = xk;  // W_0 = X_0 (X_n = 0)
+      continue;
     }
-#pragma unroll
-    for (int u = 0; u < kTables; ++u) {
-      const int k = k0 + u * kThreads;
-      if (k > n / 2) break;
-      const double b0 = two ? xb[u] : 0.0, bn = two ? xbn[u] : 0.0;
-      if (k == 0) {
-        z[fft.at(fft.rev(0))] = make_double2(xa[u], b0);  // W_0 = X_0 (X_n = 0)
-        continue;
-      }
-      const int nk = n - k;
-      z[fft.at(fft.rev(k))] = pack_inverse(xa[u], xan[u], b0, bn, tk[u]);
-      if (nk != k) z[fft.at(fft.rev(nk))] = pack_inverse(xan[u], xa[u], bn, b0, tn[u]);
-    }
+    const int nk = n - k;
+    const double2 xn = coef(nk), tk = ax.post[k];
+    z[at(ax.rev[k])] = pack_inverse(xk.x, xn.x, xk.y, xn.y, tk);
+    if (nk != k)
+      z[at(ax.rev[nk])] = pack_inverse(xn.x, xk.x, xn.y, xk.y, make_double2(-tk.y, -tk.x));
   }
-  fft.inverse(z);
+  __syncthreads();
   const double inv_n = 1.0 / (double)n;
-  double *ua = u + (long long)r0 * upitch;
-  double *ub = ua + upitch;
-  for (int j = threadIdx.x; j < n; j += kThreads) {
-    const double2 v = z[fft.at(mak(j, n))];
+  double *ua = u + rp.ra * upitch, *ub = u + rp.rb * upitch;
+  inverse_fft<PRIME>(z, ax, [&](int i, double2 v) {
+    const int j = mak_sample(i, n);
     ua[j] = v.x * inv_n;
-    if (two) ub[j] = v.y * inv_n;
-  }
+    if (rp.two) ub[j] = v.y * inv_n;
+  });
 }
 
-__global__ void k_dct_tables(double2 *tw, double2 *post, double *eig, int n) {
+__global__ void k_dct_tables(double2 *tw, double2 *post, double *eig, unsigned short *rev,
+                             Radices rad) {
+  const int n = rad.n;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   double s, c;
@@ -639,45 +1057,35 @@ __global__ void k_dct_tables(double2 *tw, double2 *post, double *eig, int n) {
   sincospi((double)k / (2.0 * (double)n), &s, &c);
   post[k] = make_double2(c, -s);
   eig[k] = 2.0 * cos(M_PI * (double)k / (double)n);
-}
-
-inline bool has_large_prime(const Radices &r) {
-  for (int s = 0; s < r.count; ++s)
-    if (r.r[s] > 8) return true;
-  return false;
+  int pos = 0, f = k;
+  for (int q = 0; q < rad.count; ++q) {
+    pos += (f % rad.p[q].r) * rad.p[q].m;
+    f /= rad.p[q].r;
+  }
+  rev[k] = (unsigned short)pos;
 }
 
 inline size_t a256(size_t v) { return (v + 255) & ~(size_t)255; }
-inline size_t smem_bytes(int n) { return (size_t)n * sizeof(double2); }
-// the most dynamic shared memory any DCT kernel launch asks for (a line of
-// kMaxLen complex values and the power-of-two twiddle tables)
-constexpr size_t kMaxSmemBytes = (size_t)kMaxLen * sizeof(double2) + Pow2Fft<13>::extra_smem(0);
+inline size_t smem_bytes(int n) { return (size_t)((n + 7) & ~7) * sizeof(double2); }
+// the most dynamic shared memory any DCT kernel launch asks for
+constexpr size_t kMaxSmemBytes = (size_t)kMaxLen * sizeof(double2);
 
-template <class T>
-struct Tag {
-  using type = T;
-};
+template <int V>
+using Int = std::integral_constant<int, V>;
 
-// Call fn(Tag<F>{}) with the FFT policy of a length: the power-of-two kernels
-// for 64 .. 8192, the general ones otherwise.
-template <class Fn>
-void with_fft(const Radices &r, Fn &&fn) {
-  const int n = r.n;
-  if (n >= 64 && (n & (n - 1)) == 0) {
-    switch (__builtin_ctz((unsigned)n)) {
-      case 6: fn(Tag<Pow2Fft<6>>{}); return;
-      case 7: fn(Tag<Pow2Fft<7>>{}); return;
-      case 8: fn(Tag<Pow2Fft<8>>{}); return;
-      case 9: fn(Tag<Pow2Fft<9>>{}); return;
-      case 10: fn(Tag<Pow2Fft<10>>{}); return;
-      case 11: fn(Tag<Pow2Fft<11>>{}); return;
-      case 12: fn(Tag<Pow2Fft<12>>{}); return;
-      case 13: fn(Tag<Pow2Fft<13>>{}); return;
-      default: break;
-    }
+// Call p2(Int<log2 n>{}) for the power-of-two kernels' lengths, gen(PRIME) otherwise.
+template <class P2Fn, class GenFn>
+void with_kernels(const Radices &r, P2Fn &&p2, GenFn &&gen) {
+  switch (r.n) {
+    case 512: p2(Int<9>{}); return;
+    case 1024: p2(Int<10>{}); return;
+    case 2048: p2(Int<11>{}); return;
+    case 4096: p2(Int<12>{}); return;
+    case 8192: p2(Int<13>{}); return;
+    default: break;
   }
-  if (has_large_prime(r)) fn(Tag<GeneralFft<true>>{});
-  else fn(Tag<GeneralFft<false>>{});
+  if (has_large_prime(r)) gen(std::true_type{});
+  else gen(std::false_type{});
 }
 
 }  // namespace dct
@@ -687,7 +1095,7 @@ using namespace gd;
 
 struct gd_dct_plan_s {
   int h = 0, w = 0;
-  long long tpitch = 0;  // row pitch of the coefficient buffer T (even: column pairs align)
+  int hp = 0;  // rows of T per column pair (h rounded up to an even number)
   dct::Radices rh, rw;
   size_t o_t = 0, o_tab_w = 0, o_tab_h = 0, total = 0;
   char *ws = nullptr;
@@ -698,7 +1106,10 @@ namespace {
 struct AxisTables {
   double2 *tw, *post;
   double *eig;
+  unsigned short *rev;
 };
+
+constexpr size_t kTableBytes = 2 * sizeof(double2) + sizeof(double) + sizeof(unsigned short);
 
 AxisTables tables(gd_dct_plan p, size_t off, int n) {
   char *b = p->ws + off;
@@ -706,6 +1117,7 @@ AxisTables tables(gd_dct_plan p, size_t off, int n) {
   t.tw = reinterpret_cast<double2 *>(b);
   t.post = t.tw + n;
   t.eig = reinterpret_cast<double *>(t.post + n);
+  t.rev = reinterpret_cast<unsigned short *>(t.eig + n);
   return t;
 }
 
@@ -717,6 +1129,7 @@ dct::Axis axis(gd_dct_plan p, bool rows) {
   a.tw = t.tw;
   a.post = t.post;
   a.eig = t.eig;
+  a.rev = t.rev;
   return a;
 }
 
@@ -734,16 +1147,16 @@ extern "C" int gd_dct_plan_create(int32_t h, int32_t w, gd_dct_plan *out) {
   gd_dct_plan p = new gd_dct_plan_s();
   p->h = h;
   p->w = w;
-  p->tpitch = (w + 1) & ~1;
-  p->rh = dct::factor(h);
-  p->rw = dct::factor(w);
+  p->hp = (h + 1) & ~1;
+  p->rh = dct::choose_passes(h);
+  p->rw = dct::choose_passes(w);
   size_t o = 0;
   p->o_t = o;
-  o = dct::a256(o + (size_t)h * p->tpitch * sizeof(double));
+  o = dct::a256(o + (size_t)((w + 1) / 2) * p->hp * sizeof(double2));
   p->o_tab_w = o;
-  o = dct::a256(o + (size_t)w * (2 * sizeof(double2) + sizeof(double)));
+  o = dct::a256(o + (size_t)w * kTableBytes);
   p->o_tab_h = o;
-  o = dct::a256(o + (size_t)h * (2 * sizeof(double2) + sizeof(double)));
+  o = dct::a256(o + (size_t)h * kTableBytes);
   p->total = o;
   *out = p;
   return GD_OK;
@@ -759,8 +1172,8 @@ extern "C" int gd_dct_plan_bind(gd_dct_plan p, void *ws, size_t bytes, cudaStrea
                                                      "256-byte aligned");
   p->ws = static_cast<char *>(ws);
   const AxisTables tw = tables(p, p->o_tab_w, p->w), th = tables(p, p->o_tab_h, p->h);
-  dct::k_dct_tables<<<(p->w + 255) / 256, 256, 0, st>>>(tw.tw, tw.post, tw.eig, p->w);
-  dct::k_dct_tables<<<(p->h + 255) / 256, 256, 0, st>>>(th.tw, th.post, th.eig, p->h);
+  dct::k_dct_tables<<<(p->w + 255) / 256, 256, 0, st>>>(tw.tw, tw.post, tw.eig, tw.rev, p->rw);
+  dct::k_dct_tables<<<(p->h + 255) / 256, 256, 0, st>>>(th.tw, th.post, th.eig, th.rev, p->rh);
   GD_CHECK_LAUNCH();
   // the tables must be complete before a solve on any stream (set-up, once per plan)
   GD_CHECK_CUDA(cudaStreamSynchronize(st));
@@ -774,15 +1187,19 @@ extern "C" int gd_dct_plan_bind(gd_dct_plan p, void *ws, size_t bytes, cudaStrea
                                                (int)dct::kMaxSmemBytes);
     if (e != cudaSuccess) err = e;
   };
-  dct::with_fft(p->rw, [&](auto tag) {
-    using F = typename decltype(tag)::type;
-    allow((const void *)dct::k_dct_rows<F>);
-    allow((const void *)dct::k_idct_rows<F>);
-  });
-  dct::with_fft(p->rh, [&](auto tag) {
-    using F = typename decltype(tag)::type;
-    allow((const void *)dct::k_dct_cols<F>);
-  });
+  dct::with_kernels(
+      p->rw,
+      [&](auto log) {
+        allow((const void *)dct::k_rows_p2<decltype(log)::value>);
+        allow((const void *)dct::k_irows_p2<decltype(log)::value>);
+      },
+      [&](auto prime) {
+        allow((const void *)dct::k_rows_gen<decltype(prime)::value>);
+        allow((const void *)dct::k_irows_gen<decltype(prime)::value>);
+      });
+  dct::with_kernels(
+      p->rh, [&](auto log) { allow((const void *)dct::k_cols_p2<decltype(log)::value>); },
+      [&](auto prime) { allow((const void *)dct::k_cols_gen<decltype(prime)::value>); });
   GD_CHECK_CUDA(err);
   return GD_OK;
 }
@@ -791,25 +1208,44 @@ extern "C" int gd_dct_solve_neumann(gd_dct_plan p, const double *b_in, double *u
                                     cudaStream_t st) {
   GD_REQUIRE(p && p->ws && b_in && u && pitch >= p->w, GD_ERR_ARG,
              "gd_dct_solve_neumann: bad arguments or unbound plan");
-  const int h = p->h, w = p->w;
-  double *T = reinterpret_cast<double *>(p->ws + p->o_t);
+  const int h = p->h, w = p->w, hp = p->hp;
+  double2 *T = reinterpret_cast<double2 *>(p->ws + p->o_t);
   const dct::Axis ax = axis(p, true), ay = axis(p, false);
   const unsigned rows = (unsigned)(h + 1) / 2, cols = (unsigned)(w + 1) / 2;
-  dct::with_fft(p->rw, [&](auto tag) {
-    using F = typename decltype(tag)::type;
-    const size_t b = dct::smem_bytes(w) + F::extra_smem(w);
-    dct::k_dct_rows<F><<<rows, dct::kThreads, b, st>>>(T, p->tpitch, b_in, pitch, h, ax);
-  });
-  dct::with_fft(p->rh, [&](auto tag) {
-    using F = typename decltype(tag)::type;
-    const size_t b = dct::smem_bytes(h) + F::extra_smem(h);
-    dct::k_dct_cols<F><<<cols, dct::kThreads, b, st>>>(T, p->tpitch, w, ay, ax.eig);
-  });
-  dct::with_fft(p->rw, [&](auto tag) {
-    using F = typename decltype(tag)::type;
-    const size_t b = dct::smem_bytes(w) + F::extra_smem(w);
-    dct::k_idct_rows<F><<<rows, dct::kThreads, b, st>>>(u, pitch, T, p->tpitch, h, ax);
-  });
+  const int tw = dct::gen_threads(p->rw), th = dct::gen_threads(p->rh);
+  dct::with_kernels(
+      p->rw,
+      [&](auto log) {
+        using F = dct::P2<decltype(log)::value>;
+        dct::k_rows_p2<decltype(log)::value><<<rows, F::TP, F::smem, st>>>(T, hp, b_in, pitch, h,
+                                                                           ax.tw, ax.post);
+      },
+      [&](auto prime) {
+        dct::k_rows_gen<decltype(prime)::value><<<rows, tw, dct::smem_bytes(w), st>>>(
+            T, hp, b_in, pitch, h, ax);
+      });
+  dct::with_kernels(
+      p->rh,
+      [&](auto log) {
+        using F = dct::P2<decltype(log)::value>;
+        dct::k_cols_p2<decltype(log)::value><<<cols, F::TP, F::smem, st>>>(
+            T, hp, w, ay.tw, ay.post, ay.eig, ax.eig);
+      },
+      [&](auto prime) {
+        dct::k_cols_gen<decltype(prime)::value><<<cols, th, dct::smem_bytes(h), st>>>(T, hp, w, ay,
+                                                                                     ax.eig);
+      });
+  dct::with_kernels(
+      p->rw,
+      [&](auto log) {
+        using F = dct::P2<decltype(log)::value>;
+        dct::k_irows_p2<decltype(log)::value><<<rows, F::TP, F::smem, st>>>(u, pitch, T, hp, h,
+                                                                            ax.tw, ax.post);
+      },
+      [&](auto prime) {
+        dct::k_irows_gen<decltype(prime)::value><<<rows, tw, dct::smem_bytes(w), st>>>(
+            u, pitch, T, hp, h, ax);
+      });
   GD_CHECK_LAUNCH();
   return GD_OK;
 }
