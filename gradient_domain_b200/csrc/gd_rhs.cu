@@ -8,6 +8,7 @@
 // spacing 1), and gd_masked_rhs follows the masked assembly of
 // poisson.py:216-224.  All three keep the reference's order of additions.
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 
@@ -175,25 +176,44 @@ struct FieldView {
 // image cell (row0, col0).  Interior cells take the backward differences; the
 // window's outer ring is written 0 (no consumer of a window reads it) or, with
 // `edges`, follows operators.py's edge rules for the window as a whole image.
-__global__ void k_guidance_div(double *__restrict__ out, FieldView fv, int row0, int col0, int h,
-                               int w) {
-  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= (long long)h * w) return;
-  const int i = (int)(k / w), j = (int)(k % w);
-  const int y = row0 + i, x = col0 + j;
-  const bool ring = i == 0 || j == 0 || i == h - 1 || j == w - 1;
-  if (ring && !fv.d.edges) {
-    out[k] = 0.0;
-    return;
+//
+// A warp walks kGuideRows rows of 31 columns: the field of a cell is formed once,
+// its left neighbour's comes from the lane beside (lane 0 only serves as the first
+// column's neighbour) and the one above from the row before (1440 x 2160 weighted
+// field: 40 us with three fields a cell and a 64-bit division, 26 us).
+constexpr int kGuideRows = 8, kGuideCols = 31, kGuideWarps = 8;
+__global__ void __launch_bounds__(32 * kGuideWarps)
+    k_guidance_div(double *__restrict__ out, FieldView fv, int row0, int col0, int h, int w) {
+  const int lane = threadIdx.x & 31;
+  const int j = (blockIdx.x * kGuideWarps + (threadIdx.x >> 5)) * kGuideCols + lane - 1;
+  if (j - lane >= w - 1) return;  // whole warp beyond the window
+  const bool inside = j >= 0 && j < w, writes = inside && lane > 0;
+  const int x = col0 + j;
+  for (int i0 = blockIdx.y * kGuideRows; i0 < h; i0 += gridDim.y * kGuideRows) {
+    const int i1 = min(i0 + kGuideRows, h);
+    double gy_up = 0.0;
+    if (i0 > 0 && inside) {
+      double unused;
+      fv.field(row0 + i0 - 1, x, unused, gy_up);
+    }
+    for (int i = i0; i < i1; ++i) {
+      double gx = 0.0, gy = 0.0;
+      if (inside) fv.field(row0 + i, x, gx, gy);
+      const double gxl = __shfl_up_sync(0xffffffffu, gx, 1);
+      if (writes) {
+        double v = 0.0;
+        const bool ring = i == 0 || j == 0 || i == h - 1 || j == w - 1;
+        if (!ring || fv.d.edges) {
+          double dx = 0.0, dy = 0.0;
+          if (w > 1) dx = j == 0 ? gx : j == w - 1 ? -gxl : __dsub_rn(gx, gxl);
+          if (h > 1) dy = i == 0 ? gy : i == h - 1 ? -gy_up : __dsub_rn(gy, gy_up);
+          v = __dadd_rn(dx, dy);
+        }
+        out[(long long)i * w + j] = v;
+      }
+      gy_up = gy;
+    }
   }
-  double gx, gy, gxl = 0.0, gyl = 0.0, unused;
-  fv.field(y, x, gx, gy);
-  if (j > 0) fv.field(y, x - 1, gxl, unused);
-  if (i > 0) fv.field(y - 1, x, unused, gyl);
-  double dx = 0.0, dy = 0.0;
-  if (w > 1) dx = j == 0 ? gx : j == w - 1 ? -gxl : __dsub_rn(gx, gxl);
-  if (h > 1) dy = i == 0 ? gy : i == h - 1 ? -gyl : __dsub_rn(gy, gyl);
-  out[k] = __dadd_rn(dx, dy);
 }
 
 inline unsigned blocks(long long work) { return (unsigned)((work + 255) / 256); }
@@ -260,7 +280,8 @@ extern "C" int gd_guidance_divergence(double *div, const gd_field_desc *field, i
              "gd_guidance_divergence: cloning fields need a source and a selection");
   GD_REQUIRE(d.kind != GD_FIELD_WEIGHTED || d.weights, GD_ERR_ARG,
              "gd_guidance_divergence: weighted fields need weights");
-  k_guidance_div<<<blocks((long long)h * w), 256, 0, st>>>(div, FieldView{d}, row0, col0, h, w);
+  const dim3 grid(ceil_div(w, kGuideCols * kGuideWarps), std::min(ceil_div(h, kGuideRows), 65535));
+  k_guidance_div<<<grid, 32 * kGuideWarps, 0, st>>>(div, FieldView{d}, row0, col0, h, w);
   GD_CHECK_LAUNCH();
   return GD_OK;
 }

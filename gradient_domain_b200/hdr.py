@@ -97,7 +97,7 @@ def tone_map_device(rad: torch.Tensor, config: ToneMapConfig, dct=None):
                           _lib.ptr(factor), 0.0, 0.0, 0.0)
     _lib.check(lib.gd_guidance_divergence(_lib.ptr(div), C.byref(desc), 0, 0, h, w, st),
                "gd_guidance_divergence")
-    compressed = torch.zeros_like(div)
+    compressed = torch.empty_like(div)
     from .solvers import DCT_MAX_SIDE, _dct_plan
     if 2 <= min(h, w) and max(h, w) <= DCT_MAX_SIDE:
         # the reference's exact transform solve (solvers.py:224-262)
