@@ -26,7 +26,8 @@ EXPORTS = (
     "gd_last_error", "gd_version", "gd_plan_create", "gd_plan_destroy",
     "gd_plan_workspace_bytes", "gd_plan_bind", "gd_plan_set_mask", "gd_plan_prepare",
     "gd_solve", "gd_solve_async", "gd_solve_finish", "gd_plan_apply_vcycle", "gd_plan_set_profiling", "gd_plan_kernel_times", "gd_plan_level_times",
-    "gd_ref_workspace_bytes", "gd_ref_vcycle", "gd_ref_vcycle_static", "gd_rbgs_smooth",
+    "gd_ref_workspace_bytes", "gd_ref_vcycle", "gd_ref_vcycle_fused", "gd_ref_vcycle_static",
+    "gd_rbgs_smooth", "gd_ref_residual_norm2",
     "gd_ref_residual", "gd_ref_dot", "gd_ref_axpby", "gd_ref_restrict", "gd_ref_prolong_add", "gd_gradient", "gd_divergence", "gd_fold_dirichlet",
     "gd_fold_boundary",
     "gd_masked_rhs", "gd_guidance_divergence", "gd_tm_scratch_bytes", "gd_tm_log_luminance",
@@ -113,6 +114,9 @@ def _declare(lib: C.CDLL) -> None:
         "gd_ref_workspace_bytes": (_sz, [_i32, _i32, _i32]),
         "gd_ref_vcycle": (C.c_int, [_vp, _vp, _i32, _i32, _f64, _i32, _i32, _i32, _i32, _vp,
                                     _sz, _vp]),
+        "gd_ref_vcycle_fused": (C.c_int, [_vp, _vp, _i32, _i32, _f64, _i32, _i32, _i32, _i32,
+                                          _vp, _sz, _vp]),
+        "gd_ref_residual_norm2": (C.c_int, [_vp, _vp, _vp, _i32, _i32, _f64, _vp, _sz, _vp]),
         "gd_ref_vcycle_static": (C.c_int, [_vp, _vp, _i32, _i32, _f64, _i32, _i32, _i32, _i32,
                                            _vp]),
         "gd_rbgs_smooth": (C.c_int, [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _f64, _i32, _vp]),

@@ -3,7 +3,7 @@
 Same interface and semantics as gradient-domain/src/gradient_domain/multigrid.py:
 ``MultigridOptions`` (:47-71), ``MultigridReport`` (:75-108), ``v_cycle``
 (:184-215) and ``solve`` (:218-255).  The V-cycle runs in the library's
-vertex-centred FP64 kernels (``gd_ref_vcycle``), which evaluate every
+vertex-centred FP64 kernels (``gd_ref_vcycle_fused``), which evaluate every
 smoothing, residual and transfer expression in the reference's order, so one
 cycle matches the NumPy one to rounding and ``solve`` takes the same number of
 cycles.  The B200 solver proper (cell-centred, mixed precision, batched) is
@@ -66,19 +66,33 @@ class RefWorkspace:
         self.scalar = torch.empty(1, dtype=torch.float64, device=dev)
         self.shape, self.coarsest_size = shape, coarsest_size
 
-    def vcycle(self, u: torch.Tensor, b: torch.Tensor, spacing: float, o: MultigridOptions):
+    def vcycle(self, u: torch.Tensor, b: torch.Tensor, spacing: float, o: MultigridOptions,
+               by_operation: bool = False):
+        """One V-cycle in place on ``u``; ``by_operation`` launches one kernel per operation
+        of the reference instead of the fused passes (the same bits)."""
         m, n = self.shape
-        _lib.check(_lib.lib().gd_ref_vcycle(_lib.ptr(u), _lib.ptr(b), m, n, float(spacing),
-                                            o.pre_smoothing, o.post_smoothing, o.coarsest_size,
-                                            o.coarsest_sweeps, _lib.ptr(self.buf),
-                                            self.buf.numel(), _lib.stream_handle()),
-                   "gd_ref_vcycle")
+        name = "gd_ref_vcycle" if by_operation else "gd_ref_vcycle_fused"
+        _lib.check(getattr(_lib.lib(), name)(_lib.ptr(u), _lib.ptr(b), m, n, float(spacing),
+                                             o.pre_smoothing, o.post_smoothing, o.coarsest_size,
+                                             o.coarsest_sweeps, _lib.ptr(self.buf),
+                                             self.buf.numel(), _lib.stream_handle()), name)
 
     def residual(self, r: torch.Tensor, u: torch.Tensor, b: torch.Tensor, spacing: float):
         m, n = self.shape
         _lib.check(_lib.lib().gd_ref_residual(_lib.ptr(r), _lib.ptr(u), _lib.ptr(b), m, n,
                                               float(spacing), _lib.stream_handle()),
                    "gd_ref_residual")
+
+    def residual_norm(self, u: torch.Tensor, b: torch.Tensor, spacing: float) -> float:
+        """||b - laplacian(u)||"""
+        m, n = self.shape
+        _lib.check(_lib.lib().gd_ref_residual_norm2(_lib.ptr(self.scalar), _lib.ptr(u),
+                                                    _lib.ptr(b), m, n, float(spacing),
+                                                    _lib.ptr(self.dot_buf),
+                                                    self.dot_buf.numel() * 8,
+                                                    _lib.stream_handle()),
+                   "gd_ref_residual_norm2")
+        return float(np.sqrt(self.scalar.item()))
 
     def dot(self, a: torch.Tensor, b: torch.Tensor) -> float:
         _lib.check(_lib.lib().gd_ref_dot(_lib.ptr(self.scalar), _lib.ptr(a), _lib.ptr(b),
@@ -184,11 +198,9 @@ def solve(b, spacing: float = 1.0, options: MultigridOptions | None = None,
     scale = float(np.sqrt(ws.dot(b_d, b_d)))
     if scale == 0.0:
         return download(u_d), MultigridReport([0.0], 0, True)
-    r_d = torch.empty_like(b_d)
 
     def rel_residual() -> float:
-        ws.residual(r_d, u_d, b_d, spacing)
-        return float(np.sqrt(ws.dot(r_d, r_d))) / scale
+        return ws.residual_norm(u_d, b_d, spacing) / scale
 
     history = [rel_residual()]
     for cycle in range(1, options.max_cycles + 1):

@@ -117,7 +117,7 @@ def _ref_pcg_dev(b_d: torch.Tensor, spacing, tolerance, max_iterations, precondi
         z = torch.zeros_like(r)
         neg = torch.zeros_like(r)
         ws.axpby(neg, r, -1.0, 0.0)
-        ws.vcycle(z, neg, spacing, opts)
+        ws.vcycle(z, neg, spacing, opts, by_operation=True)
         return z
 
     rhs = torch.zeros_like(b_d)
@@ -164,12 +164,10 @@ def _solve_multigrid(b, spacing, tolerance, max_iterations):
     b_d = _dev_array(b, dev)
     ws = RefWorkspace(tuple(b_d.shape), opts.coarsest_size, dev)
     u = torch.zeros_like(b_d)
-    r = torch.empty_like(b_d)
     scale = float(np.sqrt(ws.dot(b_d, b_d))) or 1.0
     for cycle in range(1, max_iterations + 1):
         ws.vcycle(u, b_d, spacing, opts)
-        ws.residual(r, u, b_d, spacing)
-        if float(np.sqrt(ws.dot(r, r))) / scale < tolerance:
+        if ws.residual_norm(u, b_d, spacing) / scale < tolerance:
             return download(u), cycle, True
     return download(u), max_iterations, False
 
@@ -192,9 +190,7 @@ def relative_residual(u: np.ndarray, b: np.ndarray, spacing: float) -> float:
     scale = float(np.sqrt(ws.dot(b_d, b_d)))
     if scale == 0.0:
         return 0.0
-    r = torch.empty_like(b_d)
-    ws.residual(r, u_d, b_d, spacing)
-    return float(np.sqrt(ws.dot(r, r))) / scale
+    return ws.residual_norm(u_d, b_d, spacing) / scale
 
 
 def solve_system(b, method: str = "mgcg", spacing: float = 1.0, tolerance: float = 1e-8,

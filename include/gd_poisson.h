@@ -307,6 +307,19 @@ int gd_rbgs_smooth(const void *u_dev, void *out_dev, const void *b_dev, int32_t 
                    int32_t pitch, int32_t fp64, double spacing, int32_t sweeps,
                    cudaStream_t stream);
 
+/* gd_ref_vcycle with its passes fused (two launches a level): the same bits.
+ * The workspace is the same (gd_ref_workspace_bytes). */
+int gd_ref_vcycle_fused(double *u_dev, const double *b_dev, int32_t m, int32_t n, double spacing,
+                        int32_t pre, int32_t post, int32_t coarsest_size,
+                        int32_t coarsest_sweeps, void *workspace_dev, size_t bytes,
+                        cudaStream_t stream);
+
+/* out[0] <- ||b - laplacian(u, spacing)||^2, deterministic (multigrid.py:247); the
+ * workspace is gd_ref_dot's. */
+int gd_ref_residual_norm2(double *out_dev, const double *u_dev, const double *b_dev, int32_t m,
+                          int32_t n, double spacing, void *workspace_dev, size_t bytes,
+                          cudaStream_t stream);
+
 /* r <- b - laplacian(u, spacing) (multigrid.py:210, operators.py:86-107). */
 int gd_ref_residual(double *r_dev, const double *u_dev, const double *b_dev, int32_t m,
                     int32_t n, double spacing, cudaStream_t stream);
