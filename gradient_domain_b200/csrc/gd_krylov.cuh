@@ -201,6 +201,7 @@ __global__ void __launch_bounds__(kThreads) k_pupdate(Args<T> a) {
   InstState &S = a.st[tl.inst];
   // every descriptor field is requested before the first is used
   const int rows = I.kr_rows, ctas = I.kr_end - I.kr_begin, pcur = S.pcur, status = S.status;
+  const bool idle = !a.act[blockIdx.x];  // no unknown: p stays zero
   const T beta = (T)S.beta;
   const double rz = S.rz;
   const T *z = a.arena + I.z_off;
@@ -211,7 +212,7 @@ __global__ void __launch_bounds__(kThreads) k_pupdate(Args<T> a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int share = rows / kWarps;
   const int y0 = tl.ty * rows + (threadIdx.x >> 5) * share, y1 = min(y0 + share, w.ny);
-  double part = y0 < w.ny ? pupdate_rows<T>(w, y0, y1, beta, z, p, pn, smem) : 0.0;
+  double part = y0 < w.ny && !idle ? pupdate_rows<T>(w, y0, y1, beta, z, p, pn, smem) : 0.0;
   double pAp;
   if (!instance_sum<kThreads>(a.part0, I.kr_begin, ctas, part, &S.ticket, &pAp)) return;
   if (threadIdx.x == 0) {
@@ -309,6 +310,7 @@ __global__ void __launch_bounds__(kThreads) k_cgupdate(Args<T> a) {
   InstState &S = a.st[tl.inst];
   const int rows = I.kr_rows, ctas = I.kr_end - I.kr_begin, status = S.status, flags = S.flags;
   const int iters = S.iters + 1;
+  const bool idle = !a.act[blockIdx.x];  // no unknown: d and r stay zero
   const T alpha = (T)S.alpha;
   const double rr_ref = S.rr_ref, ff = S.ff;
   const T *p = a.arena + (S.pcur ? I.q_off : I.p_off);
@@ -322,7 +324,7 @@ __global__ void __launch_bounds__(kThreads) k_cgupdate(Args<T> a) {
   const int y0 = tl.ty * rows + (threadIdx.x >> 5) * share, y1 = min(y0 + share, w.ny);
   const bool dzero = flags & FLAG_DZERO;
   double part = 0.0;
-  if (y0 < w.ny) {
+  if (y0 < w.ny && !idle) {
     if (ANY && code_off >= 0)
       part = cgupdate_rows<T, true>(w, a.codes + code_off, y0, y1, alpha, p, d, r, dzero, smem);
     else

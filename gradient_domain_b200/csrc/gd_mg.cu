@@ -39,6 +39,8 @@ struct gd_plan_s {
   std::vector<InstInfo> inst;
   std::vector<LevelInfo> lv;
   std::vector<Tile> tiles;
+  std::vector<Tile> class_blocks;     // 32 x 128 blocks of the masked instances' levels
+  std::vector<MaskItem> mask_items;   // the masked instances' tiles
   int fine_base = 0, fine_count = 0, depth = 0;
   int kr_base = 0, kr_count = 0;  // tiles of the Krylov kernels
   std::vector<int> down_base, down_count, up_base, up_count;     // strip maps per level
@@ -50,7 +52,7 @@ struct gd_plan_s {
   size_t arena_elems = 0, code_bytes = 0, dense_elems = 0, xs_elems = 0;
   int max_partials = 1;
   size_t o_lv = 0, o_inst = 0, o_st = 0, o_tiles = 0, o_arena = 0, o_codes = 0, o_dense = 0,
-         o_xs = 0, o_p0 = 0, o_p1 = 0, o_cnt = 0, o_nact = 0, o_trip = 0, total = 0;
+         o_xs = 0, o_act = 0, o_mblk = 0, o_mitem = 0, o_p0 = 0, o_p1 = 0, o_cnt = 0, o_nact = 0, o_trip = 0, total = 0;
   size_t bottom_smem = 0;
   // persistent launch of the coarse levels (gd_coarse.cuh): used when the plan has
   // tile levels below its strips and the device takes cooperative launches
@@ -338,6 +340,7 @@ struct Runner {
     a.counter = reinterpret_cast<unsigned *>(p->ws + p->o_cnt);
     a.n_active = reinterpret_cast<int *>(p->ws + p->o_nact);
     a.tiles = reinterpret_cast<const Tile *>(p->ws + p->o_tiles);
+    a.act = reinterpret_cast<const unsigned char *>(p->ws + p->o_act);
     a.ninst = p->n;
     a.tol2 = p->prm.tolerance * p->prm.tolerance;
     a.delta2 = p->fp64 ? 0.0 : p->prm.reliable_delta * p->prm.reliable_delta;
@@ -351,6 +354,7 @@ struct Runner {
 
   static Args<T> at_tiles(Args<T> a, int base) {
     a.tiles += base;
+    a.act += base;
     return a;
   }
 
@@ -884,6 +888,45 @@ int build_plan(gd_plan p, const gd_grid_desc *grids) {
     }
     p->up_count[l] = (int)p->tiles.size() - p->up_base[l];
   }
+  // the mask set-up's work: class blocks of every level, and the region of every tile
+  if (p->any_masked) {
+    for (int i = 0; i < p->n; ++i) {
+      const InstInfo &I = p->inst[i];
+      if (I.bc != BC_MASK) continue;
+      for (int l = I.level0; l <= I.coarsest; ++l)
+        for (int ty = 0; ty < ceil_div(p->lv[l].ny, kClassRows); ++ty)
+          for (int tx = 0; tx < ceil_div(p->lv[l].nx, kClassCols); ++tx)
+            p->class_blocks.push_back(Tile{l, i, ty, tx});
+    }
+    auto regions = [&](int base, int count, int kind, int cols, auto rows_of) {
+      for (int t = base; t < base + count; ++t) {
+        const Tile &q = p->tiles[t];
+        const InstInfo &I = p->inst[q.inst];
+        if (I.bc != BC_MASK) continue;
+        const LevelInfo &L = p->lv[q.level];
+        const int rows = rows_of(I, L);
+        p->mask_items.push_back(MaskItem{t, q.level, q.inst, kind, std::min(q.ty * rows, L.ny),
+                                         std::min((q.ty + 1) * rows, L.ny),
+                                         std::min(q.tx * cols, L.nx),
+                                         std::min((q.tx + 1) * cols, L.nx)});
+      }
+    };
+    regions(p->fine_base, p->fine_count, kFine, kFTX,
+            [](const InstInfo &, const LevelInfo &) { return kFTY; });
+    regions(p->kr_base, p->kr_count, kKrylov, kFTX,
+            [](const InstInfo &I, const LevelInfo &) { return I.kr_rows; });
+    for (int l = 0; l < p->depth; ++l) {
+      const int upw = l == 0 ? st::UpCta<true>::W : st::UpCta<false>::W;
+      regions(p->down_base[l], p->down_count[l], kDown, down_ow,
+              [](const InstInfo &, const LevelInfo &L) { return st::kSWarps * L.rows_per_warp; });
+      regions(p->up_base[l], p->up_count[l], kUp, up_ow,
+              [&](const InstInfo &, const LevelInfo &L) { return upw * L.rows_per_warp; });
+      regions(p->tdown_base[l], p->tdown_count[l], kTiles, p->tsmall[l] ? tile::kTXs : tile::kTX,
+              [&](const InstInfo &, const LevelInfo &) {
+                return p->tsmall[l] ? tile::kTYs : tile::kTY;
+              });
+    }
+  }
   p->max_partials = std::max({1, p->fine_count, p->kr_count, rz_parts});
   p->launch_cells.assign(2 * std::max(p->depth, 1), 0.0);
   p->fine_cells = 0;
@@ -950,6 +993,9 @@ int build_plan(gd_plan p, const gd_grid_desc *grids) {
   p->o_arena = sect(p->arena_elems * es);
   p->o_codes = sect(p->code_bytes);
   p->o_dense = sect(p->dense_elems * sizeof(double));
+  p->o_act = sect(p->tiles.size());
+  p->o_mblk = sect(p->class_blocks.size() * sizeof(Tile));
+  p->o_mitem = sect(p->mask_items.size() * sizeof(MaskItem));
   p->o_xs = sect(p->xs_elems * sizeof(double));
   p->o_p0 = sect(p->max_partials * sizeof(double));
   p->o_p1 = sect(p->max_partials * sizeof(double));
@@ -1066,6 +1112,15 @@ extern "C" int gd_plan_bind(gd_plan p, void *ws, size_t bytes, cudaStream_t st) 
   // pageable sources are staged before cudaMemcpyAsync returns: no sync needed
   GD_CHECK_CUDA(cudaMemcpyAsync(p->ws + p->o_tiles, p->tiles.data(),
                                 p->tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice, st));
+  GD_CHECK_CUDA(cudaMemsetAsync(p->ws + p->o_act, 1, p->tiles.size(), st));
+  if (p->any_masked) {
+    GD_CHECK_CUDA(cudaMemcpyAsync(p->ws + p->o_mblk, p->class_blocks.data(),
+                                  p->class_blocks.size() * sizeof(Tile), cudaMemcpyHostToDevice,
+                                  st));
+    GD_CHECK_CUDA(cudaMemcpyAsync(p->ws + p->o_mitem, p->mask_items.data(),
+                                  p->mask_items.size() * sizeof(MaskItem),
+                                  cudaMemcpyHostToDevice, st));
+  }
   return GD_OK;
 }
 
@@ -1078,15 +1133,10 @@ extern "C" int gd_plan_set_mask(gd_plan p, int32_t i, const uint8_t *mask, int32
   GD_REQUIRE(mpitch >= I.nx, GD_ERR_ARG, "gd_plan_set_mask: pitch %d < width %d", mpitch, I.nx);
   unsigned char *codes = (unsigned char *)(p->ws + p->o_codes);
   const LevelInfo &L0 = p->lv[I.level0];
-  k_codes_fine<<<ceil_div(L0.ny * L0.nx, 256), 256, 0, st>>>(codes + L0.code_off, L0.pitch, mask,
-                                                             mpitch, L0.ny, L0.nx);
-  for (int l = I.level0 + 1; l <= I.coarsest; ++l) {
-    const LevelInfo &F = p->lv[l - 1], &C = p->lv[l];
-    k_codes_coarse_act<<<ceil_div(C.ny * C.nx, 256), 256, 0, st>>>(
-        codes + C.code_off, C.pitch, C.ny, C.nx, codes + F.code_off, F.pitch, F.ny, F.nx);
-    k_codes_classes<<<ceil_div(C.ny * C.nx, 256), 256, 0, st>>>(codes + C.code_off, C.pitch,
-                                                                C.ny, C.nx);
-  }
+  const int grid = ceil_div(L0.nx, kMaskBlock) * ceil_div(L0.ny, kMaskBlock);
+  k_mask_levels<<<grid, kMaskThreads, 0, st>>>(
+      reinterpret_cast<const LevelInfo *>(p->ws + p->o_lv), I.level0, I.coarsest, codes, mask,
+      mpitch, &reinterpret_cast<InstState *>(p->ws + p->o_st)[i].ticket);
   GD_CHECK_LAUNCH();
   p->mask_set[i] = 1;
   p->prepared = false;
@@ -1098,7 +1148,25 @@ extern "C" int gd_plan_prepare(gd_plan p, cudaStream_t st) {
   for (int i = 0; i < p->n; ++i)
     GD_REQUIRE(p->inst[i].bc != GD_MASKED || p->mask_set[i], GD_ERR_STATE,
                "gd_plan_prepare: masked instance %d has no mask", i);
-  k_coarse_inverse<<<p->n, 256, 0, st>>>(
+  if (p->any_masked) {
+    const int nclass = (int)p->class_blocks.size();
+    const unsigned grid = (unsigned)(nclass + p->mask_items.size());
+    auto setup = [&](auto zero) {
+      using T = decltype(zero);
+      k_mask_setup<T><<<grid, kSetupThreads, 0, st>>>(
+          reinterpret_cast<const LevelInfo *>(p->ws + p->o_lv),
+          reinterpret_cast<const InstInfo *>(p->ws + p->o_inst),
+          reinterpret_cast<unsigned char *>(p->ws + p->o_codes),
+          reinterpret_cast<T *>(p->ws + p->o_arena),
+          reinterpret_cast<const Tile *>(p->ws + p->o_mblk), nclass,
+          reinterpret_cast<const MaskItem *>(p->ws + p->o_mitem),
+          reinterpret_cast<unsigned char *>(p->ws + p->o_act));
+    };
+    if (p->fp64) setup(0.0);
+    else setup(0.0f);
+    GD_CHECK_LAUNCH();
+  }
+  k_coarse_inverse<<<p->n, kInvThreads, 0, st>>>(
       reinterpret_cast<const LevelInfo *>(p->ws + p->o_lv),
       reinterpret_cast<const InstInfo *>(p->ws + p->o_inst),
       reinterpret_cast<const unsigned char *>(p->ws + p->o_codes),

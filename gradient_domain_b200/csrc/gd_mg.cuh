@@ -107,6 +107,18 @@ struct Tile {
   int ty, tx;
 };
 
+// What the mask set-up does for one tile of a masked instance: act[tile] says whether
+// any cell of the tile's own region (rows y0 .. y1 - 1, columns x0 .. x1 - 1 of its
+// level; x0 a multiple of 4) holds an unknown.  Kernels return at once from a tile
+// without one, so what they would have written there, zeros, is written by the
+// set-up: r (kFine), both p buffers (kKrylov), the level's u (kUp, kTiles), its
+// coarse level's b (kDown, kTiles).
+enum : int { kFine = 0, kKrylov = 1, kDown = 2, kUp = 3, kTiles = 4 };
+struct MaskItem {
+  int tile, level, inst, kind;
+  int y0, y1, x0, x1;
+};
+
 template <typename T>
 struct Args {
   const LevelInfo *lv;
@@ -121,6 +133,7 @@ struct Args {
   unsigned *counter;
   int *n_active;
   const Tile *tiles;
+  const unsigned char *act;  // per tile of `tiles`: holds an unknown (1 for rectangles)
   int ninst;
   double tol2, delta2;
   int max_iter;

@@ -459,7 +459,9 @@ __global__ void __launch_bounds__(kFThreads) k_submean(Args<T> a) {
   dep_enter();
   const InstInfo &Ig = a.inst[tl.inst];
   const bool own = a.st[tl.inst].xcur != 0;
-  const bool xz = a.st[tl.inst].xzero != 0;
+  // tiles without unknowns are zero, and no refresh writes them
+  const bool idle = !a.act[blockIdx.x];
+  const bool xz = idle || a.st[tl.inst].xzero != 0;
   if (!Ig.zero_mean && !own && !xz) return;
   const int ny = Ig.ny, nx = Ig.nx;
   const long long upitch = Ig.upitch;
@@ -484,65 +486,166 @@ __global__ void __launch_bounds__(kFThreads) k_submean(Args<T> a) {
 // ---------------------------------------------------------------------------
 // Setup kernels.
 
-// Level-0 classes of a masked instance from the caller's unknown mask.
-__global__ void k_codes_fine(unsigned char *code, int pitch, const unsigned char *mask,
-                             int mpitch, int ny, int nx) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= ny * nx) return;
-  const int y = k / nx, x = k - y * nx;
-  auto on = [&](int yy, int xx) {
-    return yy >= 0 && yy < ny && xx >= 0 && xx < nx && mask[(long long)yy * mpitch + xx] != 0;
-  };
-  unsigned char c = 0;
-  if (on(y, x)) c = (unsigned char)(1 + !on(y - 1, x) + !on(y + 1, x) + !on(y, x - 1) + !on(y, x + 1));
-  code[(long long)y * pitch + x] = c;
-}
-
-// Coarse activity: a coarse cell has an unknown when any of its children has.
-__global__ void k_codes_coarse_act(unsigned char *cc, int cpitch, int cny, int cnx,
-                                   const unsigned char *fc, int fpitch, int fny, int fnx) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= cny * cnx) return;
-  const int y = k / cnx, x = k - y * cnx;
-  int any = 0;
-  for (int dy = 0; dy < 2; ++dy)
-    for (int dx = 0; dx < 2; ++dx) {
-      const int fy = 2 * y + dy, fx = 2 * x + dx;
-      if (fy < fny && fx < fnx && fc[(long long)fy * fpitch + fx]) any = 1;
+// Activity (0 / 1) of every level of a masked instance from the caller's unknown
+// mask, in one launch: a coarse cell has an unknown when any of its children has.
+// A CTA reduces 64 x 64 cells of the mask through shared memory down to one cell
+// of level 6; the last one carries the few cells left to the coarsest level.
+constexpr int kMaskBlock = 64, kMaskThreads = 256;
+__global__ void __launch_bounds__(kMaskThreads)
+k_mask_levels(const LevelInfo *lv, int level0, int coarsest, unsigned char *codes,
+              const unsigned char *mask, int mpitch, unsigned *ticket) {
+  __shared__ unsigned char s[2][kMaskBlock * kMaskBlock];
+  const int across = (lv[level0].nx + kMaskBlock - 1) / kMaskBlock;  // blocks of a row
+  const int by = (int)blockIdx.x / across * kMaskBlock, bx = (int)blockIdx.x % across * kMaskBlock;
+  {
+    const LevelInfo &L = lv[level0];
+    const int ny = L.ny, nx = L.nx, pitch = L.pitch;
+    unsigned char *c = codes + L.code_off;
+    for (int g = threadIdx.x; g < kMaskBlock * kMaskBlock / 4; g += kMaskThreads) {
+      const int ry = g / (kMaskBlock / 4), rx = 4 * (g % (kMaskBlock / 4));
+      const int y = by + ry, x = bx + rx;
+      unsigned packed = 0u;
+      if (y < ny)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (x + j < nx && mask[(long long)y * mpitch + x + j]) packed |= 1u << (8 * j);
+      *reinterpret_cast<unsigned *>(&s[0][ry * kMaskBlock + rx]) = packed;
+      if (y < ny && x < pitch) *reinterpret_cast<unsigned *>(c + (long long)y * pitch + x) = packed;
     }
-  cc[(long long)y * cpitch + x] = (unsigned char)any;
+  }
+  int l = 1;
+  for (int size = kMaskBlock / 2; size >= 1 && level0 + l <= coarsest; size >>= 1, ++l) {
+    __syncthreads();
+    const LevelInfo &L = lv[level0 + l];
+    const unsigned char *f = s[(l + 1) & 1];
+    unsigned char *o = s[l & 1];
+    for (int g = threadIdx.x; g < size * size; g += kMaskThreads) {
+      const int ry = g / size, rx = g - ry * size;
+      const unsigned char *q = f + 4 * ry * size + 2 * rx;  // the finer block is 2 size wide
+      const unsigned char any = q[0] | q[1] | q[2 * size] | q[2 * size + 1];
+      o[ry * size + rx] = any;
+      const int y = (by >> l) + ry, x = (bx >> l) + rx;
+      if (y < L.ny && x < L.nx) codes[L.code_off + (long long)y * L.pitch + x] = any;
+    }
+  }
+  if (level0 + l > coarsest) return;  // the same for every CTA
+  if (!last_of_instance(ticket, (int)gridDim.x)) return;
+  for (; level0 + l <= coarsest; ++l) {
+    const LevelInfo &F = lv[level0 + l - 1], &L = lv[level0 + l];
+    for (int k = threadIdx.x; k < L.ny * L.nx; k += kMaskThreads) {
+      const int y = k / L.nx, x = k - y * L.nx;
+      unsigned char any = 0;
+      for (int dy = 0; dy < 2; ++dy)
+        for (int dx = 0; dx < 2; ++dx)
+          if (2 * y + dy < F.ny && 2 * x + dx < F.nx)
+            any |= __ldcg(codes + F.code_off + (long long)(2 * y + dy) * F.pitch + 2 * x + dx);
+      codes[L.code_off + (long long)y * L.pitch + x] = any;
+    }
+    __syncthreads();
+  }
 }
 
-// Turn activity flags into classes (1 + walls); in place is safe because a
-// value is non-zero exactly when the cell is active, before and after.
-__global__ void k_codes_classes(unsigned char *cc, int pitch, int ny, int nx) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= ny * nx) return;
-  const int y = k / nx, x = k - y * nx;
-  auto on = [&](int yy, int xx) {
-    return yy >= 0 && yy < ny && xx >= 0 && xx < nx && cc[(long long)yy * pitch + xx] != 0;
-  };
-  if (!on(y, x)) return;
-  const int w = !on(y - 1, x) + !on(y + 1, x) + !on(y, x - 1) + !on(y, x + 1);
-  cc[(long long)y * pitch + x] = (unsigned char)(1 + w);
+// Rows y0 .. y1 - 1, columns x0 .. x1 - 1 of an array set to zero by the whole CTA.
+template <typename T>
+__device__ __forceinline__ void zero_region(T *A, int pitch, int y0, int y1, int x0, int x1) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  for (int y = y0 + warp; y < y1; y += warps)
+    for (int x = x0 + lane; x < x1; x += 32) A[(long long)y * pitch + x] = T(0);
+}
+
+// The rest of the mask set-up, for all masked instances in one launch: activity to
+// classes (1 + walls) on every level - CTAs 0 .. nclass - 1, a 32 x 128 block each -
+// and the activity of every tile (MaskItem).  A class is non-zero exactly where the
+// activity was, so neighbours may be read before or after they are converted, and
+// the tiles need not wait for the classes.
+constexpr int kClassRows = 32, kClassCols = 128, kSetupThreads = 128;
+template <typename T>
+__global__ void __launch_bounds__(kSetupThreads)
+k_mask_setup(const LevelInfo *lv, const InstInfo *inst, unsigned char *codes, T *arena,
+             const Tile *blocks, int nclass, const MaskItem *items, unsigned char *act) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int NW = kSetupThreads / 32;
+  if ((int)blockIdx.x < nclass) {
+    const Tile b = blocks[blockIdx.x];
+    const LevelInfo &L = lv[b.level];
+    const int ny = L.ny, nx = L.nx, pitch = L.pitch;
+    unsigned char *c = codes + L.code_off;
+    const int x = b.tx * kClassCols + 4 * lane;
+    if (x >= nx) return;
+    const int y1 = min((b.ty + 1) * kClassRows, ny);
+    for (int y = b.ty * kClassRows + warp; y < y1; y += NW) {
+      unsigned char *row = c + (long long)y * pitch + x;
+      const unsigned own = *reinterpret_cast<const unsigned *>(row);
+      if (!own) continue;
+      const unsigned up = y > 0 ? *reinterpret_cast<const unsigned *>(row - pitch) : 0u;
+      const unsigned dn = y + 1 < ny ? *reinterpret_cast<const unsigned *>(row + pitch) : 0u;
+      const unsigned left = x > 0 ? row[-1] : 0u, right = x + 4 < nx ? row[4] : 0u;
+      unsigned packed = 0u;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const unsigned m = 0xffu << (8 * j);
+        if (!(own & m)) continue;
+        const bool l = j == 0 ? left != 0u : (own & (m >> 8)) != 0u;
+        const bool r = j == 3 ? right != 0u : (own & (m << 8)) != 0u;
+        packed |= (1u + !(up & m) + !(dn & m) + !l + !r) << (8 * j);
+      }
+      *reinterpret_cast<unsigned *>(row) = packed;
+    }
+    return;
+  }
+  const MaskItem it = items[blockIdx.x - nclass];
+  const LevelInfo &L = lv[it.level];
+  const int pitch = L.pitch;
+  const unsigned char *c = codes + L.code_off;
+  unsigned any = 0u;
+  for (int y = it.y0 + warp; y < it.y1; y += NW)
+    for (int x = it.x0 + 4 * lane; x < it.x1; x += 128)
+      any |= *reinterpret_cast<const unsigned *>(c + (long long)y * pitch + x);
+  const bool on = __syncthreads_or(any != 0u);
+  if (threadIdx.x == 0) act[it.tile] = on ? 1 : 0;
+  if (on) return;
+  const InstInfo &I = inst[it.inst];
+  if (it.kind == kFine) zero_region(arena + I.r_off, pitch, it.y0, it.y1, it.x0, it.x1);
+  if (it.kind == kKrylov) {
+    zero_region(arena + I.p_off, pitch, it.y0, it.y1, it.x0, it.x1);
+    zero_region(arena + I.q_off, pitch, it.y0, it.y1, it.x0, it.x1);
+  }
+  if (it.kind == kUp || it.kind == kTiles)
+    zero_region(arena + L.u_off, pitch, it.y0, it.y1, it.x0, it.x1);
+  if (it.kind == kDown || it.kind == kTiles) {
+    const LevelInfo &C = lv[it.level + 1];
+    zero_region(arena + C.b_off, C.pitch, it.y0 / 2, (it.y1 + 1) / 2, it.x0 / 2, (it.x1 + 1) / 2);
+  }
 }
 
 // Dense FP64 inverse of the coarsest operator of each instance by in-place
-// Gauss-Jordan (the matrix is SPD, or SPD after adding J/n for Neumann).
-__global__ void __launch_bounds__(256) k_coarse_inverse(const LevelInfo *lv, const InstInfo *inst,
-                                                        const unsigned char *codes,
-                                                        double *dense) {
+// Gauss-Jordan (the matrix is SPD, or SPD after adding J/n for Neumann).  A thread
+// keeps its elements (column tid % 64, every 16th row) in registers; each pivot's
+// row and column go through shared memory, alternating between two copies so that
+// a pivot costs one barrier (32 instances of 64 cells: 140 us with the matrix in
+// shared memory on 256 threads and an index division per element).
+constexpr int kInvThreads = 1024;
+__global__ void __launch_bounds__(kInvThreads) k_coarse_inverse(const LevelInfo *lv,
+                                                                const InstInfo *inst,
+                                                                const unsigned char *codes,
+                                                                double *dense) {
+  static_assert(kCoarsestCells == 64 && kInvThreads == 1024, "four rows of a column per thread");
   const InstInfo &I = inst[blockIdx.x];
   const LevelInfo L = lv[I.coarsest];
   const int n = L.ny * L.nx;
-  __shared__ double A[kCoarsestCells * kCoarsestCells];
   __shared__ unsigned char cls[kCoarsestCells];
-  for (int k = threadIdx.x; k < n; k += blockDim.x)
+  __shared__ double prow[2][kCoarsestCells], pcol[2][kCoarsestCells];
+  for (int k = threadIdx.x; k < n; k += kInvThreads)
     cls[k] = (unsigned char)cell_class(L, codes, k / L.nx, k % L.nx);
   __syncthreads();
   const double reg = (L.bc == BC_NEU) ? 1.0 / n : 0.0;
-  for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
-    const int i = k / n, j = k - i * n;
+  const int j = threadIdx.x & 63, i0 = threadIdx.x >> 6;
+  double A[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int i = i0 + 16 * r;
+    A[r] = 0.0;
+    if (i >= n || j >= n) continue;
     const int yi = i / L.nx, xi = i - yi * L.nx, yj = j / L.nx, xj = j - yj * L.nx;
     double v = reg;
     if (!cls[i] || !cls[j]) {
@@ -552,29 +655,30 @@ __global__ void __launch_bounds__(256) k_coarse_inverse(const LevelInfo *lv, con
     } else if (abs(yi - yj) + abs(xi - xj) == 1) {
       v -= 1.0;
     }
-    A[k] = v;
+    A[r] = v;
   }
-  __syncthreads();
-  __shared__ double piv_inv;
-  __shared__ double colk[kCoarsestCells];
   for (int k = 0; k < n; ++k) {
-    if (threadIdx.x == 0) piv_inv = 1.0 / A[k * n + k];
-    __syncthreads();
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-      A[k * n + j] = (j == k ? 1.0 : A[k * n + j]) * piv_inv;
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) colk[i] = A[i * n + k];
-    __syncthreads();
-    for (int q = threadIdx.x; q < n * n; q += blockDim.x) {
-      const int i = q / n, j = q - i * n;
-      if (i == k) continue;
-      const double f = colk[i];
-      A[q] = (j == k ? 0.0 : A[q]) - f * A[k * n + j];
+    double *row = prow[k & 1], *col = pcol[k & 1];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (i0 + 16 * r == k) row[j] = A[r];
+      if (j == k) col[i0 + 16 * r] = A[r];
     }
     __syncthreads();
+    const double inv = 1.0 / row[k];
+    const double scaled = (j == k ? 1.0 : row[j]) * inv;  // the pivot row after its division
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = i0 + 16 * r;
+      A[r] = i == k ? scaled : (j == k ? 0.0 : A[r]) - col[i] * scaled;
+    }
   }
   double *out = dense + L.inv_off;
-  for (int k = threadIdx.x; k < n * n; k += blockDim.x) out[k] = A[k];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int i = i0 + 16 * r;
+    if (i < n && j < n) out[i * n + j] = A[r];
+  }
 }
 
 }  // namespace gd

@@ -855,7 +855,7 @@ __global__ void __launch_bounds__(kSThreads, strip_min_ctas<T, false, kSThreads,
   const LevelInfo L = a.lv[tl.level];
   const LevelInfo Lc = a.lv[tl.level + 1];  // the next entry: levels are stored finest first
   dep_enter();
-  if (a.st[tl.inst].status != GD_ACTIVE) return;
+  if (a.st[tl.inst].status != GD_ACTIVE || !a.act[blockIdx.x]) return;
   fill_table(tab, L.wall);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int RB = L.rows_per_warp;  // even
@@ -1334,14 +1334,20 @@ __global__ void __launch_bounds__(UpCta<LEVEL0>::NT,
   const LevelInfo Lc = a.lv[tl.level + 1];  // the next entry: levels are stored finest first
   dep_enter();
   const bool active = a.st[tl.inst].status == GD_ACTIVE;
+  const bool idle = !a.act[blockIdx.x];  // no unknown: u stays zero, r.z too
+  if (!LEVEL0 && idle) return;
   if (active) {
-    fill_table(tab, L.wall);
+    if (!idle) fill_table(tab, L.wall);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int RB = L.rows_per_warp;  // level 0: a multiple of the instance's rz_rows
     const int y_out0 = (tl.ty * UpCta<LEVEL0>::W + warp) * RB;
     const InstInfo &II = a.inst[tl.inst];
     RzGroups rz{a.part0 + II.up0_begin + tl.tx, (L.nx + H::OW - 1) / H::OW, II.rz_rows, 0.0};
-    if (y_out0 < L.ny) {
+    if (LEVEL0 && idle) {
+      if (lane == 0)
+        for (int y = y_out0; y < min(y_out0 + RB, L.ny); y += rz.rows)
+          rz.base[(y / rz.rows) * rz.stride] = 0.0;
+    } else if (y_out0 < L.ny) {
       const int y_out1 = min(y_out0 + RB, L.ny);
       const int xl = tl.tx * H::OW - 4 * H::HL;
       const int x0 = xl + 4 * lane;
@@ -1775,9 +1781,13 @@ __global__ void __launch_bounds__(kThreads, 4) k_refresh_s(Args<T> a) {
   if (!INIT && blockIdx.x == 0 && threadIdx.x == 0) set_condition(a.refresh, 0u);
   const int flags = a.st[tl.inst].flags;
   const bool work = INIT || (flags & FLAG_RU);
+  // a tile without unknowns: r, d and the solution are zero there (the solution's
+  // copies need not hold the zeros, every reader tests the classes; the caller's x
+  // gets them at the end).  An initial residual of the caller's x clears x there.
+  const bool idle = !a.act[blockIdx.x] && !(INIT && !a.zero_start);
   double part = 0.0, part_f = 0.0;
   extern __shared__ __align__(16) unsigned char smem[];
-  if (work) {
+  if (work && !idle) {
     // descriptor fields in registers: the stores below could alias the descriptor
     const InstInfo &Ig = a.inst[tl.inst];
     const LevelInfo L = a.lv[Ig.level0];

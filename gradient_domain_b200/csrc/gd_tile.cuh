@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(NT) k_down_t(Args<T> a) {
   const LevelInfo L = a.lv[tl.level];
   const LevelInfo Lc = a.lv[tl.level + 1];
   dep_enter();
-  if (a.st[tl.inst].status != GD_ACTIVE) return;
+  if (a.st[tl.inst].status != GD_ACTIVE || !a.act[blockIdx.x]) return;
   extern __shared__ __align__(16) unsigned char smem[];
   down_tile<T, S1, NT, TY, TX>(a, tl, L, Lc, smem);
 }
@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(NT) k_up_t(Args<T> a) {
   const LevelInfo L = a.lv[tl.level];
   const LevelInfo Lc = a.lv[tl.level + 1];
   dep_enter();
-  if (a.st[tl.inst].status != GD_ACTIVE) return;
+  if (a.st[tl.inst].status != GD_ACTIVE || !a.act[blockIdx.x]) return;
   extern __shared__ __align__(16) unsigned char smem[];
   up_tile<T, S2, NT, TY, TX>(a, tl, L, Lc, smem);
 }
