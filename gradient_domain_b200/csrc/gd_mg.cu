@@ -543,29 +543,27 @@ void strip_widths(gd_plan p, int *down_ow, int *up_ow) {
   }
 }
 
-// Shared-memory layout of a bottom holding levels first..last (padded b, u and
-// classes per level, then the dense solve's FP64 right-hand side); returns its
-// size in bytes and, with `write`, records the offsets in the levels.
+// Shared-memory layout of a bottom holding levels first..last (per level u and the
+// residual with their ghosts, then b and the classes, in groups of four cells; see
+// BotLevel; then the dense solve's FP64 right-hand side); returns its size in bytes
+// and, with `write`, records the offsets in the levels.
 int bottom_layout(gd_plan p, int first, int last, size_t es, bool write) {
   size_t off = 0;
   auto a16 = [](size_t v) { return (v + 15) & ~(size_t)15; };
   for (int l = first; l <= last; ++l) {
     LevelInfo &L = p->lv[l];
-    const size_t px = (size_t)L.nx + 3, cells = px * ((size_t)L.ny + 3);
-    const size_t b = off;
-    off = a16(off + cells * es);
+    const size_t gx = ((size_t)L.nx + 3) / 4, groups = gx * L.ny;
+    const size_t ring = (gx + 1) * ((size_t)L.ny + 3) + 1;
     const size_t u = off;
-    off = a16(off + cells * es);
-    const size_t r = off;
-    off = a16(off + cells * es);
+    off = a16(off + 4 * ring * 2 * es);  // u and the residual, two pairs each
+    const size_t b = off;
+    off = a16(off + 2 * groups * 2 * es);
     const size_t c = off;
-    off = a16(off + cells);
+    off = a16(off + groups * 4);
     if (write) {
-      L.sm_b = (int)b;
       L.sm_u = (int)u;
-      L.sm_r = (int)r;
+      L.sm_b = (int)b;
       L.sm_c = (int)c;
-      L.sm_px = (int)px;
     }
   }
   // FP64 right-hand side of the dense solve, then the dense inverse
@@ -946,6 +944,17 @@ int build_plan(gd_plan p, const gd_grid_desc *grids) {
     bsm = std::max(bsm, (size_t)bottom_layout(p, p->inst[i].bottom, p->inst[i].coarsest, es,
                                               true));
   p->bottom_smem = bsm;
+  for (InstInfo &I : p->inst) {
+    const LevelInfo &B = p->lv[I.bottom], &C = p->lv[I.coarsest];
+    I.bot_ny = B.ny;
+    I.bot_nx = B.nx;
+    I.bot_pitch = B.pitch;
+    I.bot_b_off = B.b_off;
+    I.bot_u_off = B.u_off;
+    I.bot_nq = C.ny * C.nx;
+    I.bot_sm_d = C.sm_d;
+    I.bot_inv_off = C.inv_off;
+  }
   // the persistent coarse launch: tile levels below the last strip level, the
   // bottom, and the tile levels again on the way up
   {

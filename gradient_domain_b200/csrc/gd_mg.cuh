@@ -58,12 +58,11 @@ struct LevelInfo {
   int bc, level, coarse, is_bottom;
   float wall, pad0;
   int rows_per_warp;  // strip height of the down / up kernels on this level (even)
-  // bottom levels: byte offsets of the padded b, u, residual and class arrays
-  // in the bottom kernel's shared memory, their row pitch (nx + 3), the FP64
-  // right-hand side of the dense solve (coarsest level; the dense inverse
-  // follows it at sm_d + kCoarsestCells doubles) and the end of the layout
-  int sm_r;
-  int sm_b, sm_u, sm_c, sm_px, sm_d, sm_end;
+  // bottom levels: byte offsets of u (then the residual, up to b), b and the classes
+  // in the bottom kernel's shared memory (BotLevel), of the FP64 right-hand side of
+  // the dense solve (coarsest level; the dense inverse follows it at
+  // sm_d + kCoarsestCells doubles) and the end of the layout
+  int sm_b, sm_u, sm_c, sm_d, sm_end;
   long long b_off, u_off;  // element offsets into the T arena
   long long w_off;         // pre-smoothed iterate written by down, read by up
   long long code_off;      // byte offset into the code arena, -1 if rectangle
@@ -82,6 +81,9 @@ struct InstInfo {
   int up0_ctas;              // CTAs of the level-0 up kernel
   int zero_mean;
   int rz_rows;  // rows per r.z group partial: level 0's strip height for the instance alone
+  // the bottom's top level and coarsest solve, as their levels have them
+  int bot_ny, bot_nx, bot_pitch, bot_nq, bot_sm_d;
+  long long bot_b_off, bot_u_off, bot_inv_off;
   // set per solve
   const double *f;
   double *x;

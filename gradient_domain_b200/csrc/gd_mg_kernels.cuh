@@ -115,36 +115,164 @@ __device__ __forceinline__ int mirror_fine(int f, int n, bool neumann) {
   return f;
 }
 
+// Classes of the 4 cells x0..x0+3 of row y, packed one byte each.
+__device__ __forceinline__ unsigned row_classes(const LevelInfo &L, const unsigned char *codes,
+                                                int y, int x0) {
+  if (y < 0 || y >= L.ny || x0 >= L.nx || x0 + 3 < 0) return 0u;
+  if (L.code_off >= 0) {
+    if (x0 < 0) return 0u;  // x0 is a multiple of 4: a lane is wholly left of the grid or in it
+    return *reinterpret_cast<const unsigned *>(codes + L.code_off + (long long)y * L.pitch + x0);
+  }
+  const int wy = (y == 0) + (y == L.ny - 1);
+  unsigned packed = 0u;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int x = x0 + j;
+    if (x >= 0 && x < L.nx) {
+      const unsigned c = 1u + wy + (x == 0) + (x == L.nx - 1);
+      packed |= c << (8 * j);
+    }
+  }
+  return packed;
+}
+
 // ---------------------------------------------------------------------------
 // Bottom: the remaining V-cycle of one instance, every level in shared memory,
 // one CTA of kBThreads threads per instance.
 //
-// Each level keeps b, u and the cell classes in arrays padded with a ring of
-// zero ghosts (one row / column before the grid, two after; the restriction of
-// an odd-sized level reaches two cells past its edge).  A missing neighbour
-// then reads 0, as the operator defines, and Dirichlet / masked transfers read
-// zero ghosts, so no stencil needs a bounds check.  A warp works on whole rows
-// and its lanes on columns, so no index is divided.  The residual goes to its
-// own array, so b stays in shared memory for the up pass; only the top level's
-// b comes from (and its u goes back to) global memory.  The dense inverse of
-// the coarsest level is copied in by cp.async while the down pass runs.
+// What bounds it is the chain of phases (a half sweep, the residual, a transfer),
+// each a barrier apart, and within a phase the shared-memory wavefronts and
+// instructions of one SM.  A thread works on a group of four consecutive cells of
+// a row, held as two same-colour pairs E = (v0, v2) and O = (v1, v3): a half sweep
+// updates one pair, so it reads only that pair of the rows above and below and one
+// scalar beside, and a thread's own u, b and diagonal inverses stay in registers
+// for all sweeps of a level.  (One cell per lane and access with byte classes:
+// 31.0 us a launch for 64 x 64 cells x 3 instances, 25.1 so; event times.)
+//
+// u and the residual carry a ring of zero ghosts (a row above, two below - the
+// restriction of an odd-sized level reaches two cells past its edge - and one
+// group between rows), so a missing neighbour reads 0, as the operator defines,
+// and Dirichlet / masked transfers read zero ghosts.  Cells without an unknown,
+// the last group's cells beyond the grid among them, have a zero diagonal inverse
+// and stay zero.  The dense inverse of the coarsest level is copied in by cp.async
+// while the down pass runs.
 
+// Two same-colour cells.
 template <typename T>
-__device__ __forceinline__ void bot_sweep(T *u, const T *b, const unsigned char *c, int ny,
-                                          int nx, int px, const T *dinv, int colour) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int y = warp; y < ny; y += kBThreads / 32) {
-    const int row = (y + 1) * px + 1;
-    for (int x = 2 * lane + ((colour + y) & 1); x < nx; x += 64) {
-      const int i = row + x;
-      const int cl = c[i];
-      if (cl) u[i] = (b[i] + u[i - px] + u[i + px] + u[i - 1] + u[i + 1]) * dinv[cl];
-    }
-  }
-  __syncthreads();
+struct __align__(2 * sizeof(T)) Duo {
+  T x, y;
+};
+template <typename T>
+__device__ __forceinline__ Duo<T> duo(T x, T y) {
+  Duo<T> r;
+  r.x = x;
+  r.y = y;
+  return r;
+}
+__device__ __forceinline__ Duo<float> add2(Duo<float> a, Duo<float> b) {
+  const float2 r = __fadd2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y));
+  return duo(r.x, r.y);
+}
+__device__ __forceinline__ Duo<double> add2(Duo<double> a, Duo<double> b) {
+  return duo(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y));
+}
+__device__ __forceinline__ Duo<float> mul2(Duo<float> a, Duo<float> b) {
+  const float2 r = __fmul2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y));
+  return duo(r.x, r.y);
+}
+__device__ __forceinline__ Duo<double> mul2(Duo<double> a, Duo<double> b) {
+  return duo(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y));
+}
+__device__ __forceinline__ float fma1(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma1(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// A bottom level, staged in shared memory once per launch: geometry and the byte
+// offsets of its arrays.  Group (y, g) of u and the residual is element
+// (y + 1) gp + g + 1 of their E and O arrays; of b and the classes, y gx + g.
+struct BotLevel {
+  int ny, nx, gx, gp, neu, groups, pitch;
+  unsigned div;                 // ceil(2^32 / gx), 0 for gx == 1
+  const unsigned char *codes;   // class bytes of a masked level, else null
+  int uE, uO, rE, rO, bE, bO, c;
+};
+
+// Row and group of item k of a level.
+__device__ __forceinline__ void bot_item(const BotLevel &L, int k, int *y, int *g) {
+  *y = L.div ? (int)__umulhi((unsigned)k, L.div) : k;
+  *g = k - *y * L.gx;
 }
 
-// Padded index of fine row / column f for the restriction: Neumann mirrors the
+template <typename T>
+__device__ __forceinline__ Duo<T> *bot_duo(unsigned char *smem, int off) {
+  return reinterpret_cast<Duo<T> *>(smem + off);
+}
+
+// What a thread keeps of a group while it sweeps a level.
+template <typename T>
+struct BotGroup {
+  Duo<T> e, o, be, bo, ie, io;
+  int q, parity;  // element of u; parity of the row
+  __device__ __forceinline__ void load(unsigned char *smem, const BotLevel &L, const T *dinv,
+                                       int k) {
+    int y, g;
+    bot_item(L, k, &y, &g);
+    q = (y + 1) * L.gp + g + 1;
+    parity = y & 1;
+    e = bot_duo<T>(smem, L.uE)[q];
+    o = bot_duo<T>(smem, L.uO)[q];
+    be = bot_duo<T>(smem, L.bE)[k];
+    bo = bot_duo<T>(smem, L.bO)[k];
+    const unsigned c = reinterpret_cast<const unsigned *>(smem + L.c)[k];
+    ie = duo(dinv[c & 0xff], dinv[(c >> 16) & 0xff]);
+    io = duo(dinv[(c >> 8) & 0xff], dinv[c >> 24]);
+  }
+  // The cells of `colour` (cell (y, x) has colour (y + x) & 1), all one pair:
+  // ((((b + up) + down) + left) + right) / d.  Rows of both parities share a warp, so
+  // the pair is chosen by selects, not by a branch that would run both.
+  __device__ __forceinline__ void half(unsigned char *smem, const BotLevel &L, int colour) {
+    const bool odd = (colour + parity) & 1;
+    Duo<T> *const u = bot_duo<T>(smem, odd ? L.uO : L.uE);
+    const T *const side = reinterpret_cast<const T *>(smem + (odd ? L.uE : L.uO)) +
+                          (odd ? 2 * q + 2 : 2 * q - 1);
+    const Duo<T> up = u[q - L.gp], dn = u[q + L.gp];
+    const T sv = *side;
+    const Duo<T> n = odd ? e : o;  // the pair between the updated cells
+    const Duo<T> left = duo(odd ? n.x : sv, odd ? n.y : n.x);
+    const Duo<T> right = duo(odd ? n.y : n.x, odd ? sv : n.y);
+    const Duo<T> r = mul2(add2(add2(add2(add2(odd ? bo : be, up), dn), left), right),
+                          odd ? io : ie);
+    u[q] = r;
+    if (odd) o = r;
+    else e = r;
+  }
+};
+
+// `sweeps` sweeps of a level, colour `first` first.  A thread's first group stays in
+// registers; a level of more than kBThreads groups goes through shared memory for
+// the others.  (Loops are not unrolled: every launch of this kernel starts with a
+// cold instruction cache, and code that runs once costs its fetches.)
+template <typename T>
+__device__ __forceinline__ void bot_sweeps(unsigned char *smem, const BotLevel &L, const T *dinv,
+                                           int first, int sweeps) {
+  BotGroup<T> own;
+  const bool has = threadIdx.x < L.groups;
+  if (has) own.load(smem, L, dinv, threadIdx.x);
+#pragma unroll 1
+  for (int h = 0; h < 2 * sweeps; ++h) {
+    const int colour = (first + h) & 1;
+    if (has) own.half(smem, L, colour);
+    if (L.groups > kBThreads)
+#pragma unroll 1
+      for (int k = threadIdx.x + kBThreads; k < L.groups; k += kBThreads) {
+        BotGroup<T> more;
+        more.load(smem, L, dinv, k);
+        more.half(smem, L, colour);
+      }
+    __syncthreads();
+  }
+}
+
+// Row or column f of a level of n for the restriction: Neumann mirrors the
 // ghost at -1 and, for an even size n, the ghost at n (the adjoint of the
 // clamped prolongation); every other ghost reads zero.
 __device__ __forceinline__ int bot_mirror(int f, int n, bool neu) {
@@ -155,123 +283,184 @@ __device__ __forceinline__ int bot_mirror(int f, int n, bool neu) {
   return f;
 }
 
-// The few fields of a bottom level its phases read, staged in shared memory
-// once per launch: every phase after a barrier then finds them at shared-memory
-// latency instead of reloading the level descriptors from global memory.
-struct BotLevel {
-  int ny, nx, px, neu;
-  int sm_b, sm_u, sm_r, sm_c;
-};
+// Cell (y, x) of an array stored as pairs (E and O at byte offsets oE and oO, `base` the
+// element of the row's group 0).
+template <typename T>
+__device__ __forceinline__ T *bot_cell(unsigned char *smem, int oE, int oO, int base, int x) {
+  return reinterpret_cast<T *>(smem + ((x & 1) ? oO : oE)) + 2 * (base + (x >> 2)) + ((x >> 1) & 1);
+}
 
 // The bottom of one active instance, by the whole CTA (kBThreads threads); the
-// CTA's shared memory is free on entry and may be reused on return.  Every
-// phase runs on all warps: a phase's time is the chain of rows its busiest warp
-// walks, so fewer warps on the small levels were measured slower.
+// CTA's shared memory is free on entry and may be reused on return.
 template <typename T, int S1, int S2>
 __device__ __forceinline__ void bottom_instance(const Args<T> &a, const int inst,
                                                 unsigned char *smem) {
   InstState &S = a.st[inst];
   __shared__ T tdiag[kBottomLevels][8], tdinv[kBottomLevels][8];
   __shared__ BotLevel bl[kBottomLevels];
-  const int bottom = a.inst[inst].bottom, coarsest = a.inst[inst].coarsest;
-  const bool top_is_fine = bottom == a.inst[inst].level0;
-  const int nb = coarsest - bottom + 1;
+  // the instance's entry holds all that the first loads need
+  const InstInfo &I = a.inst[inst];
+  const int bottom = I.bottom, nb = I.coarsest - bottom + 1;
+  const bool top_is_fine = bottom == I.level0;
+  const int nq = I.bot_nq, sm_d = I.bot_sm_d, tny = I.bot_ny, tnx = I.bot_nx;
+  const long long tpitch = I.bot_pitch;
+  const T *const Bg = a.arena + I.bot_b_off;
+  T *const U = a.arena + I.bot_u_off;
+  const double *const inv_g = a.dense + I.bot_inv_off;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int NW = kBThreads / 32;
-  const int nq = a.lv[coarsest].ny * a.lv[coarsest].nx;
-  const int sm_d = a.lv[coarsest].sm_d;
+  const int tgx = (tnx + 3) / 4;
+  Duo<T> be = duo(T(0), T(0)), bo = be;  // b of the thread's first group of the top level
+  {
+    const int k = threadIdx.x, y = k / tgx, g = k - y * tgx;
+    if (k < tny * tgx) {  // a row's padding up to its pitch holds zeros
+      const T *p = Bg + y * tpitch + 4 * g;
+      be = duo(p[0], p[2]);
+      bo = duo(p[1], p[3]);
+    }
+  }
   double *const inv_s = reinterpret_cast<double *>(smem + sm_d) + kCoarsestCells;
-  {  // the coarsest inverse travels while the levels above are worked on
-    const double *inv_g = a.dense + a.lv[coarsest].inv_off;
-    for (int k = threadIdx.x; k < nq * nq; k += kBThreads)
-      __pipeline_memcpy_async(inv_s + k, inv_g + k, sizeof(double));
-    __pipeline_commit();
-  }
-  {  // zero every padded array up to the inverse (ghost rings stay zero for the whole launch)
-    const int bytes = sm_d + kCoarsestCells * (int)sizeof(double);
-    uint4 *z = reinterpret_cast<uint4 *>(smem);
-    for (int k = threadIdx.x; k < bytes / 16; k += kBThreads) z[k] = make_uint4(0, 0, 0, 0);
-  }
+  // the coarsest inverse travels while the levels above are worked on
+#pragma unroll 1
+  for (int k = threadIdx.x; k < nq * nq; k += kBThreads)
+    __pipeline_memcpy_async(inv_s + k, inv_g + k, sizeof(double));
+  __pipeline_commit();
   for (int q = threadIdx.x; q < nb * 8; q += kBThreads) {
     const int l = q >> 3, c = q & 7;
-    const float w = a.lv[bottom + l].wall;
-    const double d = c >= 1 && c <= 5 ? class_diag(c, w) : 1.0;
+    const LevelInfo &L = a.lv[bottom + l];
+    const double d = c >= 1 && c <= 5 ? class_diag(c, L.wall) : 1.0;
     tdiag[l][c] = (T)d;
     tdinv[l][c] = (c >= 1 && c <= 5 && d > 0.0) ? (T)(1.0 / d) : T(0);
     if (c == 0) {
-      const LevelInfo &L = a.lv[bottom + l];
-      bl[l] = BotLevel{L.ny, L.nx, L.sm_px, L.bc == BC_NEU ? 1 : 0, L.sm_b, L.sm_u, L.sm_r,
-                       L.sm_c};
+      BotLevel B;
+      B.ny = L.ny;
+      B.nx = L.nx;
+      B.gx = (L.nx + 3) / 4;
+      B.gp = B.gx + 1;
+      B.neu = L.bc == BC_NEU ? 1 : 0;
+      B.groups = B.ny * B.gx;
+      B.pitch = L.pitch;
+      B.div = B.gx > 1 ? 0xffffffffu / (unsigned)B.gx + 1u : 0u;
+      B.codes = L.code_off >= 0 ? a.codes + L.code_off : nullptr;
+      const int ring = ((B.ny + 3) * B.gp + 1) * (int)sizeof(Duo<T>);
+      const int plain = B.groups * (int)sizeof(Duo<T>);
+      B.uE = L.sm_u;
+      B.uO = B.uE + ring;
+      B.rE = B.uO + ring;
+      B.rO = B.rE + ring;
+      B.bE = L.sm_b;
+      B.bO = B.bE + plain;
+      B.c = L.sm_c;
+      bl[l] = B;
     }
   }
   __syncthreads();
-  // classes of every level, and b of the top level
-  for (int q = 0; q < nb; ++q) {
-    const LevelInfo L = a.lv[bottom + q];
-    unsigned char *c = smem + L.sm_c;
-    const int px = L.sm_px;
-    for (int y = warp; y < L.ny; y += NW)
-      for (int x = lane; x < L.nx; x += 32)
-        c[(y + 1) * px + 1 + x] = (unsigned char)cell_class(L, a.codes, y, x);
+  // zero u and the residual of every level (their ghosts stay zero); its classes
+#pragma unroll 1
+  for (int l = 0; l < nb; ++l) {
+    const BotLevel &B = bl[l];
+    uint4 *z = reinterpret_cast<uint4 *>(smem + B.uE);
+    const int n16 = (B.bE - B.uE) / 16;
+#pragma unroll 1
+    for (int k = threadIdx.x; k < n16; k += kBThreads) z[k] = make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+    for (int k = threadIdx.x; k < B.groups; k += kBThreads) {
+      int y, g;
+      bot_item(B, k, &y, &g);
+      unsigned c;
+      if (B.codes) {
+        c = *reinterpret_cast<const unsigned *>(B.codes + (long long)y * B.pitch + 4 * g);
+      } else {  // 1 + walls; the group's cells beyond the grid have class 0
+        const unsigned in = (unsigned)min(B.nx - 4 * g, 4);
+        c = (0x01010101u + 0x01010101u * ((y == 0) + (y == B.ny - 1))) >> (32 - 8 * in);
+        if (g == 0) c += 1u;
+        if (g == B.gx - 1) c += 1u << (8 * in - 8);
+      }
+      reinterpret_cast<unsigned *>(smem + B.c)[k] = c;
+    }
   }
   {
-    const LevelInfo &L = a.lv[bottom];
-    const T *B = a.arena + L.b_off;
-    const long long pitch = L.pitch;
-    const BotLevel Q = bl[0];
-    T *b = reinterpret_cast<T *>(smem + Q.sm_b);
-    for (int y = warp; y < Q.ny; y += NW)
-      for (int x = lane; x < Q.nx; x += 32)
-        b[(y + 1) * Q.px + 1 + x] = B[(long long)y * pitch + x];
+    const BotLevel &B = bl[0];
+    if (threadIdx.x < B.groups) {
+      bot_duo<T>(smem, B.bE)[threadIdx.x] = be;
+      bot_duo<T>(smem, B.bO)[threadIdx.x] = bo;
+    }
+#pragma unroll 1
+    for (int k = threadIdx.x + kBThreads; k < B.groups; k += kBThreads) {
+      int y, g;
+      bot_item(B, k, &y, &g);
+      const T *p = Bg + y * tpitch + 4 * g;
+      bot_duo<T>(smem, B.bE)[k] = duo(p[0], p[2]);
+      bot_duo<T>(smem, B.bO)[k] = duo(p[1], p[3]);
+    }
   }
   __syncthreads();
-  // down: smooth from zero, residual (into b), restriction
-  for (int q = 0; q + 1 < nb; ++q) {
-    const BotLevel L = bl[q];
-    const BotLevel C = bl[q + 1];
-    T *u = reinterpret_cast<T *>(smem + L.sm_u);
-    const T *b = reinterpret_cast<const T *>(smem + L.sm_b);
-    T *res = reinterpret_cast<T *>(smem + L.sm_r);
-    const unsigned char *c = smem + L.sm_c;
-    const int px = L.px;
-    for (int s = 0; s < S1; ++s) {
-      bot_sweep(u, b, c, L.ny, L.nx, px, tdinv[q], 0);
-      bot_sweep(u, b, c, L.ny, L.nx, px, tdinv[q], 1);
-    }
-    for (int y = warp; y < L.ny; y += NW) {
-      const int row = (y + 1) * px + 1;
-      for (int x = lane; x < L.nx; x += 32) {
-        const int i = row + x;
-        const int cl = c[i];
-        const T nbs = u[i - px] + u[i + px] + u[i - 1] + u[i + 1];
-        res[i] = cl ? b[i] - (tdiag[q][cl] * u[i] - nbs) : T(0);
+  // down: smooth from zero, residual, restriction
+#pragma unroll 1
+  for (int l = 0; l + 1 < nb; ++l) {
+    const BotLevel L = bl[l];
+    const BotLevel C = bl[l + 1];
+    bot_sweeps<T>(smem, L, tdinv[l], 0, S1);
+    {
+      const Duo<T> *uE = bot_duo<T>(smem, L.uE), *uO = bot_duo<T>(smem, L.uO);
+#pragma unroll 1
+      for (int k = threadIdx.x; k < L.groups; k += kBThreads) {
+        int y, g;
+        bot_item(L, k, &y, &g);
+        const int q = (y + 1) * L.gp + g + 1;
+        const unsigned c = reinterpret_cast<const unsigned *>(smem + L.c)[k];
+        const Duo<T> e = uE[q], o = uO[q];
+        const Duo<T> ve = add2(uE[q - L.gp], uE[q + L.gp]), vo = add2(uO[q - L.gp], uO[q + L.gp]);
+        const Duo<T> ne = add2(add2(ve, duo(uO[q - 1].y, o.x)), o);
+        const Duo<T> no = add2(add2(vo, e), duo(e.y, uE[q + 1].x));
+        const Duo<T> be = bot_duo<T>(smem, L.bE)[k], bo = bot_duo<T>(smem, L.bO)[k];
+        auto res = [&](unsigned cl, T b, T u, T nbs) {
+          return cl ? b - fma1(tdiag[l][cl], u, -nbs) : T(0);
+        };
+        bot_duo<T>(smem, L.rE)[q] = duo(res(c & 0xff, be.x, e.x, ne.x),
+                                        res((c >> 16) & 0xff, be.y, e.y, ne.y));
+        bot_duo<T>(smem, L.rO)[q] = duo(res((c >> 8) & 0xff, bo.x, o.x, no.x),
+                                        res(c >> 24, bo.y, o.y, no.y));
       }
     }
     __syncthreads();
-    T *bc = reinterpret_cast<T *>(smem + C.sm_b);
-    const unsigned char *cc = smem + C.sm_c;
-    const bool neu = L.neu != 0;
-    const int cpx = C.px;
-    for (int Iy = warp; Iy < C.ny; Iy += NW) {
-      int fy[4];
+    {  // coarse row I, fine group g: coarse columns 2 g and 2 g + 1 (none beyond the
+       // coarse groups: a group whose cells are all in the grid's last odd column pair)
+      const Duo<T> *rE = bot_duo<T>(smem, L.rE), *rO = bot_duo<T>(smem, L.rO);
+      const bool neu = L.neu != 0;
+#pragma unroll 1
+      for (int k = threadIdx.x; k < C.ny * L.gx; k += kBThreads) {
+        int I, g;
+        bot_item(L, k, &I, &g);
+        T acc0 = T(0), acc1 = T(0);
 #pragma unroll
-      for (int pp = 0; pp < 4; ++pp) fy[pp] = (bot_mirror(2 * Iy - 1 + pp, L.ny, neu) + 1) * px + 1;
-      for (int Jx = lane; Jx < C.nx; Jx += 32) {
-        const int ci = (Iy + 1) * cpx + 1 + Jx;
-        T acc = T(0);
-        if (cc[ci]) {
-          int fx[4];
+        for (int p = 0; p < 4; ++p) {
+          const int q = (bot_mirror(2 * I - 1 + p, L.ny, neu) + 1) * L.gp + g + 1;
+          const Duo<T> e = rE[q], o = rO[q];
+          T v[6] = {rO[q - 1].y, e.x, o.x, e.y, o.y, rE[q + 1].x};  // columns 4 g - 1 .. 4 g + 4
+          if (neu) {
+            if (g == 0) v[0] = v[1];
+            if (!(L.nx & 1)) {
 #pragma unroll
-          for (int r = 0; r < 4; ++r) fx[r] = bot_mirror(2 * Jx - 1 + r, L.nx, neu);
-#pragma unroll
-          for (int pp = 0; pp < 4; ++pp) {
-            T rowv = T(0);
-#pragma unroll
-            for (int r = 0; r < 4; ++r) rowv += (T)rweight(r) * res[fy[pp] + fx[r]];
-            acc += (T)rweight(pp) * rowv;
+              for (int m = 1; m < 6; ++m)
+                if (4 * g - 1 + m == L.nx) v[m] = v[m - 1];
+            }
           }
+          const T w = (T)rweight(p);
+          const T r0 = fma1(T(0.25), v[3], fma1(T(0.75), v[2], fma1(T(0.75), v[1], T(0.25) * v[0])));
+          const T r1 = fma1(T(0.25), v[5], fma1(T(0.75), v[4], fma1(T(0.75), v[3], T(0.25) * v[2])));
+          acc0 = p ? fma1(w, r0, acc0) : w * r0;
+          acc1 = p ? fma1(w, r1, acc1) : w * r1;
         }
-        bc[ci] = acc;
+        const int gc = I * C.gx + (g >> 1), hi = g & 1;  // cells 0, 1 or 2, 3 of the coarse group
+        const unsigned c = reinterpret_cast<const unsigned *>(smem + C.c)[gc] >> (16 * hi);
+        reinterpret_cast<T *>(bot_duo<T>(smem, C.bE) + gc)[hi] = (c & 0xff) ? acc0 : T(0);
+        reinterpret_cast<T *>(bot_duo<T>(smem, C.bO) + gc)[hi] = (c & 0xff00) ? acc1 : T(0);
+        // an odd number of fine groups leaves the last coarse group's upper half without one
+        if ((L.gx & 1) && g == L.gx - 1) {
+          reinterpret_cast<T *>(bot_duo<T>(smem, C.bE) + gc)[1] = T(0);
+          reinterpret_cast<T *>(bot_duo<T>(smem, C.bO) + gc)[1] = T(0);
+        }
       }
     }
     __syncthreads();
@@ -279,13 +468,10 @@ __device__ __forceinline__ void bottom_instance(const Args<T> &a, const int inst
   const BotLevel Lc = bl[nb - 1];
   {  // coarsest: dense FP64 inverse, one warp per row
     const int n = Lc.ny * Lc.nx;
-    const int px = Lc.px;
     double *bd = reinterpret_cast<double *>(smem + sm_d);
-    const T *b = reinterpret_cast<const T *>(smem + Lc.sm_b);
-    T *u = reinterpret_cast<T *>(smem + Lc.sm_u);
     for (int k = threadIdx.x; k < n; k += kBThreads) {
       const int y = k / Lc.nx, x = k - y * Lc.nx;
-      bd[k] = (double)b[(y + 1) * px + 1 + x];
+      bd[k] = (double)*bot_cell<T>(smem, Lc.bE, Lc.bO, y * Lc.gx, x);
     }
     __pipeline_wait_prior(0);
     __syncthreads();
@@ -310,57 +496,67 @@ __device__ __forceinline__ void bottom_instance(const Args<T> &a, const int inst
         const int t = warp + r * NW;
         if (t < n) {
           const int y = t / Lc.nx, x = t - y * Lc.nx;
-          u[(y + 1) * px + 1 + x] = (T)acc[r];
+          *bot_cell<T>(smem, Lc.uE, Lc.uO, (y + 1) * Lc.gp + 1, x) = (T)acc[r];
         }
       }
     }
     __syncthreads();
   }
-  // up: reload b, add the prolonged correction, post-smooth
-  for (int q = nb - 2; q >= 0; --q) {
-    const BotLevel L = bl[q];
-    const BotLevel C = bl[q + 1];
-    T *u = reinterpret_cast<T *>(smem + L.sm_u);
-    T *b = reinterpret_cast<T *>(smem + L.sm_b);
-    const T *e = reinterpret_cast<const T *>(smem + C.sm_u);
-    const unsigned char *c = smem + L.sm_c;
+  // up: add the prolonged correction, post-smooth
+#pragma unroll 1
+  for (int l = nb - 2; l >= 0; --l) {
+    const BotLevel L = bl[l];
+    const BotLevel C = bl[l + 1];
     const bool neu = L.neu != 0;
-    const int px = L.px, cpx = C.px;
-    for (int y = warp; y < L.ny; y += NW) {
-      const int row = (y + 1) * px + 1;
+    Duo<T> *uE = bot_duo<T>(smem, L.uE), *uO = bot_duo<T>(smem, L.uO);
+#pragma unroll 1
+    for (int k = threadIdx.x; k < L.groups; k += kBThreads) {
+      int y, g;
+      bot_item(L, k, &y, &g);
+      const unsigned c = reinterpret_cast<const unsigned *>(smem + L.c)[k];
+      if (!c) continue;
+      const int q = (y + 1) * L.gp + g + 1;
       const int cy = y >> 1;
       int cy2 = (y & 1) ? cy + 1 : cy - 1;
       if (neu) cy2 = min(max(cy2, 0), C.ny - 1);
-      const int r1 = (cy + 1) * cpx + 1, r2 = (cy2 + 1) * cpx + 1;
-      for (int x = lane; x < L.nx; x += 32) {
-        const int i = row + x;
-        if (!c[i]) continue;
-        const int cx = x >> 1;
-        int cx2 = (x & 1) ? cx + 1 : cx - 1;
-        if (neu) cx2 = min(max(cx2, 0), C.nx - 1);
-        u[i] += (T)0.5625 * e[r1 + cx] + (T)0.1875 * (e[r2 + cx] + e[r1 + cx2]) +
-                (T)0.0625 * e[r2 + cx2];
+      const int b1 = (cy + 1) * C.gp + 1, b2 = (cy2 + 1) * C.gp + 1;
+      T e1[4], e2[4];  // coarse columns 2 g - 1 .. 2 g + 2 of the two rows
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        int x = 2 * g - 1 + m;
+        if (neu) x = min(max(x, 0), C.nx - 1);
+        e1[m] = *bot_cell<T>(smem, C.uE, C.uO, b1, x);
+        e2[m] = *bot_cell<T>(smem, C.uE, C.uO, b2, x);
       }
+      auto plus = [&](unsigned cl, T u, int m, int f) {  // near column m, far column f
+        const T v = fma1(T(0.0625), e2[f],
+                         fma1(T(0.1875), e2[m] + e1[f], T(0.5625) * e1[m]));
+        return cl ? u + v : u;
+      };
+      const Duo<T> e = uE[q], o = uO[q];
+      uE[q] = duo(plus(c & 0xff, e.x, 1, 0), plus((c >> 16) & 0xff, e.y, 2, 1));
+      uO[q] = duo(plus((c >> 8) & 0xff, o.x, 1, 2), plus(c >> 24, o.y, 2, 3));
     }
     __syncthreads();
-    for (int s = 0; s < S2; ++s) {
-      bot_sweep(u, b, c, L.ny, L.nx, px, tdinv[q], 1);
-      bot_sweep(u, b, c, L.ny, L.nx, px, tdinv[q], 0);
-    }
+    bot_sweeps<T>(smem, L, tdinv[l], 1, S2);
   }
   const BotLevel L0 = bl[0];
-  const LevelInfo &G0 = a.lv[bottom];
-  T *U = a.arena + G0.u_off;
-  const long long pitch0 = G0.pitch;
-  const T *u0 = reinterpret_cast<const T *>(smem + L0.sm_u);
-  const T *b0 = reinterpret_cast<const T *>(smem + L0.sm_b);
   double part = 0.0;
-  for (int y = warp; y < L0.ny; y += NW) {
-    const int row = (y + 1) * L0.px + 1;
-    for (int x = lane; x < L0.nx; x += 32) {
-      const T v = u0[row + x];
-      U[(long long)y * pitch0 + x] = v;
-      part += (double)b0[row + x] * (double)v;
+#pragma unroll 1
+  for (int k = threadIdx.x; k < L0.groups; k += kBThreads) {
+    int y, g;
+    bot_item(L0, k, &y, &g);
+    const int q = (y + 1) * L0.gp + g + 1;
+    const Duo<T> e = bot_duo<T>(smem, L0.uE)[q], o = bot_duo<T>(smem, L0.uO)[q];
+    T *p = U + y * tpitch + 4 * g;
+    const T v[4] = {e.x, o.x, e.y, o.y};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (4 * g + j < L0.nx) p[j] = v[j];
+    if (top_is_fine) {
+      const Duo<T> be = bot_duo<T>(smem, L0.bE)[k], bo = bot_duo<T>(smem, L0.bO)[k];
+      part += ((double)be.x * (double)e.x + (double)bo.x * (double)o.x) +
+              ((double)be.y * (double)e.y + (double)bo.y * (double)o.y);
     }
   }
   if (top_is_fine) {

@@ -79,27 +79,6 @@ __device__ __forceinline__ V4<T> zero4() {
   return r;
 }
 
-// Classes of the 4 cells x0..x0+3 of row y, packed one byte each.
-__device__ __forceinline__ unsigned row_classes(const LevelInfo &L, const unsigned char *codes,
-                                                int y, int x0) {
-  if (y < 0 || y >= L.ny || x0 >= L.nx || x0 + 3 < 0) return 0u;
-  if (L.code_off >= 0) {
-    if (x0 < 0) return 0u;  // x0 is a multiple of 4: a lane is wholly left of the grid or in it
-    return *reinterpret_cast<const unsigned *>(codes + L.code_off + (long long)y * L.pitch + x0);
-  }
-  const int wy = (y == 0) + (y == L.ny - 1);
-  unsigned packed = 0u;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int x = x0 + j;
-    if (x >= 0 && x < L.nx) {
-      const unsigned c = 1u + wy + (x == 0) + (x == L.nx - 1);
-      packed |= c << (8 * j);
-    }
-  }
-  return packed;
-}
-
 __device__ __forceinline__ int cls(unsigned packed, int j) { return (packed >> (8 * j)) & 0xff; }
 
 template <typename T>

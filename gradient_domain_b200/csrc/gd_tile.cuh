@@ -175,7 +175,7 @@ __device__ __forceinline__ void down_tile(const Args<T> &a, const Tile tl, const
       const int ry = g / GX, gx = g - ry * GX;
       const int y = gy0 + ry, x = gx0 + 4 * gx;
       bv[it] = g < NG ? load_group(B, L, y, x) : st::zero4<T>();
-      cv[it] = g < NG ? st::row_classes(L, a.codes, y, x) : 0u;
+      cv[it] = g < NG ? row_classes(L, a.codes, y, x) : 0u;
     }
 #pragma unroll
     for (int it = 0; it < IT; ++it) {
@@ -314,7 +314,7 @@ __device__ __forceinline__ void up_tile(const Args<T> &a, const Tile tl, const L
       const int g = threadIdx.x + it * NT;
       const int ry = g / GX, gx = g - ry * GX;
       const int y = gy0 + ry, x = gx0 + 4 * gx;
-      cv[it] = g < NG ? st::row_classes(L, a.codes, y, x) : 0u;
+      cv[it] = g < NG ? row_classes(L, a.codes, y, x) : 0u;
       bv[it] = g < NG ? load_group(B, L, y, x) : st::zero4<T>();
       wv[it] = g < NG ? load_group(W, L, y, x) : st::zero4<T>();
     }
