@@ -483,6 +483,13 @@ struct FastGeom {
 template <int R, int NT>
 constexpr size_t coarse_ring_bytes() { return (size_t)R * (NT * 8 + (NT / kLanes) * 8); }
 
+// The same ring of the general up strips: kRing slots of two coarse columns a lane and
+// two outer ones a warp.
+template <typename T, int NT>
+constexpr size_t coarse_pairs_bytes() {
+  return (size_t)kRing * (NT + NT / kLanes) * 2 * sizeof(T);
+}
+
 // The up kernels stream two arrays and the coarse rows, the down kernels one
 // array; NT threads per CTA.
 template <typename T, int S, bool UP, bool ANY = true, int NT = kSThreads>
@@ -492,9 +499,11 @@ constexpr size_t strip_smem() {
                       : UP       ? (size_t)2 * R * NT * 16 + coarse_ring_bytes<R, NT>()
                                  : (size_t)R * NT * 16;
   if (!ANY) return fast;
+  // the general up strips copy the coarse rows through a ring too
+  const size_t general = level_smem<T, NT>() + (UP ? coarse_pairs_bytes<T, NT>() : 0);
   // the masked form adds a ring of packed row classes (4 bytes per lane and row)
   const size_t mask = sizeof(T) == 4 ? fast + (size_t)R * NT * 4 : 0;
-  return level_smem<T, NT>() > mask ? level_smem<T, NT>() : mask;
+  return general > mask ? general : mask;
 }
 
 // Per-lane constants of the fast strips on rectangle levels in any position
@@ -991,19 +1000,53 @@ __device__ __forceinline__ void up_strip(const Args<T> &a, const LevelInfo &L,
   unsigned Cw[U];
 #pragma unroll
   for (int k = 0; k < U; ++k) { Bw[k] = zero4<T>(); Uw[k] = zero4<T>(); Cw[k] = 0u; }
-  int ce_top = (y_start >> 1) - 1;  // coarse row held in Ce[0]
-#pragma unroll
-  for (int q = 0; q < 3; ++q) Ce[q] = coarse_interp(coarse_pair(E, Lc, ce_top + q, x0, neu));
-  Pair<T> next0 = coarse_pair(E, Lc, ce_top + 3, x0, neu);
-  Pair<T> next1 = coarse_pair(E, Lc, ce_top + 4, x0, neu);
+  // coarse rows cy - 1, cy, cy + 1 around row y (cy = y / 2), interpolated along x;
+  // before the first row the window is one row behind
+  const int cy0 = y_start >> 1;
+  Ce[0] = zero4<T>();
+  Ce[1] = coarse_interp(coarse_pair(E, Lc, cy0 - 1, x0, neu));
+  Ce[2] = coarse_interp(coarse_pair(E, Lc, cy0, x0, neu));
   constexpr int NT = UpCta<LEVEL0>::NT;
   const Ring<T, NT> rb(reinterpret_cast<T *>(smem));
   const Ring<T, NT> rw(reinterpret_cast<T *>(smem) + kRing * NT * 4);
   const CodeRing<NT> cring(reinterpret_cast<unsigned *>(smem + 2 * ring_bytes<T, NT>()));
+  // The coarse rows travel through the copy ring as well: row Y / 2 + 1 in the commit
+  // group of fine row Y (Y even), so that no strip waits for a load it has just
+  // issued (FP64, event times: 39 us a launch on a 500 x 750 level with loads two rows
+  // ahead, 18 us; 1000 x 1500: 51, 36 us).
+  const int lane = threadIdx.x & 31;
+  T *const pairs = reinterpret_cast<T *>(smem + level_smem<T, NT>());
+  T *const rc = pairs + 2 * threadIdx.x;
+  T *const ro = pairs + kRing * NT * 2 + 2 * (threadIdx.x >> 5) + (lane == 31);
+  constexpr int kCSlot = 2 * NT, kOSlot = 2 * (NT / kLanes);
+  const bool edge_lane = lane == 0 || lane == 31;
+  const int c0 = x0 >> 1;  // x0 is a multiple of 4, so this is exact for negative x0 too
+  const bool pair_in = c0 >= 0 && c0 + 1 < Lc.nx;
+  auto ccopy1 = [&](T *dst, const T *row, bool row_ok, int c) {
+    if (neu) c = min(max(c, 0), Lc.nx - 1);
+    const bool ok = row_ok && c >= 0 && c < Lc.nx;
+    __pipeline_memcpy_async(dst, ok ? row + c : E, sizeof(T), ok ? 0 : sizeof(T));
+  };
+  auto issue = [&](int q, int y) {
+    rb.issue(q, B, L, y, x0);
+    rw.issue(q, Wp, L, y, x0);
+    if (!INT && masked) cring.issue(q, L, a.codes, y, x0);
+    if (y & 1) return;
+    const int slot = q & (kRing - 1), cy = (y >> 1) + 1;
+    const int yy = neu ? min(max(cy, 0), Lc.ny - 1) : cy;
+    const bool row_ok = yy >= 0 && yy < Lc.ny;
+    const T *row = E + (long long)(row_ok ? yy : 0) * Lc.pitch;
+    T *dst = rc + slot * kCSlot;
+    if (pair_in) {
+      __pipeline_memcpy_async(dst, row_ok ? row + c0 : E, 2 * sizeof(T), row_ok ? 0 : 2 * sizeof(T));
+    } else {
+      ccopy1(dst, row, row_ok, c0);
+      ccopy1(dst + 1, row, row_ok, c0 + 1);
+    }
+    if (edge_lane) ccopy1(ro + slot * kOSlot, row, row_ok, c0 + (lane == 0 ? -1 : 2));
+  };
   for (int q = 0; q < kRing - 1; ++q) {
-    rb.issue(q, B, L, y_start + q, x0);
-    rw.issue(q, Wp, L, y_start + q, x0);
-    if (!INT && masked) cring.issue(q, L, a.codes, y_start + q, x0);
+    issue(q, y_start + q);
     __pipeline_commit();
   }
   for (int base = y_start; base <= y_last; base += U) {
@@ -1016,22 +1059,17 @@ __device__ __forceinline__ void up_strip(const Args<T> &a, const LevelInfo &L,
       Bw[wslot<U>(ph, 0)] = rb.read(step);
       V4<T> u = rw.read(step);
       if (!INT) Cw[wslot<U>(ph, 0)] = masked ? cring.read(step) : row_classes(L, nullptr, y, x0);
-      if (y + kRing - 1 <= y_last) {  // no copy of rows past the strip
-        rb.issue(step + kRing - 1, B, L, y + kRing - 1, x0);
-        rw.issue(step + kRing - 1, Wp, L, y + kRing - 1, x0);
-        if (!INT && masked) cring.issue(step + kRing - 1, L, a.codes, y + kRing - 1, x0);
+      if ((ph & 1) == 0) {  // y_start is even: a new coarse row
+        const int slot = step & (kRing - 1);
+        Pair<T> next{rc[slot * kCSlot], rc[slot * kCSlot + 1], T(0)};
+        if (edge_lane) next.outer = ro[slot * kOSlot];
+        Ce[0] = Ce[1];
+        Ce[1] = Ce[2];
+        Ce[2] = coarse_interp(next);
       }
+      if (y + kRing - 1 <= y_last) issue(step + kRing - 1, y + kRing - 1);  // no rows past the strip
       __pipeline_commit();
-      {  // prolongation of row y; the coarse window holds rows cy - 1, cy, cy + 1
-        const int cy = y >> 1;
-        if (ce_top + 1 < cy) {
-          Ce[0] = Ce[1];
-          Ce[1] = Ce[2];
-          Ce[2] = coarse_interp(next0);
-          next0 = next1;
-          ++ce_top;
-          next1 = coarse_pair(E, Lc, ce_top + 4, x0, neu);
-        }
+      {  // prolongation of row y
         const unsigned c = Cw[wslot<U>(ph, 0)];
         const V4<T> &oth = (ph & 1) ? Ce[2] : Ce[0];  // y odd <=> ph odd (y_start even)
 #pragma unroll
