@@ -1190,7 +1190,7 @@ namespace {
 template <typename T>
 void launch_init(gd_plan p, const Args<T> &fine, cudaStream_t st) {
   prof_begin(p, GD_K_INIT, p->fine_cells, st);
-  chain_launch(p, k_fmean<T>, p->fine_count, kFThreads, 0, st, fine);
+  chain_launch(p, k_fmean<T>, p->fine_count, kMeanThreads, 0, st, fine);
   chain_launch(p, st::k_refresh_s<T, true>, p->fine_count, st::kThreads, st::refresh_smem<T>(),
                st, fine);
   prof_end(p, st);

@@ -601,9 +601,13 @@ __device__ __forceinline__ double column_sum(const double *A, long long pitch, i
 
 // Mean of the right-hand side of zero-mean (Neumann) instances: the constant
 // component of f is outside the range of A and is dropped, as the DCT solver
-// drops it by zeroing the DC coefficient (solvers.py:258-261).
+// drops it by zeroing the DC coefficient (solvers.py:258-261).  Four threads share
+// a column of a fine tile and each requests its 16 rows before it adds the first:
+// one memory latency a tile (29-instance batch: 37 us a launch with one thread a
+// column and eight rows at a time, 15 us).
+constexpr int kMeanThreads = 512, kMeanRows = kFTY / (kMeanThreads / kFTX);
 template <typename T>
-__global__ void __launch_bounds__(kFThreads) k_fmean(Args<T> a) {
+__global__ void __launch_bounds__(kMeanThreads) k_fmean(Args<T> a) {
   const Tile tl = a.tiles[blockIdx.x];
   dep_enter();
   if (blockIdx.x == 0 && threadIdx.x == 0) {  // a solve starts
@@ -616,11 +620,21 @@ __global__ void __launch_bounds__(kFThreads) k_fmean(Args<T> a) {
     if (blockIdx.x == I.fine_begin && threadIdx.x == 0) a.st[tl.inst].fmean = 0.0;
     return;
   }
-  const int Y0 = tl.ty * kFTY, gx = tl.tx * kFTX + threadIdx.x;
-  const double part = gx < I.nx ? column_sum(I.f, I.upitch, Y0, min(Y0 + kFTY, I.ny), gx) : 0.0;
+  const int gx = tl.tx * kFTX + threadIdx.x % kFTX;
+  const int y0 = tl.ty * kFTY + threadIdx.x / kFTX * kMeanRows;
+  const double *f = I.f + y0 * I.upitch + gx;
+  const long long pitch = I.upitch;
+  const int rows = gx < I.nx ? I.ny - y0 : 0;
+  double v[kMeanRows];
+#pragma unroll
+  for (int k = 0; k < kMeanRows; ++k) v[k] = k < rows ? f[k * pitch] : 0.0;
+#pragma unroll
+  for (int o = kMeanRows / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < o; ++k) v[k] += v[k + o];
   double sum;
-  if (instance_sum<kFThreads>(a.part0, I.fine_begin, I.fine_end - I.fine_begin, part,
-                              &a.st[tl.inst].ticket, &sum) &&
+  if (instance_sum<kMeanThreads>(a.part0, I.fine_begin, I.fine_end - I.fine_begin, v[0],
+                                 &a.st[tl.inst].ticket, &sum) &&
       threadIdx.x == 0)
     a.st[tl.inst].fmean = sum / ((double)I.ny * (double)I.nx);
 }
@@ -687,10 +701,21 @@ __global__ void __launch_bounds__(kFThreads) k_submean(Args<T> a) {
 // A CTA reduces 64 x 64 cells of the mask through shared memory down to one cell
 // of level 6; the last one carries the few cells left to the coarsest level.
 constexpr int kMaskBlock = 64, kMaskThreads = 256;
+constexpr int kMaxMaskLevels = 32;  // sides below 2^31 have at most this many levels
 __global__ void __launch_bounds__(kMaskThreads)
 k_mask_levels(const LevelInfo *lv, int level0, int coarsest, unsigned char *codes,
               const unsigned char *mask, int mpitch, unsigned *ticket) {
   __shared__ unsigned char s[2][kMaskBlock * kMaskBlock];
+  // every level's descriptor at once, so that no level of the pyramid waits for its own
+  struct Level {
+    int ny, nx, pitch;
+    unsigned char *c;
+  };
+  __shared__ Level lev[kMaxMaskLevels];
+  if (threadIdx.x <= coarsest - level0) {
+    const LevelInfo &L = lv[level0 + threadIdx.x];
+    lev[threadIdx.x] = Level{L.ny, L.nx, L.pitch, codes + L.code_off};
+  }
   const int across = (lv[level0].nx + kMaskBlock - 1) / kMaskBlock;  // blocks of a row
   const int by = (int)blockIdx.x / across * kMaskBlock, bx = (int)blockIdx.x % across * kMaskBlock;
   {
@@ -712,7 +737,7 @@ k_mask_levels(const LevelInfo *lv, int level0, int coarsest, unsigned char *code
   int l = 1;
   for (int size = kMaskBlock / 2; size >= 1 && level0 + l <= coarsest; size >>= 1, ++l) {
     __syncthreads();
-    const LevelInfo &L = lv[level0 + l];
+    const Level L = lev[l];
     const unsigned char *f = s[(l + 1) & 1];
     unsigned char *o = s[l & 1];
     for (int g = threadIdx.x; g < size * size; g += kMaskThreads) {
@@ -721,21 +746,21 @@ k_mask_levels(const LevelInfo *lv, int level0, int coarsest, unsigned char *code
       const unsigned char any = q[0] | q[1] | q[2 * size] | q[2 * size + 1];
       o[ry * size + rx] = any;
       const int y = (by >> l) + ry, x = (bx >> l) + rx;
-      if (y < L.ny && x < L.nx) codes[L.code_off + (long long)y * L.pitch + x] = any;
+      if (y < L.ny && x < L.nx) L.c[(long long)y * L.pitch + x] = any;
     }
   }
   if (level0 + l > coarsest) return;  // the same for every CTA
   if (!last_of_instance(ticket, (int)gridDim.x)) return;
   for (; level0 + l <= coarsest; ++l) {
-    const LevelInfo &F = lv[level0 + l - 1], &L = lv[level0 + l];
+    const Level F = lev[l - 1], L = lev[l];
     for (int k = threadIdx.x; k < L.ny * L.nx; k += kMaskThreads) {
       const int y = k / L.nx, x = k - y * L.nx;
       unsigned char any = 0;
       for (int dy = 0; dy < 2; ++dy)
         for (int dx = 0; dx < 2; ++dx)
           if (2 * y + dy < F.ny && 2 * x + dx < F.nx)
-            any |= __ldcg(codes + F.code_off + (long long)(2 * y + dy) * F.pitch + 2 * x + dx);
-      codes[L.code_off + (long long)y * L.pitch + x] = any;
+            any |= __ldcg(F.c + (long long)(2 * y + dy) * F.pitch + 2 * x + dx);
+      L.c[(long long)y * L.pitch + x] = any;
     }
     __syncthreads();
   }
@@ -816,65 +841,97 @@ k_mask_setup(const LevelInfo *lv, const InstInfo *inst, unsigned char *codes, T 
 
 // Dense FP64 inverse of the coarsest operator of each instance by in-place
 // Gauss-Jordan (the matrix is SPD, or SPD after adding J/n for Neumann).  A thread
-// keeps its elements (column tid % 64, every 16th row) in registers; each pivot's
-// row and column go through shared memory, alternating between two copies so that
-// a pivot costs one barrier (32 instances of 64 cells: 140 us with the matrix in
-// shared memory on 256 threads and an index division per element).
-constexpr int kInvThreads = 1024;
+// keeps 4 x 4 elements in registers (rows ti + 16 a, columns tj + 16 b).  Each pivot's
+// row and column go through shared memory, in two copies by turns, so that a pivot
+// costs one barrier; with the pivot's own row and column cleared and -1 in its place
+// in the column, one multiply-add serves every element.  The next pivot's owner
+// divides once for all.  (32 instances of 64 cells: 140 us with the matrix in shared
+// memory and an index division per element, 37 us with 1024 threads of four elements,
+// 30 us.)
+constexpr int kInvThreads = 256;
 __global__ void __launch_bounds__(kInvThreads) k_coarse_inverse(const LevelInfo *lv,
                                                                 const InstInfo *inst,
                                                                 const unsigned char *codes,
                                                                 double *dense) {
-  static_assert(kCoarsestCells == 64 && kInvThreads == 1024, "four rows of a column per thread");
+  static_assert(kCoarsestCells == 64, "16 x 16 threads of 4 x 4 elements");
   const InstInfo &I = inst[blockIdx.x];
   const LevelInfo L = lv[I.coarsest];
   const int n = L.ny * L.nx;
   __shared__ unsigned char cls[kCoarsestCells];
-  __shared__ double prow[2][kCoarsestCells], pcol[2][kCoarsestCells];
+  __shared__ double prow[2][kCoarsestCells], pcol[2][kCoarsestCells], pinv[2];
   for (int k = threadIdx.x; k < n; k += kInvThreads)
     cls[k] = (unsigned char)cell_class(L, codes, k / L.nx, k % L.nx);
   __syncthreads();
   const double reg = (L.bc == BC_NEU) ? 1.0 / n : 0.0;
-  const int j = threadIdx.x & 63, i0 = threadIdx.x >> 6;
-  double A[4];
+  const int ti = threadIdx.x >> 4, tj = threadIdx.x & 15;
+  double A[4][4];
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int i = i0 + 16 * r;
-    A[r] = 0.0;
-    if (i >= n || j >= n) continue;
-    const int yi = i / L.nx, xi = i - yi * L.nx, yj = j / L.nx, xj = j - yj * L.nx;
-    double v = reg;
-    if (!cls[i] || !cls[j]) {
-      v = (i == j && !cls[i]) ? 1.0 : 0.0;
-    } else if (i == j) {
-      v += class_diag(cls[i], L.wall);
-    } else if (abs(yi - yj) + abs(xi - xj) == 1) {
-      v -= 1.0;
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int i = ti + 16 * r, j = tj + 16 * c;
+      double v = i == j ? 1.0 : 0.0;  // rows and columns beyond n: the identity
+      if (i < n && j < n) {
+        const int yi = i / L.nx, xi = i - yi * L.nx, yj = j / L.nx, xj = j - yj * L.nx;
+        v = reg;
+        if (!cls[i] || !cls[j]) {
+          v = (i == j && !cls[i]) ? 1.0 : 0.0;
+        } else if (i == j) {
+          v += class_diag(cls[i], L.wall);
+        } else if (abs(yi - yj) + abs(xi - xj) == 1) {
+          v -= 1.0;
+        }
+      }
+      A[r][c] = v;
     }
-    A[r] = v;
-  }
-  for (int k = 0; k < n; ++k) {
-    double *row = prow[k & 1], *col = pcol[k & 1];
+  if (threadIdx.x == 0) pinv[0] = 1.0 / A[0][0];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      if (i0 + 16 * r == k) row[j] = A[r];
-      if (j == k) col[i0 + 16 * r] = A[r];
-    }
-    __syncthreads();
-    const double inv = 1.0 / row[k];
-    const double scaled = (j == k ? 1.0 : row[j]) * inv;  // the pivot row after its division
+  for (int q = 0; q < 4; ++q) {
+#pragma unroll 1
+    for (int t = 0; t < 16; ++t) {
+      const int k = 16 * q + t;
+      if (k >= n) break;
+      double *row = prow[k & 1], *col = pcol[k & 1];
+      if (ti == t) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int i = i0 + 16 * r;
-      A[r] = i == k ? scaled : (j == k ? 0.0 : A[r]) - col[i] * scaled;
+        for (int c = 0; c < 4; ++c) {
+          row[tj + 16 * c] = tj + 16 * c == k ? 1.0 : A[q][c];
+          if (tj + 16 * c != k) A[q][c] = 0.0;
+        }
+      }
+      if (tj == t) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          col[ti + 16 * r] = ti + 16 * r == k ? -1.0 : A[r][q];
+          A[r][q] = 0.0;
+        }
+      }
+      __syncthreads();
+      const double inv = pinv[k & 1];
+      double rs[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) rs[c] = row[tj + 16 * c] * inv;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const double f = col[ti + 16 * r];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) A[r][c] -= f * rs[c];
+      }
+      if (ti == tj && ti == ((t + 1) & 15)) {  // the thread of pivot k + 1
+        double d = A[q][q];
+        if (t == 15 && q < 3) d = A[q < 3 ? q + 1 : 3][q < 3 ? q + 1 : 3];
+        pinv[(k + 1) & 1] = 1.0 / d;
+      }
     }
   }
   double *out = dense + L.inv_off;
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int i = i0 + 16 * r;
-    if (i < n && j < n) out[i * n + j] = A[r];
-  }
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int i = ti + 16 * r, j = tj + 16 * c;
+      if (i < n && j < n) out[i * n + j] = A[r][c];
+    }
 }
 
 }  // namespace gd
