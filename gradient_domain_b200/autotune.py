@@ -51,7 +51,7 @@ from .plan import Instance, PoissonPlan, SolveParams
 SPACE: tuple[tuple[str, tuple[int, ...]], ...] = (
     ("sweeps", (2, 1, 3)),
     ("strip_target_warps", (0, 900, 3600)),
-    ("tile_cells", (262144, 65536, 1048576)),
+    ("tile_cells", (0, 65536, 262144, 1048576)),  # 0: the library's rule
     ("bottom_cells", (4096, 1024, 16384)),
 )
 

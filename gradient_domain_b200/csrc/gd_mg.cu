@@ -591,6 +591,14 @@ int choose_bottom(gd_plan p, int level0, int last, size_t es) {
   return last;
 }
 
+// Does a level above the bottom run on the shared-memory tile kernels?
+bool on_tile_kernels(const gd_plan p, const LevelInfo &L) {
+  const long long most = p->prm.tile_cells > 0 ? p->prm.tile_cells
+                         : L.bc == BC_MASK     ? kTileCellsMasked
+                                               : kTileCells;
+  return L.level >= 1 && (long long)L.ny * L.nx <= most;
+}
+
 // Level 0's default strip rule: warps per launch.
 constexpr int kLevel0TargetWarps = 1800;
 
@@ -610,12 +618,11 @@ constexpr int kLevel0TargetWarps = 1800;
 // instead of 64 rows and 1.03 waves).  `only` >= 0: that instance alone.
 int strip_rows(const gd_plan p, const std::vector<int> &bottoms, int l, int down_ow, int up_ow,
                const long long cap[3], int target, int only = -1) {
-  const long long tile_max = p->prm.tile_cells > 0 ? p->prm.tile_cells : kTileCells;
   auto strip_level = [&](int i) {
     if (only >= 0 && i != only) return false;
     if (l >= bottoms[i]) return false;
     const LevelInfo &L = p->lv[p->inst[i].level0 + l];
-    return !(l >= 1 && (long long)L.ny * L.nx <= tile_max);  // else on the tile kernels
+    return !on_tile_kernels(p, L);
   };
   if (target > 0) {
     const int ow = std::min(down_ow, up_ow);
@@ -814,11 +821,9 @@ int build_plan(gd_plan p, const gd_grid_desc *grids) {
   p->tup_base.assign(p->depth, 0);
   p->tup_count.assign(p->depth, 0);
   p->tile_cells.assign(std::max(p->depth, 1), 0.0);
-  // coarse levels up to tile_max cells run on the shared-memory tile kernels
-  const long long tile_max = p->prm.tile_cells > 0 ? p->prm.tile_cells : kTileCells;
   auto on_tiles = [&](int i, int l) {
     const LevelInfo &F = p->lv[p->inst[i].level0 + l];
-    return l >= 1 && (long long)F.ny * F.nx <= tile_max;
+    return on_tile_kernels(p, F);
   };
   p->tsmall.assign(p->depth, 0);
   for (int l = 1; l < p->depth; ++l) {

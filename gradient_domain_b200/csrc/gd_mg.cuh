@@ -15,9 +15,15 @@ constexpr int kCoarsestCells = 64;
 constexpr int kBottomCells = 4096;
 constexpr int kBottomSmem = 220 * 1024;
 constexpr int kBottomLevels = 24;  // most levels one bottom holds
-// Coarse levels (below level 0, above the bottom) with at most kTileCells
-// cells run on the shared-memory tile kernels; larger ones on the strips.
-constexpr int kTileCells = 1 << 18;
+// Coarse levels (below level 0, above the bottom) with at most kTileCells cells, or
+// kTileCellsMasked on masked instances, run on the shared-memory tile kernels; larger
+// ones on the strips.  Solves with the level named on strips / on tiles: 375 000 cells
+// (FP64 1000 x 1500) 2.45 / 2.37 ms, 391 937 x 3 (1022 x 1533 x 3) 1.69 / 1.68,
+// 490 000 x 3 (1400 x 1400 x 3) 1.74 / 1.77 and FP64 2.95 / 3.06, 1 000 000 x 3
+// 3.00 / 3.17; masked, whose strips carry the classes' code, 489 258 x 3
+// (1411 x 1387 x 3) 3.31 / 3.20.  The rule looks at the instance alone, because the
+// two kernels round differently and a batch gives every instance its own bits.
+constexpr int kTileCells = 3 << 17, kTileCellsMasked = 1 << 19;
 
 // Fine-level (level 0) kernels: 64 rows x 128 columns per CTA of 128 threads
 // (four warps, each 16 rows x 128 columns).  Down / up kernels use the same

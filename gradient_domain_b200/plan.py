@@ -49,7 +49,7 @@ class SolveParams:
     use_graph: bool = True        # from a plan's second solve on: one graph, device-side loop
     strip_target_warps: int | None = None  # strip height: 0 = fewest waves x rows, else warps per launch
     bottom_cells: int | None = None  # largest level solved inside the one-CTA bottom (0 = 4096)
-    tile_cells: int | None = None    # largest coarse level on shared-memory tiles (0 = 262144)
+    tile_cells: int | None = None    # largest coarse level on shared-memory tiles (0 = 393216, masked 524288)
     zero_start: bool = False      # start from x = 0; x is only written (need not be zeroed)
     persistent_coarse: bool = False  # small coarse levels + bottom in one persistent launch
     dependent_launch: bool = False   # kernels launched as programmatic dependents

@@ -79,7 +79,8 @@ typedef struct gd_params {
                                  coarse levels the height with the fewest waves x
                                  rows (occupancy queried per kernel)               */
   int32_t bottom_cells;       /* largest level the one-CTA bottom takes (0 = 4096)   */
-  int32_t tile_cells;         /* largest coarse level on shared-memory tiles (0 = 262144) */
+  int32_t tile_cells;         /* largest coarse level on shared-memory tiles (0 = 393216,
+                                 masked instances 524288) */
   int32_t zero_start;         /* nonzero: every solve starts from x = 0 and x is only
                                  written (it need not be initialised), as the
                                  reference's solvers start (solvers.py:143)           */
