@@ -53,7 +53,6 @@ namespace dct {
 constexpr int kMaxLen = 8192;   // longest line (128 KB of complex values in shared memory)
 constexpr int kMaxPasses = 14;
 constexpr int kThreads = 256;   // most threads of the run-time kernels; the large-prime ones' size
-constexpr int kMaxPerThread = kMaxLen / kThreads;  // outputs per thread of a large-prime pass
 
 // One pass of a run-time transform: radix r on sub-transforms of length r m;
 // step = N / (r m); div = ceil(2^32 / m) divides butterfly numbers by m.
@@ -87,25 +86,28 @@ inline double pass_cost(int r) {
     case 14: return 8 + 19.0;
     case 15: return 8 + 18.0;
     case 16: return 8 + 17.0;
-    default: return 8 + 10.0 * r;  // a prime above 13: direct
+    default: return 16 + 2.0 * r;  // a prime above 13: symmetric sums
   }
 }
 
-// Radices of the cheapest factorisation of n, primes above 13 on their own.
-inline double cheapest(int n, int *first) {
+// Composite radices up to `cap`.
+inline bool usable(int r, int cap) { return r <= cap || r == 5 || r == 7 || r == 11 || r == 13; }
+
+// First radix of the cheapest factorisation of n, primes above 13 on their own.
+inline double cheapest(int n, int cap, int *first) {
   double best = -1.0;
   *first = n;
   if (n == 1) return 0.0;
   auto consider = [&](int r) {
     int rest;
-    const double c = pass_cost(r) + cheapest(n / r, &rest);
+    const double c = pass_cost(r) + cheapest(n / r, cap, &rest);
     if (best < 0.0 || c < best) {
       best = c;
       *first = r;
     }
   };
   for (int r = 16; r >= 2; --r)
-    if (n % r == 0) consider(r);
+    if (n % r == 0 && usable(r, cap)) consider(r);
   if (best >= 0.0) return best;
   int q = 17;
   while (q * q <= n && n % q) q += 2;
@@ -113,13 +115,19 @@ inline double cheapest(int n, int *first) {
   return best;
 }
 
-inline Radices choose_passes(int n) {
+// Passes for `lines` lines of length n.  A short line's CTA is a warp or two, and a
+// launch of few of them is as long as one thread's butterflies: radices up to kSmallCap
+// then (360 x 240: 36 us a solve with radices up to 16, 30 us), 16 where there are
+// enough CTAs, or threads in one, to keep the FP64 pipes busy.
+constexpr int kShortLine = 512, kFewLines = 8 * 148, kSmallCap = 8;
+inline Radices choose_passes(int n, int lines) {
+  const int cap = n < kShortLine && lines <= kFewLines ? kSmallCap : 16;
   Radices f;
   f.n = n;
   int r[kMaxPasses], count = 0;
   for (int m = n; m > 1;) {
     int first;
-    cheapest(m, &first);
+    cheapest(m, cap, &first);
     r[count++] = first;
     m /= first;
   }
@@ -841,38 +849,71 @@ __device__ __forceinline__ void dit_pass(double2 *z, int n, const Pass &p, const
   }
 }
 
-// A pass of a prime radix above 13, in shared memory: one output per thread and step,
-// computed into registers from the whole butterfly, then written back after a barrier.
+// A pass of a prime radix r above 13, in shared memory, by the symmetric sums and
+// differences of the samples j and r - j (formed in place first): a thread computes
+// the outputs k and r - k of a butterfly together, 4 multiply-adds per pair of
+// samples where a direct transform takes 16, into registers, and they are written
+// back after a barrier.  Neighbouring threads take neighbouring butterflies, so the
+// roots are broadcast and the samples contiguous.
+constexpr int kMaxPairs = (kMaxLen / 2 + kMaxLen / 34 + kThreads - 1) / kThreads;
 template <int SIGN>
 __device__ void prime_pass(double2 *z, int n, const Pass &p, const double2 *tw) {
-  const int r = p.r, m = p.m, L = r * m, step = p.step, s = n / r;
-  double2 res[kMaxPerThread];
+  const int r = p.r, m = p.m, step = p.step, s = n / r, H = (r - 1) / 2;
+  // s butterflies; butterfly b: first element, twiddle index k
+  for (int i = threadIdx.x; i < s * H; i += kThreads) {
+    const int j = i / s + 1, b = i - (j - 1) * s;
+    int k;
+    const int first = butterfly(p, b, &k);
+    double2 x = z[at(first + j * m)], y = z[at(first + (r - j) * m)];
+    if (SIGN > 0) {  // DIT: input twiddles
+      x = cmulc(x, tw[j * k * step]);
+      y = cmulc(y, tw[(r - j) * k * step]);
+    }
+    z[at(first + j * m)] = cadd(x, y);
+    z[at(first + (r - j) * m)] = csub(x, y);
+  }
+  __syncthreads();
+  double2 lo[kMaxPairs], hi[kMaxPairs];
 #pragma unroll
-  for (int c = 0; c < kMaxPerThread; ++c) {
-    const int o = threadIdx.x + c * kThreads;
-    if (o < n) {
-      const int blk = o / L, rem = o - blk * L;
-      const int q = rem / m, k = rem - q * m;
-      const int first = blk * L + k;
-      double2 acc = make_double2(0.0, 0.0);
+  for (int c = 0; c < kMaxPairs; ++c) {
+    const int i = threadIdx.x + c * kThreads;
+    if (i < s * (H + 1)) {
+      const int q = i / s, b = i - q * s;  // outputs q and r - q (q == 0: that one alone)
+      int k;
+      const int first = butterfly(p, b, &k);
+      double2 u = z[at(first)], v = make_double2(0.0, 0.0);
       int e = 0;  // (j q) mod r
-      for (int j = 0; j < r; ++j) {
-        double2 v = z[at(first + j * m)];
-        if (SIGN > 0 && j) v = cmulc(v, tw[j * k * step]);  // DIT: input twiddle
-        const double2 w = tw[e * s];
-        acc = cadd(acc, SIGN < 0 ? cmul(v, w) : cmulc(v, w));
+      for (int j = 1; j <= H; ++j) {
         e += q;
         if (e >= r) e -= r;
+        const double2 t = z[at(first + j * m)], d = z[at(first + (r - j) * m)];
+        const double2 w = tw[e * s];  // cos, -sin
+        u.x += w.x * t.x;
+        u.y += w.x * t.y;
+        v.x -= w.y * d.x;
+        v.y -= w.y * d.y;
       }
-      if (SIGN < 0 && q) acc = cmul(acc, tw[q * k * step]);  // DIF: output twiddle
-      res[c] = acc;
+      double2 x = make_double2(u.x - SIGN * v.y, u.y + SIGN * v.x);
+      double2 y = make_double2(u.x + SIGN * v.y, u.y - SIGN * v.x);
+      if (SIGN < 0 && q) {  // DIF: output twiddles
+        x = cmul(x, tw[q * k * step]);
+        y = cmul(y, tw[(r - q) * k * step]);
+      }
+      lo[c] = x;
+      hi[c] = y;
     }
   }
   __syncthreads();
 #pragma unroll
-  for (int c = 0; c < kMaxPerThread; ++c) {
-    const int o = threadIdx.x + c * kThreads;
-    if (o < n) z[at(o)] = res[c];
+  for (int c = 0; c < kMaxPairs; ++c) {
+    const int i = threadIdx.x + c * kThreads;
+    if (i < s * (H + 1)) {
+      const int q = i / s, b = i - q * s;
+      int k;
+      const int first = butterfly(p, b, &k);
+      z[at(first + q * m)] = lo[c];
+      if (q) z[at(first + (r - q) * m)] = hi[c];
+    }
   }
 }
 
@@ -1148,8 +1189,8 @@ extern "C" int gd_dct_plan_create(int32_t h, int32_t w, gd_dct_plan *out) {
   p->h = h;
   p->w = w;
   p->hp = (h + 1) & ~1;
-  p->rh = dct::choose_passes(h);
-  p->rw = dct::choose_passes(w);
+  p->rh = dct::choose_passes(h, w);
+  p->rw = dct::choose_passes(w, h);
   size_t o = 0;
   p->o_t = o;
   o = dct::a256(o + (size_t)((w + 1) / 2) * p->hp * sizeof(double2));
