@@ -43,6 +43,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <map>
 #include <type_traits>
 
 #include "gd_internal.cuh"
@@ -93,25 +94,29 @@ inline double pass_cost(int r) {
 // Composite radices up to `cap`.
 inline bool usable(int r, int cap) { return r <= cap || r == 5 || r == 7 || r == 11 || r == 13; }
 
-// First radix of the cheapest factorisation of n, primes above 13 on their own.
-inline double cheapest(int n, int cap, int *first) {
-  double best = -1.0;
-  *first = n;
-  if (n == 1) return 0.0;
+// Cost and first radix of the cheapest factorisation of n, primes above 13 on their own;
+// `known` holds the divisors of the length that have been looked at.
+struct Cheapest {
+  double cost;
+  int first;
+};
+inline Cheapest cheapest(int n, int cap, std::map<int, Cheapest> &known) {
+  if (n == 1) return Cheapest{0.0, 1};
+  const auto it = known.find(n);
+  if (it != known.end()) return it->second;
+  Cheapest best{-1.0, n};
   auto consider = [&](int r) {
-    int rest;
-    const double c = pass_cost(r) + cheapest(n / r, cap, &rest);
-    if (best < 0.0 || c < best) {
-      best = c;
-      *first = r;
-    }
+    const double c = pass_cost(r) + cheapest(n / r, cap, known).cost;
+    if (best.cost < 0.0 || c < best.cost) best = Cheapest{c, r};
   };
   for (int r = 16; r >= 2; --r)
     if (n % r == 0 && usable(r, cap)) consider(r);
-  if (best >= 0.0) return best;
-  int q = 17;
-  while (q * q <= n && n % q) q += 2;
-  consider(n % q ? n : q);
+  if (best.cost < 0.0) {
+    int q = 17;
+    while (q * q <= n && n % q) q += 2;
+    consider(n % q ? n : q);
+  }
+  known[n] = best;
   return best;
 }
 
@@ -125,12 +130,8 @@ inline Radices choose_passes(int n, int lines) {
   Radices f;
   f.n = n;
   int r[kMaxPasses], count = 0;
-  for (int m = n; m > 1;) {
-    int first;
-    cheapest(m, cap, &first);
-    r[count++] = first;
-    m /= first;
-  }
+  std::map<int, Cheapest> known;
+  for (int m = n; m > 1; m /= r[count - 1]) r[count++] = cheapest(m, cap, known).first;
   std::sort(r, r + count, [](int a, int b) { return a > b; });
   int L = n;
   for (int s = 0; s < count; ++s) {
