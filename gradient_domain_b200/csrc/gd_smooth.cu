@@ -146,13 +146,15 @@ __device__ __forceinline__ constexpr int sl(int ph, int k) {
   return ((ph - k) % U + U) % U;
 }
 
-// Rows of prefetch in registers: U for FP32, 2 for FP64 (both divide the even U).
+// Rows of prefetch in registers: U for FP32 with one or two sweeps, half of it with three
+// or four, whose windows leave fewer registers (4096^2: 108 and 244 us with all of it, 87
+// and 130 us with half), 2 for FP64 (all divide the even U).
 // (Measured alternatives for one FP32 sweep on 4096^2: eight rows need 157
 // registers, or spill at 128; a per-lane cp.async ring in shared memory with five
 // rows in flight at 59 registers was 3-7 % slower.)
 template <typename T, int S>
 struct SmPrefetch {
-  static constexpr int P = sizeof(T) == 4 ? SmGeom<S>::U : 2;
+  static constexpr int P = sizeof(T) != 4 ? 2 : S <= 2 ? SmGeom<S>::U : SmGeom<S>::U / 2;
 };
 
 // bw: this warp's b window in shared memory, U rows of 128 values; a lane only
