@@ -662,12 +662,18 @@ int strip_rows(const gd_plan p, const std::vector<int> &bottoms, int l, int down
   return best;
 }
 
+// The caller's residual into the plan's, zero where there is no unknown (`codes`: the
+// class bytes of a masked level 0, else null).  The zeros are not written again by a
+// later solve on the plan, and a NaN left there would reach it: a neighbouring strip
+// multiplies such a cell by its zero diagonal inverse.
 template <typename T>
-__global__ void k_load_r(T *r, int pitch, const double *src, int spitch, int ny, int nx) {
+__global__ void k_load_r(T *r, int pitch, const double *src, int spitch, int ny, int nx,
+                         const unsigned char *codes) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= ny * nx) return;
   const int y = k / nx, x = k - y * nx;
-  r[(long long)y * pitch + x] = (T)src[(long long)y * spitch + x];
+  const long long g = (long long)y * pitch + x;
+  r[g] = (!codes || codes[g]) ? (T)src[(long long)y * spitch + x] : T(0);
 }
 
 template <typename T>
@@ -1465,8 +1471,12 @@ int run_apply_vcycle(gd_plan p, int i, const double *r, double *z, int pitch, cu
                                 cudaMemcpyHostToDevice, st));
   T *arena = reinterpret_cast<T *>(p->ws + p->o_arena);
   const int cells = I.ny * I.nx;
-  k_load_r<T><<<ceil_div(cells, 256), 256, 0, st>>>(arena + I.r_off, I.pitch, r, pitch, I.ny,
-                                                    I.nx);
+  const long long code_off = p->lv[I.level0].code_off;
+  const unsigned char *codes =
+      code_off >= 0 ? reinterpret_cast<const unsigned char *>(p->ws + p->o_codes) + code_off
+                    : nullptr;
+  k_load_r<T><<<ceil_div(cells, 256), 256, 0, st>>>(arena + I.r_off, I.pitch, r, pitch, I.ny, I.nx,
+                                                    codes);
   Runner<T>::dispatch_vcycle(p, Runner<T>::args(p), st);
   k_store_z<T><<<ceil_div(cells, 256), 256, 0, st>>>(z, pitch, arena + I.z_off, I.pitch, I.ny,
                                                      I.nx);

@@ -62,3 +62,30 @@ def test_masks_one_after_another_on_one_plan(shape, precision, zero_start):
         assert not x[~on].any(), name
         # the reported residual is the true one; 2x for the order of the sums
         assert _residual(x, f, on) <= 2e-9, name
+
+
+# strips and tiles with parts that hold no unknown, and a grid that is a bottom alone
+@pytest.mark.parametrize("shape", [(700, 1100), (301, 97), (60, 60)])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_residual_outside_the_mask_is_not_read(shape, precision):
+    """What apply_vcycle's residual holds where there is no unknown changes neither its
+    result nor a later solve on the plan."""
+    h, w = shape
+    g = torch.Generator(device="cuda")
+    g.manual_seed(h * w)
+    params = SolveParams(precision=precision, tolerance=1e-9, zero_start=True)
+    for name, on in _masks(h, w, g).items():
+        f = torch.where(on, torch.randn(shape, generator=g, dtype=torch.float64, device="cuda"),
+                        torch.zeros(shape, dtype=torch.float64, device="cuda"))
+        clean, dirty = [PoissonPlan([Instance(h, w, "masked")], params) for _ in range(2)]
+        for plan in (clean, dirty):
+            plan.set_mask(0, on.to(torch.uint8))
+        z = clean.apply_vcycle(0, f)
+        assert not z[~on].any(), name
+        for junk in (float("nan"), float("inf"), -1e300):
+            r = torch.where(on, f, torch.full_like(f, junk))
+            assert torch.equal(dirty.apply_vcycle(0, r), z), (name, junk)
+            x = [torch.empty_like(f) for _ in range(2)]
+            for plan, out in zip((clean, dirty), x):
+                assert plan.solve([f], [out])[0].converged, (name, junk)
+            assert torch.equal(x[0], x[1]), (name, junk)
