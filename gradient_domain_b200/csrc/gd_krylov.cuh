@@ -287,7 +287,12 @@ __device__ __forceinline__ double cgupdate_rows(const Place<T> &w, const unsigne
       rv.v[j] = on ? rv.v[j] - alpha * ap.v[j] : T(0);
       acc += rv.v[j] * rv.v[j];
     }
-    part += (double)acc;
+    if (w.nv < 4) {  // the columns of a width that is no multiple of four: squares in FP64
+#pragma unroll
+      for (int j = 0; j < 4; ++j) part += (double)rv.v[j] * (double)rv.v[j];
+    } else {
+      part += (double)acc;
+    }
     if (w.in) {
       const long long g = (long long)y * w.pitch + w.x0;
       st::st4(d + g, dv);

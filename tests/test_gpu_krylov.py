@@ -64,3 +64,21 @@ def test_krylov_tiles(boundary, precision):
         assert _true_residual(together[i], fs[i], boundary, ons[i]) <= 2e-8, shapes[i]
     for i in (0, 2, 5):
         assert torch.equal(solve([i])[0], together[i]), shapes[i]
+
+
+@pytest.mark.parametrize("shape", [(64, 2), (64, 3), (256, 2), (256, 3)])
+def test_last_columns_square_in_fp64(shape):
+    """The columns of a width that is no multiple of four square their residual in FP64.
+
+    A smooth f of 1e-23 has search directions far above it, so p.Ap is a normal number of
+    the iteration, but every square of r is below FP32's smallest, 1.4e-45.  Summed in FP32
+    r.r would be zero and ask for a refresh at once; in FP64 the residual stays above
+    reliable_delta and the tolerance, and the only refresh is the one that ends the solve."""
+    h, w = shape
+    y = torch.arange(h, dtype=torch.float64, device="cuda")[:, None]
+    f = 1e-23 * torch.cos(np.pi * (y + 0.5) / h).expand(h, w).contiguous()
+    params = SolveParams(tolerance=1e-4, reliable_delta=1e-8, max_iterations=2, zero_start=True)
+    plan = PoissonPlan([Instance(h, w, "neumann", True)], params)
+    for _ in range(2):  # direct launches, then the graph
+        res = plan.solve([f], [torch.empty_like(f)], scale=-1.0)[0]
+        assert res.iterations >= 1 and res.refreshes == 1, res
