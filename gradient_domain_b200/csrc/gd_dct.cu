@@ -425,29 +425,30 @@ __device__ __forceinline__ void dft(double2 (&x)[R]) {
   else if constexpr (R > 1) dft_prime<R, SIGN>(x);
 }
 
-// x[q] *= w^q (forward) or conj(w)^q (inverse), q < R, the powers from w by
-// products: four at a time from the last multiple of w^4, so that few are live.
-template <int R, int SIGN>
-__device__ __forceinline__ void twiddle(double2 (&x)[R], double2 w1) {
+// x[q] *= w^q (forward) or conj(w)^q (inverse), q < R, where power(q) gives w^q for
+// q = 1, 2, 3, 4, 8, 12, from a table or at most one product; every other power is one
+// product of two of these.  (Powers by repeated products from w alone carried up to eight
+// roundings into the smoothest modes, whose small eigenvalues magnify them: error of a
+// tone-mapping solve against 80-bit transforms, 720 x 1280 4.3e-13 then, 1.5e-13 so;
+// 1024 x 1024 2.5e-13 then, 1.8e-13 so.)
+template <int R, int SIGN, class Power>
+__device__ __forceinline__ void twiddle(double2 (&x)[R], Power power) {
   auto mul = [](double2 a, double2 t) { return SIGN < 0 ? cmul(a, t) : cmulc(a, t); };
-  if constexpr (R > 1) x[1] = mul(x[1], w1);
+  const double2 w1 = power(1);
+  x[1] = mul(x[1], w1);
   if constexpr (R > 2) {
-    const double2 w2 = cmul(w1, w1);
+    const double2 w2 = power(2);
     x[2] = mul(x[2], w2);
     if constexpr (R > 3) {
-      const double2 w3 = cmul(w2, w1);
+      const double2 w3 = power(3);
       x[3] = mul(x[3], w3);
-      if constexpr (R > 4) {
-        const double2 w4 = cmul(w2, w2);
-        double2 base = w4;
 #pragma unroll
-        for (int b = 4; b < R; b += 4) {
-          x[b] = mul(x[b], base);
-          if (b + 1 < R) x[b + 1] = mul(x[b + 1], cmul(base, w1));
-          if (b + 2 < R) x[b + 2] = mul(x[b + 2], cmul(base, w2));
-          if (b + 3 < R) x[b + 3] = mul(x[b + 3], cmul(base, w3));
-          if (b + 4 < R) base = cmul(base, w4);
-        }
+      for (int b = 4; b < R; b += 4) {
+        const double2 base = power(b);
+        x[b] = mul(x[b], base);
+        if (b + 1 < R) x[b + 1] = mul(x[b + 1], cmul(base, w1));
+        if (b + 2 < R) x[b + 2] = mul(x[b + 2], cmul(base, w2));
+        if (b + 3 < R) x[b + 3] = mul(x[b + 3], cmul(base, w3));
       }
     }
   }
@@ -511,6 +512,8 @@ struct RowPair {
   }
 };
 
+constexpr int kPowers = 4;  // rows of a pass in a power-of-two length's twiddle table
+
 // ---------------------------------------------------------------------------
 // Powers of two, 512 .. 8192: N / 16 threads, sixteen values each.
 // Passes: radix 16 while the sub-transform allows, the last of radix 2^(LOG mod 4)
@@ -524,16 +527,32 @@ struct P2 {
   static constexpr int MID = (LOG - REM) / 4 - 1;   // radix-16 passes after the first
   static constexpr size_t smem = (size_t)N * sizeof(double2);
 
-  // e^{-2 pi i k / L} of this thread's butterfly in the first pass and the middle ones
-  struct Twiddles {
-    double2 w[MID + 1];
-    __device__ __forceinline__ explicit Twiddles(const double2 *tw) {
-      const int t = threadIdx.x;
-      w[0] = tw[t];
-#pragma unroll
-      for (int s = 1; s <= MID; ++s) w[s] = tw[(t & ((TP >> (4 * s)) - 1)) << (4 * s)];
-    }
-  };
+  // The table of the twiddled passes (k_p2_table): for pass s, a row of its TP >> 4 s
+  // butterflies' e^{-2 pi i k q / L} for each of q = 1, 2, 4, 8, so that a warp reads whole
+  // lines.  Rows for q = 3 and 12 too cost more than the products (4096 x 4096: 296 and
+  // 280 us a solve) and gained no accuracy to speak of.
+  template <int S>
+  static constexpr int table_offset() {
+    int o = 0;
+    for (int s = 0; s < S; ++s) o += kPowers * (TP >> (4 * s));
+    return o;
+  }
+  static constexpr int table_len = table_offset<MID + 1>();
+  static_assert(table_len <= N, "the table takes the place of the plain twiddles");
+  template <int SIGN, int S>
+  static __device__ __forceinline__ void twiddle_pass(double2 (&x)[16], const double2 *tab) {
+    constexpr int M = TP >> (4 * S);
+    const double2 *p = tab + table_offset<S>() + (threadIdx.x & (M - 1));
+    const double2 w1 = p[0], w2 = p[M], w4 = p[2 * M], w8 = p[3 * M];
+    twiddle<16, SIGN>(x, [&](int q) {
+      return q == 1   ? w1
+             : q == 2 ? w2
+             : q == 3 ? cmul(w2, w1)
+             : q == 4 ? w4
+             : q == 8 ? w8
+                      : cmul(w8, w4);
+    });
+  }
   // first element of this thread's butterfly in middle pass s (stride TP >> 4 s)
   template <int S>
   static __device__ __forceinline__ int mid_base() {
@@ -549,15 +568,15 @@ struct P2 {
     return pos;
   }
   template <int SIGN, int S>
-  static __device__ __forceinline__ void mid_pass(double2 *z, const Twiddles &tw) {
+  static __device__ __forceinline__ void mid_pass(double2 *z, const double2 *tab) {
     constexpr int M = TP >> (4 * S);
     const int b = at(mid_base<S>());
     double2 x[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) x[j] = z[b ^ at(j * M)];
-    if constexpr (SIGN > 0) twiddle<16, 1>(x, tw.w[S]);
+    if constexpr (SIGN > 0) twiddle_pass<1, S>(x, tab);
     dft16<SIGN>(x);
-    if constexpr (SIGN < 0) twiddle<16, -1>(x, tw.w[S]);
+    if constexpr (SIGN < 0) twiddle_pass<-1, S>(x, tab);
 #pragma unroll
     for (int j = 0; j < 16; ++j) z[b ^ at(j * M)] = x[j];
     __syncthreads();
@@ -565,15 +584,15 @@ struct P2 {
   // x[j] = v[t + TP j] -> x[i] = V[t + TP i]; the shared memory may be in use by
   // this thread's own columns (places = t mod TP) on entry
   static __device__ __forceinline__ void forward(double2 (&x)[16], double2 *z,
-                                                 const Twiddles &tw) {
+                                                 const double2 *tab) {
     const int b = at(threadIdx.x);
     dft16<-1>(x);
-    twiddle<16, -1>(x, tw.w[0]);
+    twiddle_pass<-1, 0>(x, tab);
 #pragma unroll
     for (int q = 0; q < 16; ++q) z[b ^ at(q * TP)] = x[q];
     __syncthreads();
-    if constexpr (MID >= 1) mid_pass<-1, 1>(z, tw);
-    if constexpr (MID >= 2) mid_pass<-1, 2>(z, tw);
+    if constexpr (MID >= 1) mid_pass<-1, 1>(z, tab);
+    if constexpr (MID >= 2) mid_pass<-1, 2>(z, tab);
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       const int p = last_base(threadIdx.x + TP * g);
@@ -588,7 +607,7 @@ struct P2 {
   }
   // the inverse (unscaled); the shared memory is free on entry
   static __device__ __forceinline__ void inverse(double2 (&x)[16], double2 *z,
-                                                 const Twiddles &tw) {
+                                                 const double2 *tab) {
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       const int p = last_base(threadIdx.x + TP * g);
@@ -600,12 +619,12 @@ struct P2 {
       for (int j = 0; j < LR; ++j) z[at(p + j)] = y[j];
     }
     __syncthreads();
-    if constexpr (MID >= 2) mid_pass<1, 2>(z, tw);
-    if constexpr (MID >= 1) mid_pass<1, 1>(z, tw);
+    if constexpr (MID >= 2) mid_pass<1, 2>(z, tab);
+    if constexpr (MID >= 1) mid_pass<1, 1>(z, tab);
     const int b = at(threadIdx.x);
 #pragma unroll
     for (int q = 0; q < 16; ++q) x[q] = z[b ^ at(q * TP)];
-    twiddle<16, 1>(x, tw.w[0]);
+    twiddle_pass<1, 0>(x, tab);
     dft16<1>(x);
   }
 };
@@ -627,7 +646,7 @@ constexpr int kP2Ctas = P2<LOG>::TP >= 512 ? 1 : 512 / P2<LOG>::TP;
 template <int LOG>
 __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
     k_rows_p2(double2 *__restrict__ T, int hp, const double *__restrict__ bsrc, long long bpitch,
-              int h, const double2 *__restrict__ twt, const double2 *__restrict__ post) {
+              int h, const double2 *__restrict__ tab, const double2 *__restrict__ post) {
   using F = P2<LOG>;
   constexpr int N = F::N, TP = F::TP;
   extern __shared__ double2 z[];
@@ -650,9 +669,6 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
       vb[j] = make_double2(rb[m], rb[m + 1]);
     }
   }
-  const typename F::Twiddles tw(twt);
-  double2 pt = post[t];
-  pt = make_double2(0.5 * pt.x, 0.5 * pt.y);
   // the even samples are this thread's, the odd ones belong to place N - 1 - m
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
@@ -662,7 +678,7 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
   __syncthreads();
 #pragma unroll
   for (int j = 8; j < 16; ++j) x[j] = z[at(t + TP * j)];
-  F::forward(x, z, tw);
+  F::forward(x, z, tab);
 #pragma unroll
   for (int i = 0; i < 16; ++i) z[at(t + TP * i)] = x[i];
   __syncthreads();
@@ -672,10 +688,8 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     const double2 zk = x[i], zn = z[at((N - (t + TP * i)) & (N - 1))];
-    const double2 tk = cmul(pt, c32(i));  // half the DCT twiddle
-    const double2 A = make_double2(zk.x + zn.x, zk.y - zn.y);
-    const double2 B = make_double2(zk.y + zn.y, zn.x - zk.x);
-    const double xa = tk.x * A.x - tk.y * A.y, xb = tk.x * B.x - tk.y * B.y;
+    const Coef4 f = split(zk, zn, cmul(post[t], c32(i)));
+    const double xa = f.ak, xb = f.bk;
     const double got = __shfl_xor_sync(0xffffffffu, odd ? xa : xb, 1);
     const double2 v = odd ? make_double2(got, xb) : make_double2(xa, got);
     if (!odd || rp.two) dst[(long long)(TP / 2 * i) * hp] = v;
@@ -684,7 +698,7 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
 
 template <int LOG>
 __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
-    k_cols_p2(double2 *__restrict__ T, int hp, int w, const double2 *__restrict__ twt,
+    k_cols_p2(double2 *__restrict__ T, int hp, int w, const double2 *__restrict__ tab,
               const double2 *__restrict__ post, const double *__restrict__ eig,
               const double *__restrict__ eig_w) {
   using F = P2<LOG>;
@@ -695,10 +709,8 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
   double2 x[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) x[j] = col[t + TP * j];
-  const typename F::Twiddles tw(twt);
-  const double2 pt = post[t];
   const double ew_a = eig_w[c0], ew_b = c0 + 1 < w ? eig_w[c0 + 1] : 0.0;
-  F::forward(x, z, tw);
+  F::forward(x, z, tab);
   // pairs (k, N - k) with k = t + TP i, i < 8: the upper halves change hands
 #pragma unroll
   for (int i = 8; i < 16; ++i) z[at(t + TP * i)] = x[i];
@@ -714,7 +726,7 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
     } else {
       const int pn = at(N - k);
       const double en = eig[N - k];
-      const double2 tk = cmul(pt, c32(i));
+      const double2 tk = cmul(post[t], c32(i));
       Coef4 c = split(x[i], z[pn], tk);
       c.ak /= (ek + ew_a) - 4.0;
       c.bk /= (ek + ew_b) - 4.0;
@@ -726,7 +738,7 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
   }
   if (t == 0) {  // k = N / 2 is its own partner
     const double ek = eig[N / 2];
-    const double2 tk = c32(8);
+    const double2 tk = post[N / 2];
     Coef4 c = split(x[8], x[8], tk);
     c.ak /= (ek + ew_a) - 4.0;
     c.bk /= (ek + ew_b) - 4.0;
@@ -736,7 +748,7 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
 #pragma unroll
   for (int i = 8; i < 16; ++i) x[i] = z[at(t + TP * i)];
   __syncthreads();
-  F::inverse(x, z, tw);
+  F::inverse(x, z, tab);
   constexpr double inv_n = 1.0 / (double)N;
 #pragma unroll
   for (int j = 0; j < 16; ++j) col[t + TP * j] = make_double2(x[j].x * inv_n, x[j].y * inv_n);
@@ -745,7 +757,7 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
 template <int LOG>
 __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
     k_irows_p2(double *__restrict__ u, long long upitch, const double2 *__restrict__ T, int hp,
-               int h, const double2 *__restrict__ twt, const double2 *__restrict__ post) {
+               int h, const double2 *__restrict__ tab, const double2 *__restrict__ post) {
   using F = P2<LOG>;
   constexpr int N = F::N, TP = F::TP;
   extern __shared__ double2 z[];
@@ -756,8 +768,6 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
   double2 x[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) x[i] = src[(long long)(TP / 2 * i) * hp];
-  const typename F::Twiddles tw(twt);
-  const double2 pt = post[t];
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     const double got = __shfl_xor_sync(0xffffffffu, odd ? x[i].x : x[i].y, 1);
@@ -771,10 +781,10 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
     const int k = t + TP * i;
     double2 xn = z[at((N - k) & (N - 1))];
     if (k == 0) xn = make_double2(0.0, 0.0);  // X_N = 0
-    x[i] = pack_inverse(x[i].x, xn.x, x[i].y, xn.y, cmul(pt, c32(i)));
+    x[i] = pack_inverse(x[i].x, xn.x, x[i].y, xn.y, cmul(post[t], c32(i)));
   }
   __syncthreads();
-  F::inverse(x, z, tw);
+  F::inverse(x, z, tab);
   constexpr double inv_n = 1.0 / (double)N;
   // place N - 1 - m holds the odd sample of pair m
 #pragma unroll
@@ -827,7 +837,7 @@ __device__ __forceinline__ void dif_pass(double2 *z, int n, const Pass &p, const
 #pragma unroll
     for (int j = 0; j < R; ++j) x[j] = src(base + j * p.m);
     dft<R, -1>(x);
-    if (p.m > 1) twiddle<R, -1>(x, tw[k * p.step]);
+    if (p.m > 1) twiddle<R, -1>(x, [&](int q) { return tw[q * k * p.step]; });
 #pragma unroll
     for (int j = 0; j < R; ++j) z[at(base + j * p.m)] = x[j];
   }
@@ -843,7 +853,7 @@ __device__ __forceinline__ void dit_pass(double2 *z, int n, const Pass &p, const
     double2 x[R];
 #pragma unroll
     for (int j = 0; j < R; ++j) x[j] = z[at(base + j * p.m)];
-    if (p.m > 1) twiddle<R, 1>(x, tw[k * p.step]);
+    if (p.m > 1) twiddle<R, 1>(x, [&](int q) { return tw[q * k * p.step]; });
     dft<R, 1>(x);
 #pragma unroll
     for (int j = 0; j < R; ++j) dst(base + j * p.m, x[j]);
@@ -1095,7 +1105,7 @@ __global__ void k_dct_tables(double2 *tw, double2 *post, double *eig, unsigned s
   if (k >= n) return;
   double s, c;
   sincospi(2.0 * (double)k / (double)n, &s, &c);
-  tw[k] = make_double2(c, -s);
+  if (tw) tw[k] = make_double2(c, -s);
   sincospi((double)k / (2.0 * (double)n), &s, &c);
   post[k] = make_double2(c, -s);
   eig[k] = 2.0 * cos(M_PI * (double)k / (double)n);
@@ -1105,6 +1115,22 @@ __global__ void k_dct_tables(double2 *tw, double2 *post, double *eig, unsigned s
     f /= rad.p[q].r;
   }
   rev[k] = (unsigned short)pos;
+}
+
+// The twiddle table of a power-of-two length (P2::table_offset), `len` entries in all.
+__global__ void k_p2_table(double2 *tab, int n, int len) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= len) return;
+  int row = n / 16, step = 1, at = g;  // butterflies of a pass, step of its twiddles
+  while (at >= kPowers * row) {
+    at -= kPowers * row;
+    row >>= 4;
+    step <<= 4;
+  }
+  const int j = at / row, k = at - j * row;
+  double s, c;
+  sincospi(2.0 * (double)((k * step) << j) / (double)n, &s, &c);
+  tab[g] = make_double2(c, -s);
 }
 
 inline size_t a256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -1214,8 +1240,16 @@ extern "C" int gd_dct_plan_bind(gd_dct_plan p, void *ws, size_t bytes, cudaStrea
                                                      "256-byte aligned");
   p->ws = static_cast<char *>(ws);
   const AxisTables tw = tables(p, p->o_tab_w, p->w), th = tables(p, p->o_tab_h, p->h);
-  dct::k_dct_tables<<<(p->w + 255) / 256, 256, 0, st>>>(tw.tw, tw.post, tw.eig, tw.rev, p->rw);
-  dct::k_dct_tables<<<(p->h + 255) / 256, 256, 0, st>>>(th.tw, th.post, th.eig, th.rev, p->rh);
+  auto fill = [&](const AxisTables &t, const dct::Radices &r) {
+    int len = 0;  // entries of a power-of-two kernel's twiddle table, in the place of tw
+    dct::with_kernels(r, [&](auto log) { len = dct::P2<decltype(log)::value>::table_len; },
+                      [](auto) {});
+    dct::k_dct_tables<<<(r.n + 255) / 256, 256, 0, st>>>(len ? nullptr : t.tw, t.post, t.eig,
+                                                         t.rev, r);
+    if (len) dct::k_p2_table<<<(len + 255) / 256, 256, 0, st>>>(t.tw, r.n, len);
+  };
+  fill(tw, p->rw);
+  fill(th, p->rh);
   GD_CHECK_LAUNCH();
   // the tables must be complete before a solve on any stream (set-up, once per plan)
   GD_CHECK_CUDA(cudaStreamSynchronize(st));

@@ -3,6 +3,7 @@
 import numpy as np
 import pytest
 import torch
+from scipy import fft
 
 from gradient_domain_b200.solvers import DctPlan
 from oracle import solvers
@@ -36,3 +37,29 @@ def test_dct_solve_matches_the_oracle(shape):
     plan.solve(view, view)
     assert torch.equal(view, u)
     assert not buf[:, 0].any() and not buf[:, w + 1:].any()
+
+
+@pytest.mark.parametrize("shape", [(720, 1280), (1000, 1000), (375, 1125), (1024, 1024)])
+def test_transform_error_in_the_smoothest_modes(shape):
+    """A right-hand side whose solution is white noise is strongest in its highest modes, and
+    the transform's rounding of those is what its smoothest modes carry, divided by their
+    small eigenvalues.  That error, times the eigenvalue, against 80-bit transforms with the
+    solver's own eigenvalues: at most six passes (three a direction) of six roundings (four
+    additions, a product by a twiddle of the table) and four of the DCT's own twiddles, each
+    of rms eps / sqrt(12) - 1.27 is measured, 1.9 to 2.2 with twiddles by repeated products."""
+    h, w = shape
+    wide = np.longdouble
+    eig = ((2 * np.cos(np.pi * np.arange(h) / h))[:, None]
+           + (2 * np.cos(np.pi * np.arange(w) / w))[None] - 4).astype(wide)
+    g = np.random.default_rng(h + w).standard_normal(shape).astype(wide)
+    g[0, 0] = 0
+    b = fft.idctn(g * eig, type=2, norm="ortho").astype(np.float64)
+    ref = fft.dctn(b.astype(wide), type=2, norm="ortho")
+    ref[0, 0] = 0
+    bd = torch.as_tensor(b).cuda()
+    u = DctPlan(h, w).solve(bd, torch.empty_like(bd)).cpu().numpy()
+    err = fft.dctn(u.astype(wide), type=2, norm="ortho") * eig - ref
+    low = err[:h // 16, :w // 16].ravel()[1:].astype(np.float64)
+    eps = np.finfo(np.float64).eps
+    bound = eps / np.sqrt(12) * np.sqrt(6 * 6 + 4)
+    assert np.sqrt(np.mean(low ** 2)) <= bound * np.sqrt(np.mean(b ** 2))
