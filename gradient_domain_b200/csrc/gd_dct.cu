@@ -32,7 +32,7 @@
 // natural out).  What bounds them is FP64 arithmetic and shared-memory
 // bandwidth, so passes are few and large (radices up to 16), the first forward
 // pass takes its operands straight from global memory, and the last inverse one
-// writes its results there.  Lengths 512 .. 8192 that are powers of two run
+// writes its results there.  Lengths 64 .. 8192 that are powers of two run
 // kernels whose every index is known at compile time, one radix-16 butterfly per
 // thread and pass, with the values in registers from the loads to the
 // coefficients: 3 passes and 2 exchanges for 4096 where radix 8 with staging
@@ -500,12 +500,12 @@ __device__ __forceinline__ double2 pack_inverse(double xa, double xan, double xb
   return make_double2(wa.x - wb.y, wa.y + wb.x);
 }
 
-// The two rows of a row CTA: places 2p and 2p + 1 of the reordering along y.
+// The two rows of a pair: places 2p and 2p + 1 of the reordering along y.
 struct RowPair {
   int p0, ra, rb;
   bool two;
-  __device__ __forceinline__ explicit RowPair(int h) {
-    p0 = 2 * blockIdx.x;
+  __device__ __forceinline__ RowPair(int pair, int h) {
+    p0 = 2 * pair;
     two = p0 + 1 < h;
     ra = mak_sample(p0, h);
     rb = two ? mak_sample(p0 + 1, h) : ra;
@@ -515,36 +515,52 @@ struct RowPair {
 constexpr int kPowers = 4;  // rows of a pass in a power-of-two length's twiddle table
 
 // ---------------------------------------------------------------------------
-// Powers of two, 512 .. 8192: N / 16 threads, sixteen values each.
-// Passes: radix 16 while the sub-transform allows, the last of radix 2^(LOG mod 4)
-// (or 16).  After the forward passes thread t holds the frequencies t + TP i.
+// Powers of two, 64 .. 8192: N / 16 threads with sixteen values each, below 512 N / 8 with
+// eight, as many pairs of lines in a CTA as a warp holds.  (A launch of few short lines is as
+// long as one thread's chain: 64 x 64 and 256 x 256 took 25.2 and 27.5 us a solve by the
+// run-time passes, 17.0 and 17.4 so; 8192 x 64 56 and 38 us.)
+// Passes: radix V while the sub-transform allows, the last of radix 2^(LOG mod LV)
+// (or V).  After the forward passes thread t of a pair holds the frequencies t + TP i.
 template <int LOG>
 struct P2 {
-  static constexpr int N = 1 << LOG, TP = N / 16;
-  static constexpr int REM = LOG % 4 ? LOG % 4 : 4;
+  static constexpr int LV = LOG < 9 ? 3 : 4, V = 1 << LV;
+  static constexpr int N = 1 << LOG, TP = N / V;
+  static constexpr int PB = TP < 32 ? 32 / TP : 1;  // pairs of lines in a CTA
+  static constexpr int REM = LOG % LV ? LOG % LV : LV;
   static constexpr int LR = 1 << REM;               // radix of the last pass
-  static constexpr int G = 16 / LR;                 // its butterflies per thread
-  static constexpr int MID = (LOG - REM) / 4 - 1;   // radix-16 passes after the first
-  static constexpr size_t smem = (size_t)N * sizeof(double2);
+  static constexpr int G = V / LR;                  // its butterflies per thread
+  static constexpr int MID = (LOG - REM) / LV - 1;  // radix-V passes after the first
+  static constexpr int threads = TP * PB;
+  static constexpr size_t smem = (size_t)PB * N * sizeof(double2);
 
-  // The table of the twiddled passes (k_p2_table): for pass s, a row of its TP >> 4 s
+  // this thread's number in its pair of lines, the pair's number and its shared memory
+  static __device__ __forceinline__ int lane() { return threadIdx.x & (TP - 1); }
+  static __device__ __forceinline__ int pair() { return blockIdx.x * PB + threadIdx.x / TP; }
+  static __device__ __forceinline__ double2 *line(double2 *smem) {
+    return smem + threadIdx.x / TP * N;
+  }
+  static inline unsigned ctas(int pairs) { return (unsigned)((pairs + PB - 1) / PB); }
+
+  // The table of the twiddled passes (k_p2_table): for pass s, a row of its TP >> LV s
   // butterflies' e^{-2 pi i k q / L} for each of q = 1, 2, 4, 8, so that a warp reads whole
   // lines.  Rows for q = 3 and 12 too cost more than the products (4096 x 4096: 296 and
   // 280 us a solve) and gained no accuracy to speak of.
   template <int S>
   static constexpr int table_offset() {
     int o = 0;
-    for (int s = 0; s < S; ++s) o += kPowers * (TP >> (4 * s));
+    for (int s = 0; s < S; ++s) o += kPowers * (TP >> (LV * s));
     return o;
   }
   static constexpr int table_len = table_offset<MID + 1>();
   static_assert(table_len <= N, "the table takes the place of the plain twiddles");
   template <int SIGN, int S>
-  static __device__ __forceinline__ void twiddle_pass(double2 (&x)[16], const double2 *tab) {
-    constexpr int M = TP >> (4 * S);
-    const double2 *p = tab + table_offset<S>() + (threadIdx.x & (M - 1));
-    const double2 w1 = p[0], w2 = p[M], w4 = p[2 * M], w8 = p[3 * M];
-    twiddle<16, SIGN>(x, [&](int q) {
+  static __device__ __forceinline__ void twiddle_pass(double2 (&x)[V], const double2 *tab) {
+    constexpr int M = TP >> (LV * S);
+    const double2 *p = tab + table_offset<S>() + (lane() & (M - 1));
+    const double2 w1 = p[0], w2 = p[M], w4 = p[2 * M];
+    double2 w8 = w4;
+    if constexpr (V == 16) w8 = p[3 * M];
+    twiddle<V, SIGN>(x, [&](int q) {
       return q == 1   ? w1
              : q == 2 ? w2
              : q == 3 ? cmul(w2, w1)
@@ -556,46 +572,46 @@ struct P2 {
   // first element of this thread's butterfly in middle pass s (stride TP >> 4 s)
   template <int S>
   static __device__ __forceinline__ int mid_base() {
-    constexpr int M = TP >> (4 * S);
-    const int t = threadIdx.x;
-    return ((t & ~(M - 1)) << 4) | (t & (M - 1));
+    constexpr int M = TP >> (LV * S);
+    const int t = lane();
+    return ((t & ~(M - 1)) << LV) | (t & (M - 1));
   }
   // place of frequency f (< N / LR) in the digit-reversed order
   static __device__ __forceinline__ int last_base(int f) {
     int pos = 0;
 #pragma unroll
-    for (int s = 0; s <= MID; ++s) pos |= ((f >> (4 * s)) & 15) << (LOG - 4 * s - 4);
+    for (int s = 0; s <= MID; ++s) pos |= ((f >> (LV * s)) & (V - 1)) << (LOG - LV * s - LV);
     return pos;
   }
   template <int SIGN, int S>
   static __device__ __forceinline__ void mid_pass(double2 *z, const double2 *tab) {
-    constexpr int M = TP >> (4 * S);
+    constexpr int M = TP >> (LV * S);
     const int b = at(mid_base<S>());
-    double2 x[16];
+    double2 x[V];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) x[j] = z[b ^ at(j * M)];
+    for (int j = 0; j < V; ++j) x[j] = z[b ^ at(j * M)];
     if constexpr (SIGN > 0) twiddle_pass<1, S>(x, tab);
-    dft16<SIGN>(x);
+    dft<V, SIGN>(x);
     if constexpr (SIGN < 0) twiddle_pass<-1, S>(x, tab);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) z[b ^ at(j * M)] = x[j];
+    for (int j = 0; j < V; ++j) z[b ^ at(j * M)] = x[j];
     __syncthreads();
   }
   // x[j] = v[t + TP j] -> x[i] = V[t + TP i]; the shared memory may be in use by
   // this thread's own columns (places = t mod TP) on entry
-  static __device__ __forceinline__ void forward(double2 (&x)[16], double2 *z,
+  static __device__ __forceinline__ void forward(double2 (&x)[V], double2 *z,
                                                  const double2 *tab) {
-    const int b = at(threadIdx.x);
-    dft16<-1>(x);
+    const int b = at(lane());
+    dft<V, -1>(x);
     twiddle_pass<-1, 0>(x, tab);
 #pragma unroll
-    for (int q = 0; q < 16; ++q) z[b ^ at(q * TP)] = x[q];
+    for (int q = 0; q < V; ++q) z[b ^ at(q * TP)] = x[q];
     __syncthreads();
     if constexpr (MID >= 1) mid_pass<-1, 1>(z, tab);
     if constexpr (MID >= 2) mid_pass<-1, 2>(z, tab);
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-      const int p = last_base(threadIdx.x + TP * g);
+      const int p = last_base(lane() + TP * g);
       double2 y[LR];
 #pragma unroll
       for (int j = 0; j < LR; ++j) y[j] = z[at(p + j)];
@@ -606,11 +622,11 @@ struct P2 {
     __syncthreads();
   }
   // the inverse (unscaled); the shared memory is free on entry
-  static __device__ __forceinline__ void inverse(double2 (&x)[16], double2 *z,
+  static __device__ __forceinline__ void inverse(double2 (&x)[V], double2 *z,
                                                  const double2 *tab) {
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-      const int p = last_base(threadIdx.x + TP * g);
+      const int p = last_base(lane() + TP * g);
       double2 y[LR];
 #pragma unroll
       for (int q = 0; q < LR; ++q) y[q] = x[g + G * q];
@@ -621,15 +637,16 @@ struct P2 {
     __syncthreads();
     if constexpr (MID >= 2) mid_pass<1, 2>(z, tab);
     if constexpr (MID >= 1) mid_pass<1, 1>(z, tab);
-    const int b = at(threadIdx.x);
+    const int b = at(lane());
 #pragma unroll
-    for (int q = 0; q < 16; ++q) x[q] = z[b ^ at(q * TP)];
+    for (int q = 0; q < V; ++q) x[q] = z[b ^ at(q * TP)];
     twiddle_pass<1, 0>(x, tab);
-    dft16<1>(x);
+    dft<V, 1>(x);
   }
 };
 
-// e^{-i pi i / 32}, i = 0 .. 15: the DCT twiddle of frequency t + TP i is that of t times it.
+// e^{-i pi i / 32}, i = 0 .. 15: the DCT twiddle of frequency t + TP i is that of t times
+// this of 16 i / V.
 __device__ __forceinline__ double2 c32(int i) {
   constexpr double c[17] = {1.0, 0.9951847266721969, 0.9807852804032304, 0.9569403357322088,
                             0.9238795325112867, 0.881921264348355, 0.8314696123025452,
@@ -641,29 +658,31 @@ __device__ __forceinline__ double2 c32(int i) {
 
 // CTAs per SM for 128 registers a thread.
 template <int LOG>
-constexpr int kP2Ctas = P2<LOG>::TP >= 512 ? 1 : 512 / P2<LOG>::TP;
+constexpr int kP2Ctas = P2<LOG>::threads >= 512 ? 1 : 512 / P2<LOG>::threads;
 
 template <int LOG>
-__global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
+__global__ void __launch_bounds__(P2<LOG>::threads, kP2Ctas<LOG>)
     k_rows_p2(double2 *__restrict__ T, int hp, const double *__restrict__ bsrc, long long bpitch,
               int h, const double2 *__restrict__ tab, const double2 *__restrict__ post) {
   using F = P2<LOG>;
-  constexpr int N = F::N, TP = F::TP;
-  extern __shared__ double2 z[];
-  const int t = threadIdx.x;
-  const RowPair rp(h);
+  constexpr int N = F::N, TP = F::TP, V = F::V;
+  extern __shared__ double2 smem[];
+  double2 *const z = F::line(smem);
+  const int t = F::lane(), pairs = (h + 1) / 2;
+  const bool live = F::PB == 1 || F::pair() < pairs;  // else the last pair again, not stored
+  const RowPair rp(live ? F::pair() : pairs - 1, h);
   const double *ra = bsrc + rp.ra * bpitch, *rb = bsrc + rp.rb * bpitch;
-  double2 x[16];
-  double2 va[8], vb[8];
+  double2 x[V];
+  double2 va[V / 2], vb[V / 2];
   if (((reinterpret_cast<uintptr_t>(ra) | reinterpret_cast<uintptr_t>(rb)) & 15) == 0) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < V / 2; ++j) {
       va[j] = reinterpret_cast<const double2 *>(ra)[t + TP * j];
       vb[j] = reinterpret_cast<const double2 *>(rb)[t + TP * j];
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < V / 2; ++j) {
       const int m = 2 * (t + TP * j);
       va[j] = make_double2(ra[m], ra[m + 1]);
       vb[j] = make_double2(rb[m], rb[m + 1]);
@@ -671,52 +690,55 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
   }
   // the even samples are this thread's, the odd ones belong to place N - 1 - m
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
+  for (int j = 0; j < V / 2; ++j) {
     x[j] = make_double2(va[j].x, rp.two ? vb[j].x : 0.0);
     z[at(N - 1 - (t + TP * j))] = make_double2(va[j].y, rp.two ? vb[j].y : 0.0);
   }
   __syncthreads();
 #pragma unroll
-  for (int j = 8; j < 16; ++j) x[j] = z[at(t + TP * j)];
+  for (int j = V / 2; j < V; ++j) x[j] = z[at(t + TP * j)];
   F::forward(x, z, tab);
 #pragma unroll
-  for (int i = 0; i < 16; ++i) z[at(t + TP * i)] = x[i];
+  for (int i = 0; i < V; ++i) z[at(t + TP * i)] = x[i];
   __syncthreads();
   // lanes 2l and 2l + 1 hold one column pair: the even one takes row a, the odd one row b
   const int odd = t & 1;
   double2 *dst = T + (long long)(t >> 1) * hp + rp.p0 + odd;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
+  for (int i = 0; i < V; ++i) {
     const double2 zk = x[i], zn = z[at((N - (t + TP * i)) & (N - 1))];
-    const Coef4 f = split(zk, zn, cmul(post[t], c32(i)));
+    const Coef4 f = split(zk, zn, cmul(post[t], c32(16 / V * i)));
     const double xa = f.ak, xb = f.bk;
     const double got = __shfl_xor_sync(0xffffffffu, odd ? xa : xb, 1);
     const double2 v = odd ? make_double2(got, xb) : make_double2(xa, got);
-    if (!odd || rp.two) dst[(long long)(TP / 2 * i) * hp] = v;
+    if (live && (!odd || rp.two)) dst[(long long)(TP / 2 * i) * hp] = v;
   }
 }
 
 template <int LOG>
-__global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
+__global__ void __launch_bounds__(P2<LOG>::threads, kP2Ctas<LOG>)
     k_cols_p2(double2 *__restrict__ T, int hp, int w, const double2 *__restrict__ tab,
               const double2 *__restrict__ post, const double *__restrict__ eig,
               const double *__restrict__ eig_w) {
   using F = P2<LOG>;
-  constexpr int N = F::N, TP = F::TP;
-  extern __shared__ double2 z[];
-  const int t = threadIdx.x, c0 = 2 * blockIdx.x;
-  double2 *col = T + (long long)blockIdx.x * hp;
-  double2 x[16];
+  constexpr int N = F::N, TP = F::TP, V = F::V;
+  extern __shared__ double2 smem[];
+  double2 *const z = F::line(smem);
+  const int t = F::lane(), pairs = (w + 1) / 2;
+  const bool live = F::PB == 1 || F::pair() < pairs;  // else zeros, not stored
+  const int pair = live ? F::pair() : 0, c0 = 2 * pair;
+  double2 *col = T + (long long)pair * hp;
+  double2 x[V];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) x[j] = col[t + TP * j];
+  for (int j = 0; j < V; ++j) x[j] = live ? col[t + TP * j] : make_double2(0.0, 0.0);
   const double ew_a = eig_w[c0], ew_b = c0 + 1 < w ? eig_w[c0 + 1] : 0.0;
   F::forward(x, z, tab);
-  // pairs (k, N - k) with k = t + TP i, i < 8: the upper halves change hands
+  // pairs (k, N - k) with k = t + TP i, i < V / 2: the upper halves change hands
 #pragma unroll
-  for (int i = 8; i < 16; ++i) z[at(t + TP * i)] = x[i];
+  for (int i = V / 2; i < V; ++i) z[at(t + TP * i)] = x[i];
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < V / 2; ++i) {
     const int k = t + TP * i;
     const double ek = eig[k];
     if (k == 0) {
@@ -726,7 +748,7 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
     } else {
       const int pn = at(N - k);
       const double en = eig[N - k];
-      const double2 tk = cmul(post[t], c32(i));
+      const double2 tk = cmul(post[t], c32(16 / V * i));
       Coef4 c = split(x[i], z[pn], tk);
       c.ak /= (ek + ew_a) - 4.0;
       c.bk /= (ek + ew_b) - 4.0;
@@ -739,37 +761,40 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
   if (t == 0) {  // k = N / 2 is its own partner
     const double ek = eig[N / 2];
     const double2 tk = post[N / 2];
-    Coef4 c = split(x[8], x[8], tk);
+    Coef4 c = split(x[V / 2], x[V / 2], tk);
     c.ak /= (ek + ew_a) - 4.0;
     c.bk /= (ek + ew_b) - 4.0;
     z[at(N / 2)] = pack_inverse(c.ak, c.ak, c.bk, c.bk, tk);
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 8; i < 16; ++i) x[i] = z[at(t + TP * i)];
+  for (int i = V / 2; i < V; ++i) x[i] = z[at(t + TP * i)];
   __syncthreads();
   F::inverse(x, z, tab);
   constexpr double inv_n = 1.0 / (double)N;
 #pragma unroll
-  for (int j = 0; j < 16; ++j) col[t + TP * j] = make_double2(x[j].x * inv_n, x[j].y * inv_n);
+  for (int j = 0; j < V; ++j)
+    if (live) col[t + TP * j] = make_double2(x[j].x * inv_n, x[j].y * inv_n);
 }
 
 template <int LOG>
-__global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
+__global__ void __launch_bounds__(P2<LOG>::threads, kP2Ctas<LOG>)
     k_irows_p2(double *__restrict__ u, long long upitch, const double2 *__restrict__ T, int hp,
                int h, const double2 *__restrict__ tab, const double2 *__restrict__ post) {
   using F = P2<LOG>;
-  constexpr int N = F::N, TP = F::TP;
-  extern __shared__ double2 z[];
-  const int t = threadIdx.x, odd = t & 1;
-  const RowPair rp(h);
+  constexpr int N = F::N, TP = F::TP, V = F::V;
+  extern __shared__ double2 smem[];
+  double2 *const z = F::line(smem);
+  const int t = F::lane(), odd = t & 1, pairs = (h + 1) / 2;
+  const bool live = F::PB == 1 || F::pair() < pairs;  // else the last pair again, not stored
+  const RowPair rp(live ? F::pair() : pairs - 1, h);
   // the even lane of a column pair loads row a, the odd one row b
   const double2 *src = T + (long long)(t >> 1) * hp + rp.p0 + (rp.two ? odd : 0);
-  double2 x[16];
+  double2 x[V];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) x[i] = src[(long long)(TP / 2 * i) * hp];
+  for (int i = 0; i < V; ++i) x[i] = src[(long long)(TP / 2 * i) * hp];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
+  for (int i = 0; i < V; ++i) {
     const double got = __shfl_xor_sync(0xffffffffu, odd ? x[i].x : x[i].y, 1);
     x[i] = odd ? make_double2(got, x[i].y) : make_double2(x[i].x, got);  // (X_a[k], X_b[k])
     if (!rp.two) x[i].y = 0.0;
@@ -777,23 +802,24 @@ __global__ void __launch_bounds__(P2<LOG>::TP, kP2Ctas<LOG>)
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
+  for (int i = 0; i < V; ++i) {
     const int k = t + TP * i;
     double2 xn = z[at((N - k) & (N - 1))];
     if (k == 0) xn = make_double2(0.0, 0.0);  // X_N = 0
-    x[i] = pack_inverse(x[i].x, xn.x, x[i].y, xn.y, cmul(post[t], c32(i)));
+    x[i] = pack_inverse(x[i].x, xn.x, x[i].y, xn.y, cmul(post[t], c32(16 / V * i)));
   }
   __syncthreads();
   F::inverse(x, z, tab);
   constexpr double inv_n = 1.0 / (double)N;
   // place N - 1 - m holds the odd sample of pair m
 #pragma unroll
-  for (int j = 8; j < 16; ++j) z[at(t + TP * j)] = x[j];
+  for (int j = V / 2; j < V; ++j) z[at(t + TP * j)] = x[j];
   __syncthreads();
+  if (!live) return;
   double *ua = u + rp.ra * upitch, *ub = u + rp.rb * upitch;
   const bool vec = ((reinterpret_cast<uintptr_t>(ua) | reinterpret_cast<uintptr_t>(ub)) & 15) == 0;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
+  for (int j = 0; j < V / 2; ++j) {
     const int m = t + TP * j;
     const double2 o = z[at(N - 1 - m)];
     const double2 a = make_double2(x[j].x * inv_n, o.x * inv_n);
@@ -1002,7 +1028,7 @@ __global__ void __launch_bounds__(kThreads, PRIME ? 1 : 2)
                int h, Axis ax) {
   extern __shared__ double2 z[];
   const int n = ax.rad.n;
-  const RowPair rp(h);
+  const RowPair rp(blockIdx.x, h);
   const double *ra = b + rp.ra * bpitch, *rb = b + rp.rb * bpitch;
   forward_fft<PRIME>(z, ax, [&](int i) {
     const int j = mak_sample(i, n);
@@ -1070,7 +1096,7 @@ __global__ void __launch_bounds__(kThreads, PRIME ? 1 : 2)
                 int h, Axis ax) {
   extern __shared__ double2 z[];
   const int n = ax.rad.n;
-  const RowPair rp(h);
+  const RowPair rp(blockIdx.x, h);
   const double *Td = reinterpret_cast<const double *>(T);
   auto coef = [&](int k) {  // (X_a[k], X_b[k])
     const double *p = Td + ((long long)(k >> 1) * hp + rp.p0) * 2 + (k & 1);
@@ -1118,14 +1144,14 @@ __global__ void k_dct_tables(double2 *tw, double2 *post, double *eig, unsigned s
 }
 
 // The twiddle table of a power-of-two length (P2::table_offset), `len` entries in all.
-__global__ void k_p2_table(double2 *tab, int n, int len) {
+__global__ void k_p2_table(double2 *tab, int n, int lv, int len) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= len) return;
-  int row = n / 16, step = 1, at = g;  // butterflies of a pass, step of its twiddles
+  int row = n >> lv, step = 1, at = g;  // butterflies of a pass, step of its twiddles
   while (at >= kPowers * row) {
     at -= kPowers * row;
-    row >>= 4;
-    step <<= 4;
+    row >>= lv;
+    step <<= lv;
   }
   const int j = at / row, k = at - j * row;
   double s, c;
@@ -1141,10 +1167,14 @@ constexpr size_t kMaxSmemBytes = (size_t)kMaxLen * sizeof(double2);
 template <int V>
 using Int = std::integral_constant<int, V>;
 
-// Call p2(Int<log2 n>{}) for the power-of-two kernels' lengths, gen(PRIME) otherwise.
+// Call p2(Int<log2 n>{}) for the power-of-two kernels' lengths, gen(PRIME) otherwise
+// (16 and 32, which are one or two passes, gain nothing from a kernel of their own).
 template <class P2Fn, class GenFn>
 void with_kernels(const Radices &r, P2Fn &&p2, GenFn &&gen) {
   switch (r.n) {
+    case 64: p2(Int<6>{}); return;
+    case 128: p2(Int<7>{}); return;
+    case 256: p2(Int<8>{}); return;
     case 512: p2(Int<9>{}); return;
     case 1024: p2(Int<10>{}); return;
     case 2048: p2(Int<11>{}); return;
@@ -1241,12 +1271,17 @@ extern "C" int gd_dct_plan_bind(gd_dct_plan p, void *ws, size_t bytes, cudaStrea
   p->ws = static_cast<char *>(ws);
   const AxisTables tw = tables(p, p->o_tab_w, p->w), th = tables(p, p->o_tab_h, p->h);
   auto fill = [&](const AxisTables &t, const dct::Radices &r) {
-    int len = 0;  // entries of a power-of-two kernel's twiddle table, in the place of tw
-    dct::with_kernels(r, [&](auto log) { len = dct::P2<decltype(log)::value>::table_len; },
-                      [](auto) {});
+    int len = 0, lv = 0;  // entries of a power-of-two kernel's twiddle table, in the place of tw
+    dct::with_kernels(
+        r,
+        [&](auto log) {
+          len = dct::P2<decltype(log)::value>::table_len;
+          lv = dct::P2<decltype(log)::value>::LV;
+        },
+        [](auto) {});
     dct::k_dct_tables<<<(r.n + 255) / 256, 256, 0, st>>>(len ? nullptr : t.tw, t.post, t.eig,
                                                          t.rev, r);
-    if (len) dct::k_p2_table<<<(len + 255) / 256, 256, 0, st>>>(t.tw, r.n, len);
+    if (len) dct::k_p2_table<<<(len + 255) / 256, 256, 0, st>>>(t.tw, r.n, lv, len);
   };
   fill(tw, p->rw);
   fill(th, p->rh);
@@ -1287,14 +1322,14 @@ extern "C" int gd_dct_solve_neumann(gd_dct_plan p, const double *b_in, double *u
   const int h = p->h, w = p->w, hp = p->hp;
   double2 *T = reinterpret_cast<double2 *>(p->ws + p->o_t);
   const dct::Axis ax = axis(p, true), ay = axis(p, false);
-  const unsigned rows = (unsigned)(h + 1) / 2, cols = (unsigned)(w + 1) / 2;
+  const int rows = (h + 1) / 2, cols = (w + 1) / 2;
   const int tw = dct::gen_threads(p->rw), th = dct::gen_threads(p->rh);
   dct::with_kernels(
       p->rw,
       [&](auto log) {
         using F = dct::P2<decltype(log)::value>;
-        dct::k_rows_p2<decltype(log)::value><<<rows, F::TP, F::smem, st>>>(T, hp, b_in, pitch, h,
-                                                                           ax.tw, ax.post);
+        dct::k_rows_p2<decltype(log)::value><<<F::ctas(rows), F::threads, F::smem, st>>>(
+            T, hp, b_in, pitch, h, ax.tw, ax.post);
       },
       [&](auto prime) {
         dct::k_rows_gen<decltype(prime)::value><<<rows, tw, dct::smem_bytes(w), st>>>(
@@ -1304,7 +1339,7 @@ extern "C" int gd_dct_solve_neumann(gd_dct_plan p, const double *b_in, double *u
       p->rh,
       [&](auto log) {
         using F = dct::P2<decltype(log)::value>;
-        dct::k_cols_p2<decltype(log)::value><<<cols, F::TP, F::smem, st>>>(
+        dct::k_cols_p2<decltype(log)::value><<<F::ctas(cols), F::threads, F::smem, st>>>(
             T, hp, w, ay.tw, ay.post, ay.eig, ax.eig);
       },
       [&](auto prime) {
@@ -1315,8 +1350,8 @@ extern "C" int gd_dct_solve_neumann(gd_dct_plan p, const double *b_in, double *u
       p->rw,
       [&](auto log) {
         using F = dct::P2<decltype(log)::value>;
-        dct::k_irows_p2<decltype(log)::value><<<rows, F::TP, F::smem, st>>>(u, pitch, T, hp, h,
-                                                                            ax.tw, ax.post);
+        dct::k_irows_p2<decltype(log)::value><<<F::ctas(rows), F::threads, F::smem, st>>>(
+            u, pitch, T, hp, h, ax.tw, ax.post);
       },
       [&](auto prime) {
         dct::k_irows_gen<decltype(prime)::value><<<rows, tw, dct::smem_bytes(w), st>>>(

@@ -12,9 +12,9 @@ pytestmark = pytest.mark.gpu
 
 # every in-register radix as a length of its own, two and three passes, a prime
 # above 13 alone and next to other factors, and both directions of the
-# power-of-two kernels (512 .. 8192) beside each kind of the other axis
+# power-of-two kernels (64 .. 8192) beside each kind of the other axis
 SHAPES = [(2, 3), (4, 5), (6, 7), (8, 9), (10, 11), (12, 13), (14, 15), (16, 64), (17, 256),
-          (90, 143), (19 * 4, 23 * 17), (1080, 480), (512, 1024), (1024, 513), (2048, 6),
+          (64, 128), (256, 64), (33, 128), (128, 70), (90, 143), (19 * 4, 23 * 17), (1080, 480), (512, 1024), (1024, 513), (2048, 6),
           (7, 2048), (4096, 5), (3, 4096), (8192, 3), (2, 8192)]
 
 
@@ -63,3 +63,33 @@ def test_transform_error_in_the_smoothest_modes(shape):
     eps = np.finfo(np.float64).eps
     bound = eps / np.sqrt(12) * np.sqrt(6 * 6 + 4)
     assert np.sqrt(np.mean(low ** 2)) <= bound * np.sqrt(np.mean(b ** 2))
+
+
+def _device_us(run, passes=20, rounds=10):
+    """Shortest device time of one of `passes` back-to-back calls, in microseconds."""
+    run()
+    best = np.inf
+    for _ in range(rounds):
+        start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda._sleep(2_000_000)  # the calls are queued before the device reaches them
+        start.record()
+        for _ in range(passes):
+            run()
+        stop.record()
+        stop.synchronize()
+        best = min(best, start.elapsed_time(stop) * 1e3 / passes)
+    return best
+
+
+def test_small_powers_of_two_are_not_slower_than_larger_ones():
+    """Launches of few short lines are as long as one thread's chain: a side of 64 to 256
+    must not take longer than one of 512 (25 to 28 us against 25 by the run-time passes)."""
+    def solve_us(n):
+        plan = DctPlan(n, n)
+        b = torch.randn((n, n), dtype=torch.float64, device="cuda")
+        u = torch.empty_like(b)
+        return _device_us(lambda: plan.solve(b, u))
+
+    larger = solve_us(512)
+    for n in (64, 128, 256):
+        assert solve_us(n) <= 0.95 * larger, n
