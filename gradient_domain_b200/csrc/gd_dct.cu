@@ -43,7 +43,6 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <map>
 #include <type_traits>
 
 #include "gd_internal.cuh"
@@ -94,44 +93,56 @@ inline double pass_cost(int r) {
 // Composite radices up to `cap`.
 inline bool usable(int r, int cap) { return r <= cap || r == 5 || r == 7 || r == 11 || r == 13; }
 
-// Cost and first radix of the cheapest factorisation of n, primes above 13 on their own;
-// `known` holds the divisors of the length that have been looked at.
-struct Cheapest {
-  double cost;
-  int first;
-};
-inline Cheapest cheapest(int n, int cap, std::map<int, Cheapest> &known) {
-  if (n == 1) return Cheapest{0.0, 1};
-  const auto it = known.find(n);
-  if (it != known.end()) return it->second;
-  Cheapest best{-1.0, n};
-  auto consider = [&](int r) {
-    const double c = pass_cost(r) + cheapest(n / r, cap, known).cost;
-    if (best.cost < 0.0 || c < best.cost) best = Cheapest{c, r};
-  };
-  for (int r = 16; r >= 2; --r)
-    if (n % r == 0 && usable(r, cap)) consider(r);
-  if (best.cost < 0.0) {
-    int q = 17;
-    while (q * q <= n && n % q) q += 2;
-    consider(n % q ? n : q);
-  }
-  known[n] = best;
-  return best;
-}
-
 // Passes for `lines` lines of length n.  A short line's CTA is a warp or two, and a
 // launch of few of them is as long as one thread's butterflies: radices up to kSmallCap
 // then (360 x 240: 36 us a solve with radices up to 16, 30 us), 16 where there are
 // enough CTAs, or threads in one, to keep the FP64 pipes busy.
 constexpr int kShortLine = 512, kFewLines = 8 * 148, kSmallCap = 8;
+constexpr int kMaxDivisors = 64;  // of a length up to kMaxLen (7560 has most)
 inline Radices choose_passes(int n, int lines) {
   const int cap = n < kShortLine && lines <= kFewLines ? kSmallCap : 16;
   Radices f;
   f.n = n;
+  // the divisors of n in ascending order, with the cost of each one's cheapest
+  // factorisation and its first radix; a divisor without a small radix takes its least prime
+  constexpr int kRoot = 91;  // above the square root of kMaxLen
+  int divisor[kMaxDivisors], first[kMaxDivisors], divisors = 0;
+  double cost[kMaxDivisors];
+  unsigned char low[kRoot], high[kRoot];  // where divisor d and divisor n / d are
+  for (int d = 1; d * d <= n; ++d)
+    if (n % d == 0) {
+      low[d] = (unsigned char)divisors;
+      divisor[divisors++] = d;
+    }
+  for (int i = divisors - 1; i >= 0; --i) {
+    high[divisor[i]] = low[divisor[i]];
+    if (divisor[i] * divisor[i] == n) continue;
+    high[divisor[i]] = (unsigned char)divisors;
+    divisor[divisors++] = n / divisor[i];
+  }
+  // where the divisor d is, `other` being n / d
+  auto place = [&](int d, int other) { return d <= other ? low[d] : high[other]; };
+  cost[0] = 0.0;
+  for (int i = 1; i < divisors; ++i) {
+    const int d = divisor[i], other = n / d;
+    cost[i] = -1.0;
+    auto consider = [&](int r) {
+      const double c = pass_cost(r) + cost[place(d / r, other * r)];
+      if (cost[i] < 0.0 || c < cost[i]) {
+        cost[i] = c;
+        first[i] = r;
+      }
+    };
+    for (int r = 16; r >= 2; --r)
+      if (d % r == 0 && usable(r, cap)) consider(r);
+    if (cost[i] < 0.0) {
+      int q = 17;
+      while (q * q <= d && d % q) q += 2;
+      consider(d % q ? d : q);
+    }
+  }
   int r[kMaxPasses], count = 0;
-  std::map<int, Cheapest> known;
-  for (int m = n; m > 1; m /= r[count - 1]) r[count++] = cheapest(m, cap, known).first;
+  for (int m = n; m > 1; m /= r[count - 1]) r[count++] = first[place(m, n / m)];
   std::sort(r, r + count, [](int a, int b) { return a > b; });
   int L = n;
   for (int s = 0; s < count; ++s) {
@@ -541,7 +552,7 @@ struct P2 {
   }
   static inline unsigned ctas(int pairs) { return (unsigned)((pairs + PB - 1) / PB); }
 
-  // The table of the twiddled passes (k_p2_table): for pass s, a row of its TP >> LV s
+  // The table of the twiddled passes (k_dct_tables): for pass s, a row of its TP >> LV s
   // butterflies' e^{-2 pi i k q / L} for each of q = 1, 2, 4, 8, so that a warp reads whole
   // lines.  Rows for q = 3 and 12 too cost more than the products (4096 x 4096: 296 and
   // 280 us a solve) and gained no accuracy to speak of.
@@ -1124,14 +1135,28 @@ __global__ void __launch_bounds__(kThreads, PRIME ? 1 : 2)
   });
 }
 
+// An axis' tables.  `len` > 0: a power of two's own kernels, radix 2^lv, whose table of
+// `len` entries (P2::table_offset) takes the place of the plain twiddles.
 __global__ void k_dct_tables(double2 *tw, double2 *post, double *eig, unsigned short *rev,
-                             Radices rad) {
+                             Radices rad, int lv, int len) {
   const int n = rad.n;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
+  int e = k;  // exponent of the twiddle in place k
+  if (len) {
+    int row = n >> lv, step = 1, at = k;  // butterflies of a pass, step of its twiddles
+    while (row > 0 && at >= kPowers * row) {
+      at -= kPowers * row;
+      row >>= lv;
+      step <<= lv;
+    }
+    if (k < len) e = (at % row * step) << (at / row);
+  }
   double s, c;
-  sincospi(2.0 * (double)k / (double)n, &s, &c);
-  if (tw) tw[k] = make_double2(c, -s);
+  if (!len || k < len) {
+    sincospi(2.0 * (double)e / (double)n, &s, &c);
+    tw[k] = make_double2(c, -s);
+  }
   sincospi((double)k / (2.0 * (double)n), &s, &c);
   post[k] = make_double2(c, -s);
   eig[k] = 2.0 * cos(M_PI * (double)k / (double)n);
@@ -1141,22 +1166,6 @@ __global__ void k_dct_tables(double2 *tw, double2 *post, double *eig, unsigned s
     f /= rad.p[q].r;
   }
   rev[k] = (unsigned short)pos;
-}
-
-// The twiddle table of a power-of-two length (P2::table_offset), `len` entries in all.
-__global__ void k_p2_table(double2 *tab, int n, int lv, int len) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= len) return;
-  int row = n >> lv, step = 1, at = g;  // butterflies of a pass, step of its twiddles
-  while (at >= kPowers * row) {
-    at -= kPowers * row;
-    row >>= lv;
-    step <<= lv;
-  }
-  const int j = at / row, k = at - j * row;
-  double s, c;
-  sincospi(2.0 * (double)((k * step) << j) / (double)n, &s, &c);
-  tab[g] = make_double2(c, -s);
 }
 
 inline size_t a256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -1279,9 +1288,7 @@ extern "C" int gd_dct_plan_bind(gd_dct_plan p, void *ws, size_t bytes, cudaStrea
           lv = dct::P2<decltype(log)::value>::LV;
         },
         [](auto) {});
-    dct::k_dct_tables<<<(r.n + 255) / 256, 256, 0, st>>>(len ? nullptr : t.tw, t.post, t.eig,
-                                                         t.rev, r);
-    if (len) dct::k_p2_table<<<(len + 255) / 256, 256, 0, st>>>(t.tw, r.n, lv, len);
+    dct::k_dct_tables<<<(r.n + 255) / 256, 256, 0, st>>>(t.tw, t.post, t.eig, t.rev, r, lv, len);
   };
   fill(tw, p->rw);
   fill(th, p->rh);

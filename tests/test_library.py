@@ -66,3 +66,24 @@ def test_plan_flags_are_checked_on_the_host():
         rc = _lib.lib().gd_plan_create(grids, 1, ctypes.byref(prm), ctypes.byref(out))
         assert rc == -1 and not out.value
         assert field.encode() in _lib.lib().gd_last_error()
+
+
+def test_transform_plans_are_cheap_to_create():
+    """The choice of a transform's passes is part of every first solve of a shape: a length of
+    64 divisors (7560) must not cost many times what a trivial one does (11 times when the
+    divisors were looked up in a std::map)."""
+    import time
+    lib = _lib.lib()
+
+    def seconds(n):
+        best = float("inf")
+        for _ in range(500):
+            out = ctypes.c_void_p()
+            t0 = time.perf_counter()
+            rc = lib.gd_dct_plan_create(n, n, ctypes.byref(out))
+            best = min(best, time.perf_counter() - t0)
+            assert rc == 0
+            lib.gd_dct_plan_destroy(out)
+        return best
+
+    assert seconds(7560) <= 8 * seconds(2)
