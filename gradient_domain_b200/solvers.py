@@ -222,7 +222,12 @@ DCT_MAX_SIDE = 8192  # longest line a DCT pass holds in shared memory
 
 class DctPlan:
     """DCT Neumann solver for one grid shape (gd_dct_* of the C ABI): the library's own
-    FFT kernels, three passes over the grid, sides of 2 to 8192 cells."""
+    FFT kernels, three passes over the grid, sides of 2 to 8192 cells.
+
+    The coefficients between the passes live in the plan's workspace, so solves of one plan
+    run one after another: a solve on another stream than the last one's waits for that one
+    (threads may share a plan; each enqueues its solve whole).  Under graph capture, and for
+    replays of such a graph, the order is the caller's."""
 
     def __init__(self, h: int, w: int):
         self.shape = (h, w)
@@ -235,6 +240,9 @@ class DctPlan:
         self.workspace = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
         _lib.check(lib.gd_dct_plan_bind(handle, _lib.ptr(self.workspace), nbytes,
                                         _lib.stream_handle()), "gd_dct_plan_bind")
+        self._lock = threading.Lock()
+        self._done = torch.cuda.Event()  # after the latest solve, and the stream it ran on
+        self._ran_on: int | None = None
 
     def solve(self, b: torch.Tensor, u: torch.Tensor) -> torch.Tensor:
         """u = zero-mean solution of laplacian(u) = b (FP64 device tensors, one row pitch)."""
@@ -244,15 +252,26 @@ class DctPlan:
                 raise ValueError(f"expected {self.shape} float64 tensors on {self.device}")
         if b.stride(0) != u.stride(0):
             raise ValueError("b and u must share a row pitch (u may be b: solved in place)")
-        _lib.check(_lib.lib().gd_dct_solve_neumann(self._handle, _lib.ptr(b), _lib.ptr(u),
-                                                   u.stride(0), _lib.stream_handle()),
-                   "gd_dct_solve_neumann")
+        stream = torch.cuda.current_stream(self.device)
+        handle = _lib.stream_handle(stream)
+        with self._lock:
+            ordered = not torch.cuda.is_current_stream_capturing()
+            if ordered and self._ran_on not in (None, handle):
+                stream.wait_event(self._done)
+            _lib.check(_lib.lib().gd_dct_solve_neumann(self._handle, _lib.ptr(b), _lib.ptr(u),
+                                                       u.stride(0), handle),
+                       "gd_dct_solve_neumann")
+            if ordered:
+                self._done.record(stream)
+                self._ran_on = handle
         return u
 
     def __del__(self):
         if getattr(self, "_handle", None):
             try:
                 torch.cuda.current_stream(self.device).synchronize()
+                if self._ran_on is not None:
+                    self._done.synchronize()  # the last solve, whichever stream it ran on
                 _lib.lib().gd_dct_plan_destroy(self._handle)
             except Exception:
                 pass
