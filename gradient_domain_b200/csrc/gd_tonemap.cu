@@ -235,10 +235,11 @@ __global__ void __launch_bounds__(kTmThreads)
 // their IEEE bit patterns order like the values.  Two histograms of twelve bits
 // (the first formed while the image is written) leave about n / 10000 candidates,
 // which one more pass over the values collects into a list for its last CTA to
-// search.  Values that crowd into one slice of 2^-12 of an octave overflow the
-// list: unless they are all the same value, a third histogram and a second
-// collection (which return at once otherwise) narrow the slice to 2^-24, and if
-// that overflows too the last CTA searches the array itself.
+// search.  Values that crowd into one slice of 2^-12 of an octave (a nearly flat
+// image) overflow the list: unless they are all the same value, four more histograms
+// (which return at once otherwise) fix the other forty bits, by the whole grid like
+// the first two.  (gd_tm_compose at 1440 x 2160: 29 ms when the last CTA searched such an
+// image alone, 0.43 so, 0.17 where the list suffices.)
 
 constexpr int kBins = 4096;
 constexpr int kListMax = 1 << 16;
@@ -248,7 +249,7 @@ struct SelectState {
   unsigned long long rank;       // of the wanted element among those that share them
   unsigned long long below;      // elements below all of those
   unsigned long long least, most;  // of those, as seen by the collection
-  unsigned long long above;      // the smallest element beyond them
+  unsigned long long above;      // the smallest element seen beyond them
   unsigned long long selected, count_le, next;  // results
   unsigned long long matched;    // elements that share the prefix
   unsigned count;                // places of the list given out
@@ -308,9 +309,10 @@ __device__ __forceinline__ unsigned long long warp_scan(unsigned long long v) {
   return v;
 }
 
-// By the last CTA: the bin that holds the wanted rank extends the prefix; the counters
-// are cleared for the next histogram.
-__device__ void choose_bin(SelectState *s, unsigned *hist) {
+// By the last CTA: the bin of `width` bits that holds the wanted rank extends the prefix;
+// the counters are cleared for the next histogram.  `last`: these are the key's lowest bits
+// (at most four, so that thread 0 holds every bin), and the selection is finished.
+__device__ void choose_bin(SelectState *s, unsigned *hist, int width, bool last) {
   constexpr int kEach = kBins / kTmThreads;
   __shared__ unsigned long long warp_sums[kTmThreads / 32];
   __shared__ int bin_of;
@@ -341,38 +343,65 @@ __device__ void choose_bin(SelectState *s, unsigned *hist) {
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    s->prefix = s->prefix << 12 | (unsigned long long)bin_of;
+    const unsigned long long outer = s->prefix << width;
+    s->prefix = outer | (unsigned long long)bin_of;
     s->rank = rank - below_bin;
     s->below += below_bin;
+    if (last) {
+      unsigned long long next = __ldcg(&s->above);
+      int q = bin_of + 1;
+      while (q < kEach && !c[q]) ++q;
+      if (q < kEach) next = outer | (unsigned long long)q;
+      s->selected = s->prefix;
+      s->count_le = s->below + c[bin_of];
+      s->next = next;
+      s->done = 1;
+    }
   }
 #pragma unroll
   for (int q = 0; q < kEach; ++q) hist[threadIdx.x * kEach + q] = 0u;
 }
 
-// Histogram of the twelve bits at `shift` of the values that share the prefix above them.
+// Histogram of the `width` bits at `shift` of the values that share the prefix above them.
+// LATE: a histogram after the collection, which also notes the smallest value beyond the
+// prefix (a longer prefix leaves no fewer values beyond it, so the last one's minimum holds).
+template <bool LATE>
 __global__ void __launch_bounds__(kTmThreads) k_select_hist(unsigned *__restrict__ hist,
                                                             const double *__restrict__ v,
                                                             long long n, SelectState *s,
-                                                            int shift) {
-  if (s->done) return;
+                                                            int shift, int width) {
+  if (LATE && s->done) return;
   __shared__ unsigned h[kBins];
   for (int b = threadIdx.x; b < kBins; b += kTmThreads) h[b] = 0u;
   __syncthreads();
   const unsigned long long prefix = s->prefix;
+  const unsigned mask = (1u << width) - 1u;
+  unsigned long long above = ~0ull;
   const long long stride = (long long)gridDim.x * kTmThreads;
   for (long long k0 = (long long)blockIdx.x * kTmThreads + threadIdx.x; k0 < n; k0 += 4 * stride) {
     unsigned long long key[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const long long k = k0 + u * stride;
-      key[u] = k < n ? (unsigned long long)__double_as_longlong(v[k]) : ~prefix << (shift + 12);
+      key[u] = k < n ? (unsigned long long)__double_as_longlong(v[k]) : ~prefix << (shift + width);
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (key[u] >> (shift + 12) == prefix) atomicAdd(&h[(key[u] >> shift) & (kBins - 1)], 1u);
+    for (int u = 0; u < 4; ++u) {
+      const unsigned long long top = key[u] >> (shift + width);
+      if (top == prefix) atomicAdd(&h[(unsigned)(key[u] >> shift) & mask], 1u);
+      else if (LATE && k0 + u * stride < n && top > prefix && key[u] < above) above = key[u];
+    }
+  }
+  if constexpr (LATE) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long q = __shfl_down_sync(0xffffffffu, above, o);
+      above = q < above ? q : above;
+    }
+    if ((threadIdx.x & 31) == 0 && above != ~0ull) atomicMin(&s->above, above);
   }
   add_hist(hist, h);
-  if (last_cta(s)) choose_bin(s, hist);
+  if (last_cta(s)) choose_bin(s, hist, width, shift == 0);
 }
 
 // The wanted element among the keys get(0) .. get(m - 1) that share the prefix above
@@ -436,13 +465,11 @@ __device__ void search(SelectState *s, long long m, int bits, Get get) {
 }
 
 // The values that share the prefix above `bits` into the list, and the smallest beyond
-// them; the last CTA finishes the selection when they fit (or are one value), and
-// with `final` in any case.
+// them; the last CTA finishes the selection when they fit or are one value.
 __global__ void __launch_bounds__(kTmThreads) k_select_collect(const double *__restrict__ v,
                                                                long long n, SelectState *s,
-                                                               unsigned long long *list, int bits,
-                                                               int final) {
-  if (s->done) return;
+                                                               unsigned long long *list,
+                                                               int bits) {
   const unsigned long long prefix = s->prefix;
   unsigned long long least = ~0ull, most = 0ull, above = ~0ull, matched = 0ull;
   const long long stride = (long long)gridDim.x * kTmThreads;
@@ -498,14 +525,6 @@ __global__ void __launch_bounds__(kTmThreads) k_select_collect(const double *__r
     }
   } else if (m <= (unsigned long long)kListMax) {
     search(s, (long long)m, bits, [&](long long k) { return __ldcg(&list[k]); });
-  } else if (final) {
-    search(s, n, bits, [&](long long k) { return (unsigned long long)__double_as_longlong(v[k]); });
-  } else if (threadIdx.x == 0) {  // for the next collection
-    s->count = 0u;
-    s->matched = 0ull;
-    s->least = ~0ull;
-    s->most = 0ull;
-    s->above = ~0ull;
   }
 }
 
@@ -570,7 +589,7 @@ __global__ void __launch_bounds__(kTmThreads)
     }
   }
   add_hist(hist, h);
-  if (last_cta(sel)) choose_bin(sel, hist);
+  if (last_cta(sel)) choose_bin(sel, hist, 12, false);
 }
 
 // np.percentile(image, q) with the linear method, then clip(image / peak, 0, 1).
@@ -678,10 +697,11 @@ extern "C" int gd_tm_compose(double *out, double *image, const double *radiance,
   auto *const make_image = saturation == 0.5 ? k_tm_image<true> : k_tm_image<false>;
   make_image<<<wide, kTmThreads, 0, st>>>(image, radiance, lum, compressed, s.part, kTmBlocks, n,
                                           saturation, s.sel, s.hist);
-  k_select_hist<<<wide, kTmThreads, 0, st>>>(s.hist, image, n3, s.sel, 40);
-  k_select_collect<<<wide, kTmThreads, 0, st>>>(image, n3, s.sel, s.list, 40, 0);
-  k_select_hist<<<wide, kTmThreads, 0, st>>>(s.hist, image, n3, s.sel, 28);
-  k_select_collect<<<wide, kTmThreads, 0, st>>>(image, n3, s.sel, s.list, 28, 1);
+  k_select_hist<false><<<wide, kTmThreads, 0, st>>>(s.hist, image, n3, s.sel, 40, 12);
+  k_select_collect<<<wide, kTmThreads, 0, st>>>(image, n3, s.sel, s.list, 40);
+  for (int shift : {28, 16, 4, 0})  // return at once where the list was enough
+    k_select_hist<true><<<kTmBlocks, kTmThreads, 0, st>>>(s.hist, image, n3, s.sel, shift,
+                                                          shift ? 12 : 4);
   const int vec = ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(image)) & 15) == 0;
   k_tm_finish<<<8 * kTmBlocks, kTmThreads, 0, st>>>(out, image, n3, s.sel, lo, t, vec);
   GD_CHECK_LAUNCH();

@@ -2,8 +2,11 @@
 
 import numpy as np
 import pytest
+import torch
 
 import gradient_domain_b200 as gd
+from gradient_domain_b200 import _lib
+from gradient_domain_b200 import hdr as hdr_gpu
 from oracle import hdr
 
 pytestmark = pytest.mark.gpu
@@ -16,13 +19,13 @@ def _radiance(kind, shape, rng):
         r = np.exp(rng.standard_normal(shape + (3,)))
         r[..., 0][rng.random(shape) < 0.3] = 0.0
         return r
-    # values crowd into one slice of an octave: nothing (one value), a slice of 2^-12
-    # and one of 2^-24 hold more of them than the candidate list
-    spread = {"flat": 0.0, "crowded": 1e-5, "packed": 1e-9}[kind]
+    # values crowd into one slice of an octave: nothing (one value), slices of 2^-12, 2^-24,
+    # 2^-36 and 2^-48 hold more of them than the candidate list
+    spread = {"flat": 0.0, "crowded": 1e-5, "packed": 1e-9, "tight": 1e-12, "ulps": 4e-15}[kind]
     return 0.7 * (1.0 + spread * rng.random(shape + (3,)))
 
 
-@pytest.mark.parametrize("kind", ["noise", "zeros", "flat", "crowded", "packed"])
+@pytest.mark.parametrize("kind", ["noise", "zeros", "flat", "crowded", "packed", "tight", "ulps"])
 @pytest.mark.parametrize("shape,levels,saturation", [((160, 181), 8, 0.5), ((161, 160), 1, 0.7),
                                                      ((17, 33), 8, 0.5)])
 def test_tone_map_matches_the_oracle(kind, shape, levels, saturation):
@@ -34,3 +37,38 @@ def test_tone_map_matches_the_oracle(kind, shape, levels, saturation):
     # them over the image
     np.testing.assert_allclose(factor, ref_factor, rtol=1e-10, atol=0)
     np.testing.assert_allclose(out, ref, rtol=1e-9, atol=1e-12)
+
+
+def test_percentile_time_does_not_depend_on_the_values():
+    """A nearly flat image, whose values crowd within 2^-24 of the percentile, is selected by
+    the whole grid too: at most four times as long as noise (four histograms more on top of
+    two and a collection; one CTA alone took 70 times as long)."""
+    h, w = 1440, 2160
+    lib = _lib.lib()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(2)
+
+    def rand(*shape):
+        return torch.rand(*shape, generator=g, dtype=torch.float64, device="cuda")
+
+    def compose_ms(spread):
+        rad, lum = rand(h, w, 3) + 0.5, rand(h, w) + 0.5
+        comp = rand(h, w) * spread
+        image, out = torch.empty_like(rad), torch.empty_like(rad)
+        scratch = hdr_gpu._scratch(rad.device)
+        best = np.inf
+        for _ in range(4):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            # saturation 0: the image is exp(comp - max comp) in all channels
+            _lib.check(lib.gd_tm_compose(_lib.ptr(out), _lib.ptr(image), _lib.ptr(rad),
+                                         _lib.ptr(lum), _lib.ptr(comp), h, w, 0.0, 99.5,
+                                         _lib.ptr(scratch), _lib.stream_handle()), "compose")
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        peak = torch.from_numpy(np.percentile(image.cpu().numpy(), [99.5])).cuda()
+        assert torch.equal(out, (image / peak).clamp(0, 1))
+        return best
+
+    assert compose_ms(1e-13) <= 4 * compose_ms(1.0)
