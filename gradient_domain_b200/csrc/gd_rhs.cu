@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cstdarg>
 #include <cstdio>
+#include <type_traits>
 
 #include "gd_internal.cuh"
 
@@ -177,17 +178,58 @@ struct FieldView {
 // window's outer ring is written 0 (no consumer of a window reads it) or, with
 // `edges`, follows operators.py's edge rules for the window as a whole image.
 //
-// A warp walks kGuideRows rows of 31 columns: the field of a cell is formed once,
-// its left neighbour's comes from the lane beside (lane 0 only serves as the first
-// column's neighbour) and the one above from the row before (1440 x 2160 weighted
-// field: 40 us with three fields a cell and a 64-bit division, 26 us).
-constexpr int kGuideRows = 8, kGuideCols = 31, kGuideWarps = 8;
+// Both kernels form a cell's field once; its left neighbour's comes from the lane beside,
+// whose first column only serves that.
+__device__ __forceinline__ double guide_value(int i, int j, int h, int w, bool edges, double gx,
+                                              double gxl, double gy, double gy_up) {
+  if (!edges && (i == 0 || j == 0 || i == h - 1 || j == w - 1)) return 0.0;
+  double dx = 0.0, dy = 0.0;
+  if (w > 1) dx = j == 0 ? gx : j == w - 1 ? -gxl : __dsub_rn(gx, gxl);
+  if (h > 1) dy = i == 0 ? gy : i == h - 1 ? -gy_up : __dsub_rn(gy, gy_up);
+  return __dadd_rn(dx, dy);
+}
+
+// k_guidance_tile: a CTA's threads are rows of LANES columns (32, or the few that hold a
+// narrow window), its first row serving the one below through shared memory, so that all
+// its cells are in flight at once.  64 x 64 weighted field 6 us where a walk of eight rows
+// takes 10; mixed 512 x 512 8 and 13 us, 1440 x 2160 50 and 55.
+constexpr int kGuideThreads = 288;
+template <int LANES>
+constexpr int kTileRows = kGuideThreads / LANES - 1;
+template <int LANES>
+__global__ void __launch_bounds__(kGuideThreads)
+    k_guidance_tile(double *__restrict__ out, FieldView fv, int row0, int col0, int h, int w) {
+  __shared__ double gy_of[kGuideThreads];
+  const int r = threadIdx.x / LANES, c = threadIdx.x % LANES;
+  const int j = blockIdx.x * (LANES - 1) + c - 1;
+  constexpr int rows = kTileRows<LANES>;
+  for (int i0 = blockIdx.y * rows; i0 < h; i0 += gridDim.y * rows) {
+    const int i = i0 + r - 1;
+    const bool inside = i >= 0 && i < h && j >= 0 && j < w;
+    double gx = 0.0, gy = 0.0;
+    if (inside) fv.field(row0 + i, col0 + j, gx, gy);
+    const double gxl = __shfl_up_sync(0xffffffffu, gx, 1);
+    gy_of[threadIdx.x] = gy;
+    __syncthreads();
+    if (inside && r > 0 && c > 0)
+      out[(long long)i * w + j] =
+          guide_value(i, j, h, w, fv.d.edges, gx, gxl, gy, gy_of[threadIdx.x - LANES]);
+    __syncthreads();
+  }
+}
+
+// k_guidance_walk: a warp walks kGuideRows rows of 31 columns, the row above in registers.
+// For weighted fields (two loads a cell) of at least kGuideWalks such walks, where there are
+// warps enough to hide a walk's chain and a CTA per eight rows costs more than it hides:
+// 1500 x 1500 (9212 walks) 20 us, 21 in tiles; 1440 x 2160 26 and 31; 4096 x 4096 151 and
+// 190; but 1200 x 1600 (7800 walks) 19 both, 1100 x 1300 17 and 15.
+constexpr int kGuideRows = 8, kGuideCols = 31, kGuideWarps = 8, kGuideWalks = 8192;
 __global__ void __launch_bounds__(32 * kGuideWarps)
-    k_guidance_div(double *__restrict__ out, FieldView fv, int row0, int col0, int h, int w) {
+    k_guidance_walk(double *__restrict__ out, FieldView fv, int row0, int col0, int h, int w) {
   const int lane = threadIdx.x & 31;
   const int j = (blockIdx.x * kGuideWarps + (threadIdx.x >> 5)) * kGuideCols + lane - 1;
   if (j - lane >= w - 1) return;  // whole warp beyond the window
-  const bool inside = j >= 0 && j < w, writes = inside && lane > 0;
+  const bool inside = j >= 0 && j < w;
   const int x = col0 + j;
   for (int i0 = blockIdx.y * kGuideRows; i0 < h; i0 += gridDim.y * kGuideRows) {
     const int i1 = min(i0 + kGuideRows, h);
@@ -200,17 +242,8 @@ __global__ void __launch_bounds__(32 * kGuideWarps)
       double gx = 0.0, gy = 0.0;
       if (inside) fv.field(row0 + i, x, gx, gy);
       const double gxl = __shfl_up_sync(0xffffffffu, gx, 1);
-      if (writes) {
-        double v = 0.0;
-        const bool ring = i == 0 || j == 0 || i == h - 1 || j == w - 1;
-        if (!ring || fv.d.edges) {
-          double dx = 0.0, dy = 0.0;
-          if (w > 1) dx = j == 0 ? gx : j == w - 1 ? -gxl : __dsub_rn(gx, gxl);
-          if (h > 1) dy = i == 0 ? gy : i == h - 1 ? -gy_up : __dsub_rn(gy, gy_up);
-          v = __dadd_rn(dx, dy);
-        }
-        out[(long long)i * w + j] = v;
-      }
+      if (inside && lane > 0)
+        out[(long long)i * w + j] = guide_value(i, j, h, w, fv.d.edges, gx, gxl, gy, gy_up);
       gy_up = gy;
     }
   }
@@ -280,8 +313,22 @@ extern "C" int gd_guidance_divergence(double *div, const gd_field_desc *field, i
              "gd_guidance_divergence: cloning fields need a source and a selection");
   GD_REQUIRE(d.kind != GD_FIELD_WEIGHTED || d.weights, GD_ERR_ARG,
              "gd_guidance_divergence: weighted fields need weights");
-  const dim3 grid(ceil_div(w, kGuideCols * kGuideWarps), std::min(ceil_div(h, kGuideRows), 65535));
-  k_guidance_div<<<grid, 32 * kGuideWarps, 0, st>>>(div, FieldView{d}, row0, col0, h, w);
+  if (d.kind == GD_FIELD_WEIGHTED &&
+      (long long)ceil_div(w, kGuideCols) * ceil_div(h, kGuideRows) >= kGuideWalks) {
+    const dim3 grid(ceil_div(w, kGuideCols * kGuideWarps),
+                    std::min(ceil_div(h, kGuideRows), 65535));
+    k_guidance_walk<<<grid, 32 * kGuideWarps, 0, st>>>(div, FieldView{d}, row0, col0, h, w);
+  } else {
+    auto tiles = [&](auto lanes) {
+      constexpr int L = decltype(lanes)::value;
+      const dim3 grid(ceil_div(w, L - 1), std::min(ceil_div(h, kTileRows<L>), 65535));
+      k_guidance_tile<L><<<grid, kGuideThreads, 0, st>>>(div, FieldView{d}, row0, col0, h, w);
+    };
+    if (w <= 3) tiles(std::integral_constant<int, 4>{});
+    else if (w <= 7) tiles(std::integral_constant<int, 8>{});
+    else if (w <= 15) tiles(std::integral_constant<int, 16>{});
+    else tiles(std::integral_constant<int, 32>{});
+  }
   GD_CHECK_LAUNCH();
   return GD_OK;
 }
