@@ -92,11 +92,33 @@ __device__ __forceinline__ double total_max(const double *part, int count) {
   return total;
 }
 
-// CTAs over an h x w array, kTmThreads columns each and about `ctas` in all: a CTA
-// walks rows blockIdx.y, blockIdx.y + gridDim.y, ... of its columns.
+// Columns (log2) of a CTA over an array of width w: kTmThreads, or on a narrow array the
+// power of two that holds it, the threads then being several rows (attenuation of
+// 20000 x 20: 112 us with a row a CTA, 50 so; 6000 x 17 50 and 30).
+inline int cta_columns(int w) {
+  int c = 5;
+  while ((1 << c) < kTmThreads && (1 << c) < w) ++c;
+  return c;
+}
+
+// Where a thread of such a CTA works: rows row, row + rows, ... of columns column,
+// column + columns, ... with `lg` = cta_columns(w).
+struct Walk {
+  int row, rows, column, columns;
+  __device__ __forceinline__ explicit Walk(int lg) {
+    const int each = kTmThreads >> lg;
+    row = blockIdx.y * each + (threadIdx.x >> lg);
+    rows = gridDim.y * each;
+    column = (blockIdx.x << lg) + (threadIdx.x & ((1 << lg) - 1));
+    columns = gridDim.x << lg;
+  }
+};
+
+// CTAs over an h x w array, about `ctas` in all.
 inline dim3 grid_2d(int h, int w, int ctas) {
-  const int gx = std::min((w + kTmThreads - 1) / kTmThreads, ctas);
-  return dim3(gx, std::max(1, std::min(h, ctas / gx)));
+  const int cols = 1 << cta_columns(w), each = kTmThreads / cols;
+  const int gx = std::min((w + cols - 1) / cols, ctas);
+  return dim3(gx, std::max(1, std::min((h + each - 1) / each, ctas / gx)));
 }
 
 __global__ void k_tm_luminance(double *__restrict__ logl, double *__restrict__ lum,
@@ -120,9 +142,10 @@ __global__ void k_tm_luminance(double *__restrict__ logl, double *__restrict__ l
 constexpr int kDownRows = 2;
 __global__ void __launch_bounds__(kTmThreads) k_tm_downsample(double *__restrict__ out,
                                                               const double *__restrict__ in, int h,
-                                                              int w) {
+                                                              int w, int lg) {
   const int oh = (h + 1) / 2, ow = (w + 1) / 2;
-  const int j = blockIdx.x * kTmThreads + threadIdx.x;
+  const Walk walk(lg);
+  const int j = walk.column;
   if (j >= ow) return;
   const double wgt[5] = {1.0 / 16.0, 4.0 / 16.0, 6.0 / 16.0, 4.0 / 16.0, 1.0 / 16.0};
   int col[5];
@@ -135,7 +158,7 @@ __global__ void __launch_bounds__(kTmThreads) k_tm_downsample(double *__restrict
     for (int b = 0; b < 5; ++b) hb = __dadd_rn(hb, __dmul_rn(wgt[b], row[col[b]]));
     return hb;
   };
-  for (int i0 = blockIdx.y * kDownRows; i0 < oh; i0 += gridDim.y * kDownRows) {
+  for (int i0 = walk.row * kDownRows; i0 < oh; i0 += walk.rows * kDownRows) {
     const int i1 = min(i0 + kDownRows, oh);
     double hb[5];
 #pragma unroll
@@ -178,10 +201,12 @@ __device__ __forceinline__ double tm_magnitude(const double *a, int h, int w, in
 
 __global__ void __launch_bounds__(kTmThreads) k_tm_mag_partials(double *__restrict__ part,
                                                                 const double *__restrict__ a,
-                                                                int h, int w, Spacing sp) {
+                                                                int h, int w, int lg,
+                                                                Spacing sp) {
+  const Walk walk(lg);
   double s = 0.0;
-  for (int j = blockIdx.x * kTmThreads + threadIdx.x; j < w; j += gridDim.x * kTmThreads)
-    for (int i = blockIdx.y; i < h; i += gridDim.y)
+  for (int j = walk.column; j < w; j += walk.columns)
+    for (int i = walk.row; i < h; i += walk.rows)
       s = __dadd_rn(s, tm_magnitude(a, h, w, i, j, sp));
   s = block_reduce_sum(s);
   if (threadIdx.x == 0) part[blockIdx.y * gridDim.x + blockIdx.x] = s;
@@ -197,11 +222,12 @@ __device__ __forceinline__ double tm_linspace(int i, int n_coarse, int n_fine, d
 __global__ void __launch_bounds__(kTmThreads)
     k_tm_factor(double *__restrict__ factor, const double *__restrict__ a,
                 const double *__restrict__ coarse, const double *__restrict__ part, int nparts,
-                int h, int w, int ch, int cw, Spacing sp, double alpha, double beta, double eps,
-                double step_y, double step_x) {
+                int h, int w, int lg, int ch, int cw, Spacing sp, double alpha, double beta,
+                double eps, double step_y, double step_x) {
   const double mean = total_sum(part, nparts) / (double)((long long)h * w);
   const double scale = __dmul_rn(alpha, fmax(mean, eps));
-  for (int j = blockIdx.x * kTmThreads + threadIdx.x; j < w; j += gridDim.x * kTmThreads) {
+  const Walk walk(lg);
+  for (int j = walk.column; j < w; j += walk.columns) {
     int c0 = 0, c1 = 0;
     double wx = 0.0;
     if (coarse) {
@@ -210,7 +236,7 @@ __global__ void __launch_bounds__(kTmThreads)
       c1 = min(c0 + 1, cw - 1);
       wx = __dsub_rn(rx, (double)c0);
     }
-    for (int i = blockIdx.y; i < h; i += gridDim.y) {
+    for (int i = walk.row; i < h; i += walk.rows) {
       const double m = fmax(tm_magnitude(a, h, w, i, j, sp), eps);
       const double local = __dmul_rn(scale / m, pow(m / scale, beta));
       const long long k = (long long)i * w + j;
@@ -650,10 +676,10 @@ extern "C" int gd_tm_log_luminance(double *logl, double *lum, const double *radi
 extern "C" int gd_tm_downsample(double *out, const double *in, int32_t h, int32_t w,
                                 cudaStream_t st) {
   GD_REQUIRE(out && in && h > 0 && w > 0, GD_ERR_ARG, "gd_tm_downsample: bad arguments");
-  const int oh = (h + 1) / 2, ow = (w + 1) / 2;
-  const dim3 grid((ow + kTmThreads - 1) / kTmThreads,
-                  std::min((oh + kDownRows - 1) / kDownRows, 65535));
-  k_tm_downsample<<<grid, kTmThreads, 0, st>>>(out, in, h, w);
+  const int oh = (h + 1) / 2, ow = (w + 1) / 2, lg = cta_columns(ow), cols = 1 << lg;
+  const int rows = kTmThreads / cols * kDownRows;  // outputs of a CTA
+  const dim3 grid((ow + cols - 1) / cols, std::min((oh + rows - 1) / rows, 65535));
+  k_tm_downsample<<<grid, kTmThreads, 0, st>>>(out, in, h, w, lg);
   GD_CHECK_LAUNCH();
   return GD_OK;
 }
@@ -668,11 +694,12 @@ extern "C" int gd_tm_level_factor(double *factor, const double *level, const dou
   const TmScratch s = tm_scratch(scratch);
   const Spacing sp(2.0 * spacing);
   const dim3 gm = grid_2d(h, w, kTmBlocks), gf = grid_2d(h, w, 8 * kTmBlocks);
+  const int lg = cta_columns(w);
   const double step_y = h > 1 ? (double)(ch - 1) / (double)(h - 1) : 0.0;
   const double step_x = w > 1 ? (double)(cw - 1) / (double)(w - 1) : 0.0;
-  k_tm_mag_partials<<<gm, kTmThreads, 0, st>>>(s.part, level, h, w, sp);
+  k_tm_mag_partials<<<gm, kTmThreads, 0, st>>>(s.part, level, h, w, lg, sp);
   k_tm_factor<<<gf, kTmThreads, 0, st>>>(factor, level, coarse, s.part, (int)(gm.x * gm.y), h, w,
-                                         ch, cw, sp, alpha, beta, epsilon, step_y, step_x);
+                                         lg, ch, cw, sp, alpha, beta, epsilon, step_y, step_x);
   GD_CHECK_LAUNCH();
   return GD_OK;
 }

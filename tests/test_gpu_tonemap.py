@@ -72,3 +72,34 @@ def test_percentile_time_does_not_depend_on_the_values():
         return best
 
     assert compose_ms(1e-13) <= 4 * compose_ms(1.0)
+
+
+@pytest.mark.parametrize("shape", [(2000, 17), (17, 2000), (900, 33), (600, 65), (400, 129),
+                                   (300, 257)])
+def test_attenuation_of_narrow_images_matches_the_oracle(shape):
+    """Widths around the powers of two that a CTA's columns take."""
+    logl = np.random.default_rng(sum(shape)).standard_normal(shape)
+    want = hdr.attenuation_field(logl, hdr.ToneMapConfig())
+    got = gd.attenuation_field(logl, gd.ToneMapConfig())
+    # a logarithm, a power and the mean's order of sums differ by a few ulp
+    np.testing.assert_allclose(got, want, rtol=1e-12, atol=0)
+
+
+def test_attenuation_time_of_a_narrow_image():
+    """20000 x 20 has a seventh of the cells of 1440 x 2000: its attenuation takes at most half
+    as long (as long, when every row took a CTA of 256 columns)."""
+    def device_us(h, w):
+        logl = torch.randn((h, w), dtype=torch.float64, device="cuda")
+        scratch = hdr_gpu._scratch(logl.device)
+        best = np.inf
+        for _ in range(10):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda._sleep(3_000_000)  # the launches are queued before the device reaches them
+            a.record()
+            hdr_gpu._attenuation_dev(logl, gd.ToneMapConfig(levels=2), scratch)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b) * 1e3)
+        return best
+
+    assert device_us(20000, 20) <= 0.5 * device_us(1440, 2000)
