@@ -55,6 +55,11 @@ SPACE: tuple[tuple[str, tuple[int, ...]], ...] = (
     ("bottom_cells", (4096, 1024, 16384)),
 )
 
+# Of the kernels and rules that entries were timed with; entries of another one never apply.
+# Raised when a change of kernels, of SPACE or of the defaults behind its zeros makes the old
+# choices stale (2: the register-group tile kernels and the strip / tile rule by boundary type).
+REVISION = 2
+
 _CACHE_LOCK = threading.Lock()
 _MEMORY: dict[tuple[str, str], dict] = {}
 
@@ -96,6 +101,7 @@ def _load(path: str) -> dict:
 
 
 def _store(path: str, key: str, entry: dict) -> None:
+    entry = {**entry, "revision": REVISION}
     _MEMORY[(path, key)] = entry
     os.makedirs(os.path.dirname(os.path.abspath(path)), exist_ok=True)
     data = _load(path)
@@ -104,6 +110,10 @@ def _store(path: str, key: str, entry: dict) -> None:
     with open(tmp, "w") as fh:
         json.dump(data, fh, indent=1, sort_keys=True)
     os.replace(tmp, path)
+
+
+def _current(entry: dict | None) -> bool:
+    return bool(entry) and entry.get("revision") == REVISION
 
 
 def _apply(params: SolveParams, choice: dict) -> SolveParams:
@@ -126,7 +136,7 @@ def lookup(instances: Sequence[Instance], params: SolveParams | None = None,
         else:  # read the file once per key; an untuned key is remembered as such
             entry = _load(path).get(key) or {}
             _MEMORY[(path, key)] = entry
-    if not entry or entry.get("device", device_name()) != device_name():
+    if not _current(entry) or entry.get("device", device_name()) != device_name():
         return params
     return _apply(params, entry.get("choice", {}))
 
@@ -266,7 +276,7 @@ def tune(instances: Sequence[Instance], params: SolveParams | None = None,
     if not force:
         with _CACHE_LOCK:
             entry = _MEMORY.get((path, key)) or _load(path).get(key)
-        if entry:
+        if _current(entry):
             return _apply(params, entry.get("choice", {}))
     if any(inst.boundary == "masked" for inst in instances) and masks is None:
         raise ValueError("masked instances need their masks to be tuned")

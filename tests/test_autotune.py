@@ -117,3 +117,27 @@ def test_untuned_keys_are_read_from_the_file_once(tmp_path, monkeypatch):
     for _ in range(3):
         assert autotune.resolve(insts, SolveParams(), path) == SolveParams()
     assert len(reads) == 1
+
+
+@pytest.mark.parametrize("stamp", [{}, {"revision": 1}, {"revision": autotune.REVISION + 1}])
+def test_entries_of_another_revision_never_apply(tmp_path, monkeypatch, stamp):
+    """A choice timed with other kernels or rules: ignored by lookup and resolve, timed anew
+    by tune."""
+    path = str(tmp_path / "tune.json")
+    insts = [Instance(640, 480, "neumann", True)]
+    key = autotune.tune_key(insts, SolveParams())
+    old = {"choice": {"sweeps": 3, "tile_cells": 262144}, "ms": 1.0, "default_ms": 1.1, **stamp}
+    with open(path, "w") as fh:
+        json.dump({key: old}, fh)
+    assert autotune.lookup(insts, SolveParams(), path) == SolveParams()
+    assert autotune.resolve(insts, SolveParams(), path) == SolveParams()
+    monkeypatch.setattr(autotune, "time_solve", lambda *args: 1.0)
+    monkeypatch.setattr(autotune._lib, "device", lambda: "cpu")
+    monkeypatch.setattr(autotune, "_synthetic_rhs", lambda *args: None)
+    monkeypatch.setattr(autotune.torch.cuda, "get_device_name", lambda *args: "cpu")
+    autotune.tune(insts, SolveParams(), path=path)
+    with open(path) as fh:
+        entry = json.load(fh)[key]
+    assert entry["revision"] == autotune.REVISION and entry["choice"]["sweeps"] == 2
+    autotune._MEMORY.clear()  # as another process reads it
+    assert autotune.lookup(insts, SolveParams(), path).sweeps == 2
