@@ -89,3 +89,27 @@ def test_residual_outside_the_mask_is_not_read(shape, precision):
             for plan, out in zip((clean, dirty), x):
                 assert plan.solve([f], [out])[0].converged, (name, junk)
             assert torch.equal(x[0], x[1]), (name, junk)
+
+
+@pytest.mark.parametrize("shape", [(700, 1100), (301, 297)])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_persistent_coarse_launch_skips_the_same_tiles(shape, precision):
+    """The persistent coarse launch leaves out tiles without unknowns as the level launches
+    do: the same bits, on direct launches and in the solve graph, beside a rectangle."""
+    h, w = shape
+    g = torch.Generator(device="cuda")
+    g.manual_seed(h + 2 * w)
+    insts = [Instance(h, w, "masked"), Instance(h, w, "neumann", True)]
+    plans = [PoissonPlan(insts, SolveParams(precision=precision, tolerance=1e-9, zero_start=True,
+                                            persistent_coarse=p)) for p in (False, True)]
+    for name, on in _masks(h, w, g).items():
+        f = [torch.randn(shape, generator=g, dtype=torch.float64, device="cuda") for _ in insts]
+        f[0] = torch.where(on, f[0], torch.zeros_like(f[0]))
+        for _ in range(2):
+            got = []
+            for plan in plans:
+                plan.set_mask(0, on.to(torch.uint8))
+                x = [torch.full_like(q, float("nan")) for q in f]
+                assert all(r.converged for r in plan.solve(f, x, scale=-1.0)), name
+                got.append(x)
+            assert all(torch.equal(p, q) for p, q in zip(*got)), name
