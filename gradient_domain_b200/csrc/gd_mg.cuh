@@ -17,12 +17,23 @@ constexpr int kBottomSmem = 220 * 1024;
 constexpr int kBottomLevels = 24;  // most levels one bottom holds
 // Coarse levels (below level 0, above the bottom) with at most kTileCells cells, or
 // kTileCellsMasked on masked instances, run on the shared-memory tile kernels; larger
-// ones on the strips.  Solves with the level named on strips / on tiles: 375 000 cells
-// (FP64 1000 x 1500) 2.45 / 2.37 ms, 391 937 x 3 (1022 x 1533 x 3) 1.69 / 1.68,
-// 490 000 x 3 (1400 x 1400 x 3) 1.74 / 1.77 and FP64 2.95 / 3.06, 1 000 000 x 3
-// 3.00 / 3.17; masked, whose strips carry the classes' code, 489 258 x 3
-// (1411 x 1387 x 3) 3.31 / 3.20.  The rule looks at the instance alone, because the
-// two kernels round differently and a batch gives every instance its own bits.
+// ones on the strips.  Time of an iteration on tiles over that on strips, by the cells of
+// the level in question, one and three equal instances in the plan:
+//                         280k   350k   392k   420k   490k   520k   560k   640k   800k  1000k
+//   mixed             1  0.928  0.918  0.927  0.931  0.933  0.939  0.959  0.967  0.966  0.987
+//                     3  0.983  0.977  0.994  1.014  1.010  1.015  1.030  1.031  1.045  1.058
+//   FP64              1  0.941  0.968  0.972  0.965  0.967  0.973  1.007  1.018  1.021  1.041
+//                     3  1.043  1.014  1.011  1.042  1.058  1.057  1.085  1.084  1.088  1.119
+//   masked, a disc    1  0.938  0.956  0.948  0.956  0.958  0.957  0.959  0.955  0.971  0.967
+//                     3  0.973  0.972  0.976  0.980  0.987  0.991  0.982  0.989  1.006  1.028
+//   masked, FP64 disc 1  0.927  0.946  0.969  0.993  0.992  0.993  0.993  0.996  1.003  1.026
+//   masked, all cells 3  0.988  0.976  0.985  0.999  1.011  1.017  1.012  1.017  1.029  1.042
+// The more instances, the earlier the strips win, but the rule may look at one instance
+// only, because the two kernels round differently and a batch gives every instance its own
+// bits.  The lines lie where a colour image (three instances) changes sides: between 392k
+// and 420k on rectangles in mixed precision (FP64 loses 1 % there and wins 3 % alone), and
+// between 420k (every cell an unknown) and 800k (a disc) on masked levels, whose strips
+// carry the classes' code.
 constexpr int kTileCells = 3 << 17, kTileCellsMasked = 1 << 19;
 
 // Fine-level (level 0) kernels: 64 rows x 128 columns per CTA of 128 threads
