@@ -82,9 +82,10 @@ __global__ void __launch_bounds__(kBThreads, 1) k_coarse(Args<T> a, Phases ph) {
         if (a.st[k].status == GD_ACTIVE) bottom_instance<T, S, S>(a, k, smem);
       } else {
         const Tile tl = a.tiles[ph.base[q] + k];
+        const bool idle = !a.act[ph.base[q] + k];  // requested with the tile
         const LevelInfo L = a.lv[tl.level];
         const LevelInfo Lc = a.lv[tl.level + 1];
-        if (a.st[tl.inst].status != GD_ACTIVE || !a.act[ph.base[q] + k]) continue;
+        if (a.st[tl.inst].status != GD_ACTIVE || idle) continue;
         if (kind == kPhaseDown)
           tile::down_tile<T, S, kBThreads, tile::kTYs, tile::kTXs>(a, tl, L, Lc, smem);
         else
