@@ -11,6 +11,10 @@
 // masked rows loaded on use; event times of single launches, mixed precision).
 // tile_rows() has the rule.
 //
+// The search direction lives in two buffers: k_pupdate reads the current one
+// (including halo cells owned by other CTAs) and writes the other, so no CTA
+// overwrites a value another CTA still has to read.
+//
 // Level 0 has wall coefficient 0 (Neumann) or 1, so a cell's diagonal is
 // 4 - walls (1 - w), exact in FP32 and formed from a per-lane column term and a
 // row term; masked levels always have 4.  Cells without an unknown and the

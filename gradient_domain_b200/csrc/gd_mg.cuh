@@ -36,11 +36,9 @@ constexpr int kBottomLevels = 24;  // most levels one bottom holds
 // carry the classes' code.
 constexpr int kTileCells = 3 << 17, kTileCellsMasked = 1 << 19;
 
-// Fine-level (level 0) kernels: 64 rows x 128 columns per CTA of 128 threads
-// (four warps, each 16 rows x 128 columns).  Down / up kernels use the same
-// CTA shape with a per-level strip height.
+// Tiles of the level-0 kernels that walk no strips (means, FP64 refresh, solution): 64 rows
+// x 128 columns, 128 threads unless a kernel says otherwise.
 constexpr int kFTY = 64, kFTX = 128, kFThreads = 128;
-constexpr int kVThreads = 128;     // down / up kernels
 constexpr int kBThreads = 1024;    // bottom kernel
 
 enum : int { BC_DIR = 0, BC_NEU = 1, BC_MASK = 2 };

@@ -13,9 +13,9 @@
 // red-black Gauss-Seidel with colour 0 then 1 before restriction and colour 1
 // then 0 after prolongation, so the cycle is a symmetric operator.  Each level
 // costs two passes over HBM (the register-streaming kernels of gd_stream.cuh):
-// `down` smooths from zero, forms the residual and restricts it; `up`
-// recomputes that pre-smoothed iterate from b instead of storing it, adds P e
-// and post-smooths.  Small levels run in `k_bottom` (this file), one CTA per
+// `down` smooths from zero, writes that iterate, forms the residual and restricts
+// it; `up` reads the iterate back, adds P e and post-smooths.  Small levels run on
+// shared-memory tiles (gd_tile.cuh) and in `k_bottom` (this file), one CTA per
 // instance, down to a dense FP64 solve.
 #pragma once
 
@@ -24,10 +24,6 @@
 #include "gd_mg.cuh"
 
 namespace gd {
-
-__device__ __forceinline__ bool in_grid(const LevelInfo &L, int y, int x) {
-  return y >= 0 && y < L.ny && x >= 0 && x < L.nx;
-}
 
 // Last-CTA handshake over the `ctas` CTAs of one instance: each calls it once;
 // returns true in the last one.  The instance's ticket is zero again after it
@@ -73,13 +69,6 @@ __device__ __forceinline__ bool instance_sum(double *part, int first, int ctas, 
   return true;
 }
 
-// The search direction lives in two buffers: k_pupdate reads the current one
-// (including halo cells owned by other CTAs) and writes the other, so no CTA
-// overwrites a value another CTA still has to read.
-__device__ __forceinline__ long long p_offset(const InstInfo &I, int which) {
-  return which ? I.q_off : I.p_off;
-}
-
 __device__ __forceinline__ void finish_rz(InstState &S, double rz,
                                           cudaGraphConditionalHandle refresh) {
   if (!(rz > 0.0) || !isfinite(rz)) {
@@ -93,27 +82,8 @@ __device__ __forceinline__ void finish_rz(InstState &S, double rz,
   S.rz = rz;
 }
 
-template <typename T>
-__device__ __forceinline__ void make_tables(T *diag, T *dinv, float wall) {
-  if (threadIdx.x < 8) {
-    const int c = threadIdx.x;
-    const double d = c >= 1 && c <= 5 ? class_diag(c, wall) : 1.0;
-    diag[c] = (T)d;
-    dinv[c] = (c >= 1 && c <= 5 && d > 0.0) ? (T)(1.0 / d) : (T)0;
-  }
-}
-
 // Bilinear-adjoint weights of one axis for fine offsets 2I-1 .. 2I+2.
 __device__ __forceinline__ float rweight(int a) { return (a == 0 || a == 3) ? 0.25f : 0.75f; }
-
-// Neumann restriction reads the mirrored residual at fine index -1 and, for an
-// even fine size n, at index n (the clamped ghost of P^T).
-__device__ __forceinline__ int mirror_fine(int f, int n, bool neumann) {
-  if (!neumann) return f;
-  if (f == -1) return 0;
-  if (f == n && !(n & 1)) return n - 1;
-  return f;
-}
 
 // Classes of the 4 cells x0..x0+3 of row y, packed one byte each.
 __device__ __forceinline__ unsigned row_classes(const LevelInfo &L, const unsigned char *codes,
@@ -575,13 +545,10 @@ __global__ void __launch_bounds__(kBThreads, 1) k_bottom(Args<T> a) {
 }
 
 // ---------------------------------------------------------------------------
-// Elementwise level-0 kernels over 64 x 128 tiles (the Krylov kernels with
-// halos are in gd_stream.cuh).
+// Elementwise level-0 kernels over 64 x 128 tiles (the Krylov kernels are in
+// gd_krylov.cuh, the FP64 refresh in gd_stream.cuh).  A thread owns a column of the
+// tile, so every warp access is 32 consecutive elements.
 
-// x += d for instances with a pending FP64 refresh (d then restarts from zero
-// through FLAG_DZERO instead of being cleared here).  A thread owns one
-// column of the 64 x 128 tile, so every warp access is 32 consecutive
-// elements; the independent rows are unrolled for several loads in flight.
 // Sum of column x over rows y0 .. y1 - 1 of an FP64 array, eight independent
 // loads in flight per thread and a fixed summation tree.
 __device__ __forceinline__ double column_sum(const double *A, long long pitch, int y0, int y1,

@@ -4,7 +4,8 @@
 // columns (4 per lane, one 128-bit vector for FP32) and walks down its strip
 // one row at a time; the rows it still needs live in small register windows,
 // vertical neighbours are window entries and horizontal neighbours at lane
-// boundaries come from warp shuffles.  Nothing is staged in shared memory.
+// boundaries come from warp shuffles.  Shared memory only holds the rings through
+// which rows arrive.
 //
 // The smoothing kernels pipeline the red-black half sweeps: when row y is
 // loaded, half sweep 1 runs on row y, half sweep 2 on row y-1, ..., so after
@@ -288,21 +289,6 @@ __device__ __forceinline__ void hsweep_zero(V4<T> &u, const V4<T> &b, unsigned c
                                             const Coef<T, INT> &K) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) u.v[j] = ((j & 1) == J0) ? mul_rn(b.v[j], K.inv(c, j)) : T(0);
-}
-
-// A u on a row (zero where there is no unknown).
-template <typename T, bool INT>
-__device__ __forceinline__ V4<T> arow(const V4<T> &u, const V4<T> &up, const V4<T> &dn, T left,
-                                      T right, unsigned c, const Coef<T, INT> &K) {
-  V4<T> r;
-  const T lf[4] = {left, u.v[0], u.v[1], u.v[2]};
-  const T rt[4] = {u.v[1], u.v[2], u.v[3], right};
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const T v = K.d(c, j) * u.v[j] - (up.v[j] + dn.v[j] + lf[j] + rt[j]);
-    r.v[j] = K.on(c, j) ? v : T(0);
-  }
-  return r;
 }
 
 // Window slot of "row y - k" at unrolled phase PH of a circular window of U rows.

@@ -2,7 +2,7 @@
 
 Run once in a container that holds the reference sources:
 
-    PYTHONDONTWRITEBYTECODE=1 python tests/golden/make_golden.py /root/reference
+    PYTHONDONTWRITEBYTECODE=1 python tests/golden/make_golden.py <reference checkout>
 
 It imports ``gradient-domain/src`` from the given reference checkout, runs the
 reference's own functions on small seeded inputs and writes
@@ -172,7 +172,9 @@ def suite(reference_root: str) -> None:
 
 if __name__ == "__main__":
     args = [a for a in sys.argv[1:] if not a.startswith("--")]
-    root = args[0] if args else "/root/reference"
+    if not args:
+        sys.exit("usage: make_golden.py <reference checkout> [--suite]")
+    root = args[0]
     if "--suite" not in sys.argv:
         main(root)
     suite(root)
