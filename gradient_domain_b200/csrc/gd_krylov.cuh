@@ -291,7 +291,8 @@ __device__ __forceinline__ double cgupdate_rows(const Place<T> &w, const unsigne
       rv.v[j] = on ? rv.v[j] - alpha * ap.v[j] : T(0);
       acc += rv.v[j] * rv.v[j];
     }
-    if (w.nv < 4) {  // the columns of a width that is no multiple of four: squares in FP64
+    // the columns of a width that is no multiple of four: squares in FP64
+    if (sizeof(T) == 4 && w.nv < 4) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) part += (double)rv.v[j] * (double)rv.v[j];
     } else {
