@@ -686,8 +686,8 @@ def dct_main(args) -> None:
     ms = e0.elapsed_time(e1) / args.steps
     hbm, peak_kind = peaks()
     cells = n_ch * h * w
-    line = {"config": {"workload": f"dct-neumann {h}x{w}x{n_ch}", "kernels": "k_dct_rows, "
-                       "k_dct_cols, k_idct_rows (three passes per channel)"},
+    line = {"config": {"workload": f"dct-neumann {h}x{w}x{n_ch}", "kernels": "k_rows_*, "
+                       "k_cols_*, k_irows_* (three passes per channel)"},
             "ms_per_step": ms, "mpix_s": cells / (ms / 1e3) / 1e6,
             "bytes_per_cell": {"algorithmic": 16, "passes": 48},
             "hbm_frac_of_passes": 48 * cells / (ms / 1e3) / 1e9 / hbm, "peak_gbs": hbm,

@@ -37,9 +37,9 @@
 // thread and pass, with the values in registers from the loads to the
 // coefficients: 3 passes and 2 exchanges for 4096 where radix 8 with staging
 // took 4 passes and 6.  Other lengths take the radices of the cheapest
-// factorisation (choose_passes) at run time.  Measured per channel, rows + columns
-// + rows: 4096 x 4096 72 + 117 + 84 us (88 + 284 + 111 before), 1080 x 1920
-// 26 + 41 + 23 us (54 + 82 + 44).
+// factorisation (choose_passes) at run time.  Measured a channel: 4096 x 4096 275 us
+// (75 rows, 122 columns, 83 rows under ncu; 490 with row-major T, radix 8 and staging),
+// 1080 x 1920 97 us (181).
 
 #include <algorithm>
 #include <cstdint>
@@ -69,6 +69,9 @@ struct Radices {
 // FP64 instructions per point of one pass of radix r (butterfly and twiddles,
 // counted from the code below), plus what a pass costs besides: its exchange
 // through shared memory and its barrier, worth about eight instructions a point.
+// A model, measured against two to four other factorisations each: its choice was the
+// fastest for squares of 1000 (43.6 us a solve, the next 55.9), 1440 (84, 94), 2160
+// (190, 203) and 3000 (350, 389), and at 1920 (12 x 16 x 10, 160 us) 8 % behind 16 x 15 x 8.
 inline double pass_cost(int r) {
   switch (r) {
     case 2: return 8 + 4.0;
@@ -95,7 +98,8 @@ inline bool usable(int r, int cap) { return r <= cap || r == 5 || r == 7 || r ==
 
 // Passes for `lines` lines of length n.  A short line's CTA is a warp or two, and a
 // launch of few of them is as long as one thread's butterflies: radices up to kSmallCap
-// then (360 x 240: 36 us a solve with radices up to 16, 30 us), 16 where there are
+// then (360 x 240: 35.6 us a solve with radices up to 16, 25.3 so; 240 x 320 32.5 and 27.3;
+// 480 x 480 29.3 and 27.3), 16 where there are
 // enough CTAs, or threads in one, to keep the FP64 pipes busy.
 constexpr int kShortLine = 512, kFewLines = 8 * 148, kSmallCap = 8;
 constexpr int kMaxDivisors = 64;  // of a length up to kMaxLen (7560 has most)
