@@ -103,10 +103,12 @@ inline bool usable(int r, int cap) { return r <= cap || r == 5 || r == 7 || r ==
 // enough CTAs, or threads in one, to keep the FP64 pipes busy.
 constexpr int kShortLine = 512, kFewLines = 8 * 148, kSmallCap = 8;
 constexpr int kMaxDivisors = 64;  // of a length up to kMaxLen (7560 has most)
+inline bool power_of_two_kernels(int n) { return n >= 64 && (n & (n - 1)) == 0; }
 inline Radices choose_passes(int n, int lines) {
   const int cap = n < kShortLine && lines <= kFewLines ? kSmallCap : 16;
   Radices f;
   f.n = n;
+  if (power_of_two_kernels(n)) return f;  // their passes are fixed
   // the divisors of n in ascending order, with the cost of each one's cheapest
   // factorisation and its first radix; a divisor without a small radix takes its least prime
   constexpr int kRoot = 91;  // above the square root of kMaxLen
@@ -1141,9 +1143,16 @@ __global__ void __launch_bounds__(kThreads, PRIME ? 1 : 2)
 
 // An axis' tables.  `len` > 0: a power of two's own kernels, radix 2^lv, whose table of
 // `len` entries (P2::table_offset) takes the place of the plain twiddles.
-__global__ void k_dct_tables(double2 *tw, double2 *post, double *eig, unsigned short *rev,
-                             Radices rad, int lv, int len) {
-  const int n = rad.n;
+struct TableJob {
+  double2 *tw, *post;
+  double *eig;
+  unsigned short *rev;
+  Radices rad;
+  int lv, len;
+};
+__global__ void k_dct_tables(TableJob rows, TableJob cols) {
+  const TableJob &J = blockIdx.y ? cols : rows;
+  const int n = J.rad.n, lv = J.lv, len = J.len;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   int e = k;  // exponent of the twiddle in place k
@@ -1159,17 +1168,17 @@ __global__ void k_dct_tables(double2 *tw, double2 *post, double *eig, unsigned s
   double s, c;
   if (!len || k < len) {
     sincospi(2.0 * (double)e / (double)n, &s, &c);
-    tw[k] = make_double2(c, -s);
+    J.tw[k] = make_double2(c, -s);
   }
   sincospi((double)k / (2.0 * (double)n), &s, &c);
-  post[k] = make_double2(c, -s);
-  eig[k] = 2.0 * cos(M_PI * (double)k / (double)n);
+  J.post[k] = make_double2(c, -s);
+  J.eig[k] = 2.0 * cos(M_PI * (double)k / (double)n);
   int pos = 0, f = k;
-  for (int q = 0; q < rad.count; ++q) {
-    pos += (f % rad.p[q].r) * rad.p[q].m;
-    f /= rad.p[q].r;
+  for (int q = 0; q < J.rad.count; ++q) {
+    pos += (f % J.rad.p[q].r) * J.rad.p[q].m;
+    f /= J.rad.p[q].r;
   }
-  rev[k] = (unsigned short)pos;
+  J.rev[k] = (unsigned short)pos;
 }
 
 inline size_t a256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -1283,19 +1292,19 @@ extern "C" int gd_dct_plan_bind(gd_dct_plan p, void *ws, size_t bytes, cudaStrea
                                                      "256-byte aligned");
   p->ws = static_cast<char *>(ws);
   const AxisTables tw = tables(p, p->o_tab_w, p->w), th = tables(p, p->o_tab_h, p->h);
-  auto fill = [&](const AxisTables &t, const dct::Radices &r) {
-    int len = 0, lv = 0;  // entries of a power-of-two kernel's twiddle table, in the place of tw
+  auto job = [&](const AxisTables &t, const dct::Radices &r) {
+    dct::TableJob j{t.tw, t.post, t.eig, t.rev, r, 0, 0};
     dct::with_kernels(
         r,
         [&](auto log) {
-          len = dct::P2<decltype(log)::value>::table_len;
-          lv = dct::P2<decltype(log)::value>::LV;
+          j.len = dct::P2<decltype(log)::value>::table_len;
+          j.lv = dct::P2<decltype(log)::value>::LV;
         },
         [](auto) {});
-    dct::k_dct_tables<<<(r.n + 255) / 256, 256, 0, st>>>(t.tw, t.post, t.eig, t.rev, r, lv, len);
+    return j;
   };
-  fill(tw, p->rw);
-  fill(th, p->rh);
+  const dim3 grid((std::max(p->w, p->h) + 255) / 256, 2);
+  dct::k_dct_tables<<<grid, 256, 0, st>>>(job(tw, p->rw), job(th, p->rh));
   GD_CHECK_LAUNCH();
   // the tables must be complete before a solve on any stream (set-up, once per plan)
   GD_CHECK_CUDA(cudaStreamSynchronize(st));

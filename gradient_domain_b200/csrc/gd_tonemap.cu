@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(kTmThreads)
 // image) overflow the list: unless they are all the same value, four more histograms
 // (which return at once otherwise) fix the other forty bits, by the whole grid like
 // the first two.  (gd_tm_compose at 1440 x 2160: 29 ms when the last CTA searched such an
-// image alone, 0.43 so, 0.17 where the list suffices.)
+// image alone, 0.45 so, 0.17 where the list suffices.)
 
 constexpr int kBins = 4096;
 // Longer lists go on with the histograms: the one CTA that searches a list takes about
