@@ -232,6 +232,9 @@ class DctPlan:
     def __init__(self, h: int, w: int):
         self.shape = (h, w)
         self.device = _lib.device()
+        self._lock = threading.Lock()
+        self._done = torch.cuda.Event()  # after the latest solve, and the stream it ran on
+        self._ran_on: int | None = None
         lib = _lib.lib()
         handle = C.c_void_p()
         _lib.check(lib.gd_dct_plan_create(h, w, C.byref(handle)), "gd_dct_plan_create")
@@ -240,9 +243,6 @@ class DctPlan:
         self.workspace = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
         _lib.check(lib.gd_dct_plan_bind(handle, _lib.ptr(self.workspace), nbytes,
                                         _lib.stream_handle()), "gd_dct_plan_bind")
-        self._lock = threading.Lock()
-        self._done = torch.cuda.Event()  # after the latest solve, and the stream it ran on
-        self._ran_on: int | None = None
 
     def solve(self, b: torch.Tensor, u: torch.Tensor) -> torch.Tensor:
         """u = zero-mean solution of laplacian(u) = b (FP64 device tensors, one row pitch)."""

@@ -90,6 +90,16 @@ def test_a_plan_is_destroyed_after_its_last_solve(plan):
     assert log[-1] == ("destroy",) and ("synchronize event", (8, 2)) in log
 
 
+def test_a_plan_whose_set_up_failed_is_destroyed(plan, monkeypatch):
+    made, solve, log = plan
+    monkeypatch.setattr(type(_lib.lib()), "gd_dct_plan_bind", lambda *args: -1)
+    monkeypatch.setattr(type(_lib.lib()), "gd_last_error", lambda self: b"no", raising=False)
+    del log[:]
+    with pytest.raises(_lib.GDError):
+        solvers.DctPlan(4, 4)
+    assert log[-1] == ("destroy",)
+
+
 def test_capture_neither_waits_nor_is_waited_for(plan):
     made, solve, log = plan
     solve(0)
