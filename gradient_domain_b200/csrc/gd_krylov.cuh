@@ -292,12 +292,14 @@ __device__ __forceinline__ double cgupdate_rows(const Place<T> &w, const unsigne
       acc += rv.v[j] * rv.v[j];
     }
     // the columns of a width that is no multiple of four: squares in FP64
+    double sq = (double)acc;
     if (sizeof(T) == 4 && w.nv < 4) {
+      double q[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) part += (double)rv.v[j] * (double)rv.v[j];
-    } else {
-      part += (double)acc;
+      for (int j = 0; j < 4; ++j) q[j] = (double)rv.v[j] * (double)rv.v[j];
+      sq = (q[0] + q[1]) + (q[2] + q[3]);
     }
+    part += sq;
     if (w.in) {
       const long long g = (long long)y * w.pitch + w.x0;
       st::st4(d + g, dv);
